@@ -15,11 +15,12 @@
 //    packed FP32x2 instructions (fma/mul/sub .f32x2 of sm_100a, each element rounded like the scalar
 //    instruction), with no per-pixel owner lookup or shared-memory traffic; the warp steps as often
 //    as its longest row needs, and each accepted pixel issues one predicated RED;
-//  * a device-side work queue for Gaussians covering more than kBigFragments pixels: their rows are
-//    cut into chunks of about kChunkPixels pixels that a persistent kernel steals across all SMs (no
-//    cross-warp tail, no host synchronisation). A chunk has R rows (a power of two <= 32) and each
-//    row is split into 32 / R segments, one lane per segment, so wide footprints keep every lane
-//    walking;
+//  * a device-side work queue for the Gaussians with larger AABBs (dense_scene): st_order_kernel
+//    puts a long queue in depth order and a persistent kernel takes its tiles of 8 x 8 pixels front to
+//    back (no cross-warp tail, no host synchronisation). Every tile has an upper bound of
+//    its keys' depths (tile_bound); one lane per tile drops the tiles that lie behind their bound or
+//    off the ellipse, and the warp walks the rest, two pixels per lane, lowering the bounds with the
+//    keys it reads. Keys only decrease during a pass, so a dropped fragment could not have won;
 //  * u64 atomicMin (fire-and-forget RED) on the L2-resident framebuffer.
 //
 // Bit-exactness. The reference's alpha exponent `dx * (cx * dx + cy * dy) + cz * dy * dy` is
@@ -30,6 +31,7 @@
 // Both forms are written out here with explicitly rounded intrinsics. With hybrid scheduling
 // the reference gathers the Gaussians whose AABB exceeds 512 pixels (the first
 // min(N, 2^20) of them, accumulate_hybrid.cu:26-27,98-111); those use the gather form.
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "sgs_internal.h"
@@ -41,17 +43,21 @@ namespace {
 constexpr uint32_t kBlock = 256;
 constexpr uint32_t kWarpsPerBlock = kBlock / 32;
 constexpr uint32_t kFullMask = 0xffffffffu;
-// Gaussians whose AABB exceeds this many pixels go to the work queue.
-constexpr uint32_t kBigFragments = 2048;
-// Pixels per stolen chunk of a queued Gaussian (whole rows, at most 32 of them).
-constexpr uint32_t kChunkPixels = 2048;
-constexpr uint32_t kQueueBlocksPerSM = 8;
+constexpr uint32_t kQueueBlocksPerSM = 4;
+// AABBs with more pixels are queued: kDenseMinPixels where the Gaussians above that size cover the
+// framebuffer many times over, kMinPixels elsewhere (dense_scene).
+constexpr uint32_t kMinPixels = 2048;
+constexpr uint32_t kDenseMinPixels = 256;
+constexpr float kSampleMaxPixels = 4096.0f;  // a sampled Gaussian counts for at most this many pixels
+constexpr uint32_t kOrderBlock = 512;
+constexpr uint32_t kMaxClaim = 16;     // items a consumer warp takes per atomic on the cursor
+constexpr uint32_t kPartQuads = 32;    // quads of four tiles in an item (a part of a queued Gaussian)
 // Hybrid scheduling: AABBs above this many pixels are gathered by the reference (accumulate_hybrid.cu:26).
 constexpr uint32_t kBinningPixelThreshold = 512;
 // Flag in RowGaussian::flags: evaluate with the hybrid gather's contraction.
 constexpr uint32_t kGatherFormFlag = 0x80000000u;
 
-// Per-Gaussian constants of the row/span expansion (64 bytes, four 16-byte words).
+// Per-Gaussian constants of the row/span expansion and of a queue entry (64 bytes, four 16-byte words).
 struct RowGaussian {
     float mx, my;       // mean2d - 0.5: pixel (x, y) has delta (x - mx, y - my)
     float cx, cy;       // exp2-scaled conic (x, y)
@@ -61,9 +67,34 @@ struct RowGaussian {
     uint32_t key_lo, key_hi;
     uint32_t x_min;
     uint32_t y_min, w;
-    uint32_t row_first; // first row position in the warp's row list (level 1)
+    uint32_t row_first; // first row position in the warp's row list (level 1); queue: height
     uint32_t flags;     // kGatherFormFlag
 };
+static_assert(sizeof(RowGaussian) == kStEntryBytes, "the workspace reserves kStEntryBytes per queue entry");
+
+// Queue entry e: the first q.entries_a entries lie in the queue section, the rest in the borrowed one.
+__device__ __forceinline__ RowGaussian* queue_entry(const StQueue& q, const uint32_t e) {
+    RowGaussian* const base = static_cast<RowGaussian*>(e < q.entries_a ? q.a : q.b);
+    return base + (e < q.entries_a ? e : e - q.entries_a);
+}
+
+// Aligned quads of four tiles of the fixed 8 x 8 grid that an AABB touches, and the items its
+// Gaussian is cut into.
+struct QuadRect {
+    uint32_t x0, y0, w, h;
+};
+__device__ __forceinline__ QuadRect quad_rect(const uint32_t x_min, const uint32_t w, const uint32_t y_min,
+                                              const uint32_t h) {
+    QuadRect t;
+    t.x0 = x_min / (4u * kBoundTile);
+    t.y0 = y_min / kBoundTile;
+    t.w = (x_min + w - 1u) / (4u * kBoundTile) - t.x0 + 1u;
+    t.h = (y_min + h - 1u) / kBoundTile - t.y0 + 1u;
+    return t;
+}
+__device__ __forceinline__ uint32_t part_count(const QuadRect& t) {
+    return min((t.w * t.h + kPartQuads - 1u) / kPartQuads, kMaxParts);
+}
 
 // Packed FP32x2 arithmetic (sm_100a): two independent round-to-nearest operations per instruction,
 // bit-identical to the scalar __fsub_rn / __fmul_rn / __fmaf_rn of each element.
@@ -156,24 +187,16 @@ __device__ __forceinline__ void red_min_if(unsigned long long* address, const un
         : "memory");
 }
 
-// Each lane walks segment `seg` of `1 << log_segs` equal parts of the span of its row y (when
-// valid), two pixels per step; the warp takes as many steps as its longest segment needs
-// (scatter_utils.cuh:35-46 per pixel).
+// Each lane walks the span of its row y (when valid), two pixels per step; the warp takes as many
+// steps as its longest row needs (scatter_utils.cuh:35-46 per pixel).
 template <bool kBlue, bool kHybrid, bool kMulti>
 __device__ __forceinline__ void walk_rows(const AccumulateParams& a, const FrameRng& rng, const bool valid,
-                                          const RowGaussian& G, const uint32_t y, const uint32_t seg = 0,
-                                          const uint32_t log_segs = 0) {
+                                          const RowGaussian& G, const uint32_t y) {
     uint32_t xs = 0, len = 0;
     float dy = 0.0f;
     if (valid) {
         dy = __fsub_rn(static_cast<float>(y), G.my);
         row_span(G.x_min, G.w, G.mx, G.span, dy, xs, len);
-        if (log_segs > 0) {
-            const uint32_t part = (len + (1u << log_segs) - 1u) >> log_segs;
-            const uint32_t skip = min(seg * part, len);
-            xs += skip;
-            len = min(len - skip, part);
-        }
     }
     const uint32_t steps = __reduce_max_sync(kFullMask, len);
     if (steps == 0) return;
@@ -237,25 +260,140 @@ __device__ __forceinline__ void walk_rows(const AccumulateParams& a, const Frame
     }
 }
 
-// Rows per chunk of a queued Gaussian of AABB width w: about kChunkPixels pixels, a power of two
-// between 1 and 32; each row of the chunk is walked in 32 / rows segments.
-__device__ __forceinline__ uint32_t log_chunk_rows(const uint32_t w) {
-    const uint32_t rows = max(1u, min(32u, kChunkPixels / max(w, 1u)));
-    return 31u - __clz(rows);
+// Whether the tile (tx, ty) may hold a pixel with alpha >= 1/255: the x-extent of the ellipse over the
+// tile's rows, a concave function of dy on either side whose maximum lies at +-dy_star or at the end
+// of the rows nearest to it, widened like a row's span (sgs_rows.cuh).
+__device__ __forceinline__ bool tile_on_ellipse(const RowGaussian& G, const uint32_t tx, const uint32_t ty) {
+    if (!(G.span.k2 > 0.0f)) return true;
+    const float x0 = static_cast<float>(tx * kBoundTile) - G.mx, y0 = static_cast<float>(ty * kBoundTile) - G.my;
+    constexpr float kSide = static_cast<float>(kBoundTile - 1u);
+    const float dymax = sqrtf(G.span.dymax2);
+    const float eps_y = kSpanPixelMargin + 4.0e-6f * (fabsf(y0) + dymax);
+    const float lo = fmaxf(y0 - eps_y, -dymax), hi = fminf(y0 + kSide + eps_y, dymax);
+    if (!(lo <= hi)) return lo != lo || hi != hi;
+    // right end at dy: slope dy + sqrt(k2 (dymax2 - dy^2)), largest at dy = slope sqrt(dymax2 / (k2 + slope^2))
+    const float star = G.span.slope * dymax * rsqrtf(G.span.k2 + G.span.slope * G.span.slope);
+    const float dr = fminf(fmaxf(star, lo), hi), dl = fminf(fmaxf(-star, lo), hi);
+    const float right = fmaf(G.span.slope, dr, sqrtf(G.span.k2 * fmaxf(fmaf(-dr, dr, G.span.dymax2), 0.0f)));
+    const float left = fmaf(G.span.slope, dl, -sqrtf(G.span.k2 * fmaxf(fmaf(-dl, dl, G.span.dymax2), 0.0f)));
+    const float eps = 0.1f + 1.0e-4f * (fabsf(right) + fabsf(left) + fabsf(x0));
+    // written so that a non-finite bound keeps the tile
+    return !(right + eps < x0) && !(left - eps > x0 + kSide);
 }
 
-// Rows [r0, r0 + (1 << log_rows)) of G, clipped to r_end: lane l walks segment l >> log_rows of row
-// r0 + (l & (rows - 1)).
+// A lane's two pixels of tile (tx, ty), (lane & 7, lane / 8) and four rows below, and their keys: 0 (which
+// nothing can beat) off the image.
+struct TilePixels {
+    unsigned long long* p;  // the upper pixel in the first sample's framebuffer
+    bool img0, img1;
+};
+__device__ __forceinline__ TilePixels tile_pixels(const AccumulateParams& a, const uint32_t tx, const uint32_t ty,
+                                                  const uint32_t lane) {
+    const uint32_t x = tx * kBoundTile + (lane & 7u), y = ty * kBoundTile + (lane >> 3);
+    TilePixels t;
+    t.p = a.framebuffer + (static_cast<size_t>(y) * a.cam.width_int + x);
+    t.img0 = x < a.cam.width_int && y < a.stq.height;
+    t.img1 = x < a.cam.width_int && y + 4u < a.stq.height;
+    return t;
+}
+struct TileKeys {
+    unsigned long long k0, k1;
+};
+__device__ __forceinline__ TileKeys tile_keys(const TilePixels& t, const size_t offset, const size_t below) {
+    TileKeys k;
+    k.k0 = t.img0 ? __ldcg(t.p + offset) : 0ull;
+    k.k1 = t.img1 ? __ldcg(t.p + offset + below) : 0ull;
+    return k;
+}
+
+// The warp walks tile (tx, ty) for Gaussian G, a lane the two pixels `px`: those whose key is
+// already nearer are left alone, and the largest depth of the tile's keys lowers its bound. `first`:
+// the tile's keys in the first sample's framebuffer (read ahead); with several samples per call the
+// other framebuffers' keys are read kKeyBatch samples at a time.
 template <bool kBlue, bool kHybrid, bool kMulti>
-__device__ __forceinline__ void walk_chunk(const AccumulateParams& a, const FrameRng& rng, const uint32_t lane,
-                                           const RowGaussian& G, const uint32_t r0, const uint32_t log_rows,
-                                           const uint32_t r_end) {
-    const uint32_t r = r0 + (lane & ((1u << log_rows) - 1u));
-    walk_rows<kBlue, kHybrid, kMulti>(a, rng, r < r_end, G, G.y_min + r, lane >> log_rows, 5u - log_rows);
+__device__ __forceinline__ void walk_tile(const AccumulateParams& a, const FrameRng& rng, const RowGaussian& G,
+                                          const uint32_t tx, const uint32_t ty, const uint32_t lane,
+                                          const TilePixels& px, const TileKeys& first) {
+    constexpr uint32_t kKeyBatch = kMulti ? 4u : 1u;
+    const uint32_t x = tx * kBoundTile + (lane & 7u);
+    const uint32_t y0 = ty * kBoundTile + (lane >> 3), y1 = y0 + 4u;
+    const bool col = x - G.x_min < G.w;
+    const bool in0 = col && y0 - G.y_min < G.row_first, in1 = col && y1 - G.y_min < G.row_first;
+    const size_t below = 4u * static_cast<size_t>(a.cam.width_int);
+    const unsigned long long key = (static_cast<unsigned long long>(G.key_hi) << 32) | G.key_lo;
+    uint32_t* const bound = a.stq.tile_bound + (static_cast<size_t>(ty) * a.stq.bound_pitch + tx);
+    if (!kMulti && !__any_sync(kFullMask, (in0 && key < first.k0) || (in1 && key < first.k1))) {
+        // nothing of the tile is left to win
+        const uint32_t far = __reduce_max_sync(
+            kFullMask, max(static_cast<uint32_t>(first.k0 >> 32), static_cast<uint32_t>(first.k1 >> 32)));
+        if (lane == 0) atomicMin(bound, far);
+        return;
+    }
+
+    // alpha of both pixels with the reference's contraction of the exponent
+    const float dx = __fsub_rn(static_cast<float>(x), G.mx);
+    const unsigned long long dy =
+        f2_sub(f2_pack(static_cast<float>(y0), static_cast<float>(y1)), f2_pack(G.my, G.my));
+    const unsigned long long cydy = f2_mul(f2_pack(G.cy, G.cy), dy), czdy = f2_mul(f2_pack(G.cz, G.cz), dy);
+    const unsigned long long dx2 = f2_pack(dx, dx);
+    const unsigned long long inner = f2_fma(f2_pack(G.cx, G.cx), dx2, cydy);
+    const bool gather_form = kHybrid && (G.flags & kGatherFormFlag);
+    const float2 e = f2_unpack(gather_form ? f2_fma(dx2, inner, f2_mul(czdy, dy))
+                                           : f2_fma(czdy, dy, f2_mul(dx2, inner)));
+    const float2 alpha = f2_unpack(
+        f2_mul(f2_pack(G.opacity, G.opacity), f2_pack(exp2f(fminf(e.x, 0.0f)), exp2f(fminf(e.y, 0.0f)))));
+    const bool hit0 = in0 && alpha.x >= kMinAlpha, hit1 = in1 && alpha.y >= kMinAlpha;
+    uint32_t bx;
+    const uint32_t seed0 = row_seed<kBlue>(rng, G.key_lo, y0, bx);
+    const uint32_t seed1 = row_seed<kBlue>(rng, G.key_lo, y1, bx);
+
+    uint32_t farthest = 0;
+    const uint32_t n_samples = kMulti ? a.n_samples : 1u;
+    size_t offset = 0;
+    for (uint32_t base = 0; base < n_samples; base += kKeyBatch, offset += kKeyBatch * a.fb_stride) {
+        TileKeys k[kKeyBatch];
+#pragma unroll
+        for (uint32_t j = 0; j < kKeyBatch; ++j)
+            k[j] = base + j == 0          ? first
+                   : base + j < n_samples ? tile_keys(px, offset + j * a.fb_stride, below)
+                                          : TileKeys{0ull, 0ull};
+#pragma unroll
+        for (uint32_t j = 0; j < kKeyBatch; ++j) {
+            farthest = max(farthest, max(static_cast<uint32_t>(k[j].k0 >> 32), static_cast<uint32_t>(k[j].k1 >> 32)));
+            const bool can0 = hit0 && key < k[j].k0, can1 = hit1 && key < k[j].k1;
+            if (!__any_sync(kFullMask, can0 || can1)) continue;
+            const uint32_t sm = base + j;
+            float2 u;
+            if (kBlue) {
+                const FrameRng rs = kMulti ? frame_rng_at(a, rng.frame + sm) : rng;
+                u = make_float2(st_blue_threshold(rs, seed0, x, bx), st_blue_threshold(rs, seed1, x, bx));
+            } else {
+                // row seeds differ between frames only in the frame term
+                const uint32_t df = kMulti ? (rng.frame * 1973u) ^ ((rng.frame + sm) * 1973u) : 0u;
+                u = f2_unpack(f2_sub(f2_pack(__uint_as_float(st_threshold_bits(seed0 ^ df, x)),
+                                             __uint_as_float(st_threshold_bits(seed1 ^ df, x))),
+                                     f2_pack(1.0f, 1.0f)));
+            }
+            unsigned long long* const p = px.p + (kMulti ? offset + j * a.fb_stride : 0u);
+            red_min_if(p, key, can0 && u.x < alpha.x);
+            red_min_if(p + below, key, can1 && u.y < alpha.y);
+        }
+    }
+    farthest = __reduce_max_sync(kFullMask, farthest);
+    if (lane == 0 && farthest != 0xffffffffu) atomicMin(bound, farthest);
+}
+
+// Whether the Gaussians above kDenseMinPixels cover the framebuffer many times over, by the clear pass's
+// sample. Then nearly all of what lies behind the first few surfaces is culled in the queue, so that it
+// takes all of them, in depth order; elsewhere the row walker is the faster one for footprints of up to
+// some 2000 pixels, and ordering a short queue costs more than it saves.
+__device__ __forceinline__ bool dense_scene(const AccumulateParams& a) {
+    const float4 c = *reinterpret_cast<const float4*>(a.queue->covered);
+    return c.x + c.y + c.z + c.w > a.stq.dense_pixels;
 }
 
 // One thread per Gaussian (accumulate_scatter.cu:19-77 for the projection and the AABB).
-template <bool kBlue, bool kHybrid, bool kMulti>
+template <bool kBlue, bool kHybrid, bool kMulti, bool kSplit>
 __global__ void __launch_bounds__(kBlock, 4) st_scatter_kernel(const AccumulateParams a) {
     __shared__ RowGaussian s_gauss[kWarpsPerBlock][32];
     __shared__ uint32_t s_rank[kWarpsPerBlock][32];
@@ -264,13 +402,19 @@ __global__ void __launch_bounds__(kBlock, 4) st_scatter_kernel(const AccumulateP
     const uint32_t wib = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
     const uint32_t upto_mask = kFullMask >> (31u - lane);
-    const uint32_t idx = blockIdx.x * kBlock + threadIdx.x;
+    // kSplit (small scenes): 2^log_row_split warps share 32 Gaussians, each walking every 2^log_row_split-th
+    // batch of their rows (all project them; the first one queues the large ones)
+    const uint32_t gwarp = blockIdx.x * kWarpsPerBlock + wib;
+    const uint32_t log_split = kSplit ? a.stq.log_row_split : 0u;
+    const uint32_t sub = gwarp & ((1u << log_split) - 1u);
+    const uint32_t idx = (gwarp >> log_split) * 32u + lane;
     bool active = idx < a.n;
     const uint32_t g = active ? idx : a.n - 1;
 
     Projected p;
     if (!project_gaussian(active, g, a.means, a.scales, a.rotations, a.opacities, a.w2c, a.cam, p, a.pre, a.quant)) return;
     const FrameRng rng = frame_rng(a);
+    const bool dense = dense_scene(a);
 
     const PixelRect rect = pixel_rect(p.bounds, a.cam);
     const uint32_t count = active ? rect.width * rect.height : 0u;
@@ -293,7 +437,8 @@ __global__ void __launch_bounds__(kBlock, 4) st_scatter_kernel(const AccumulateP
     G.span = span_constants(G.cx, G.cy, G.cz, G.opacity);
 
     if (kHybrid) {
-        // the reference gathers the first min(N, 2^20) Gaussians with more than 512 pixels
+        // the reference gathers the first min(N, 2^20) Gaussians with more than 512 pixels (warps sharing
+        // their Gaussians only run with fewer than that, when all are gathered)
         const bool binned = active && count > kBinningPixelThreshold;
         const uint32_t ballot = __ballot_sync(kFullMask, binned);
         if (ballot != 0) {
@@ -305,28 +450,39 @@ __global__ void __launch_bounds__(kBlock, 4) st_scatter_kernel(const AccumulateP
         }
     }
 
-    // large footprints: reserve row chunks in the work queue (or keep them when it is full)
+    // larger footprints: an entry in the work queue (or kept here when it is full); one atomic per warp
     bool keep_big = false;
     bool has_rows = count > 0;
-    if (count > kBigFragments) {
-        has_rows = false;
-        const uint32_t log_rpc = log_chunk_rows(rect.width);
-        const uint32_t chunks = (rect.height + (1u << log_rpc) - 1u) >> log_rpc;
-        const unsigned long long old = atomicAdd(&a.queue->packed, (1ull << kQueueEntryShift) | chunks);
-        const uint32_t e = static_cast<uint32_t>(old >> kQueueEntryShift);
-        const unsigned long long first_chunk = old & kQueueChunkMask;
-        if (e < a.q.capacity && first_chunk + chunks <= kMaxQueueChunks) {
-            a.q.key[e] = key;
-            a.q.geom[e] = make_float4(G.mx, G.my, G.cx, G.cy);
-            a.q.geom2[e] = make_float4(G.cz, G.opacity, __uint_as_float(rect.x_min), __uint_as_float(rect.width));
-            a.q.meta[e] = make_uint4(rect.y_min, rect.height, log_rpc | G.flags, static_cast<uint32_t>(first_chunk));
-        } else {
-            keep_big = true;
-            atomicAdd(&a.queue->overflow, 1u);
-            // an entry past 32-bit chunk indices is marked unused (the marked entries are the last ones:
-            // entries and chunks are reserved together)
-            if (e < a.q.capacity) a.q.meta[e] = make_uint4(0u, 0u, 0u, kUnusedQueueEntry);
+    const bool large = count > (dense ? kDenseMinPixels : kMinPixels);
+    const bool want = large && sub == 0;
+    if (large) has_rows = false;
+    const uint32_t big = __ballot_sync(kFullMask, want);
+    if (big != 0) {
+        const uint32_t leader = __ffs(big) - 1;
+        uint32_t e = 0;
+        if (lane == leader) e = atomicAdd(&a.queue->st_entries, static_cast<uint32_t>(__popc(big)));
+        e = __shfl_sync(kFullMask, e, leader) + __popc(big & lt_mask);
+        const bool fits = want && e < a.stq.capacity;
+        const uint32_t parts =
+            fits ? part_count(quad_rect(rect.x_min, rect.width, rect.y_min, rect.height)) : 0u;
+        const uint32_t incl = warp_inclusive_sum(parts, lane);
+        uint32_t item = 0;
+        if (lane == 31 && incl != 0) item = atomicAdd(&a.queue->st_items, incl);
+        item = __shfl_sync(kFullMask, item, 31) + (incl - parts);
+        const bool listed = fits && item + parts <= a.stq.list_capacity;
+        if (fits) {
+            RowGaussian st = G;
+            st.row_first = listed ? rect.height : 0u;  // no rows: the order pass skips the entry
+            *queue_entry(a.stq, e) = st;
         }
+        if (!dense) {
+            for (uint32_t i = 0; i < parts && item + i < a.stq.list_capacity; ++i)
+                a.stq.list[item + i] = listed ? i << kItemEntryBits | e : kNoItem;
+        } else if (listed) {
+            atomicAdd(a.stq.histogram + depth_bucket(G.key_hi), parts);
+        }
+        keep_big = want && !listed;
+        if (keep_big) atomicAdd(&a.queue->overflow, 1u);
     }
 
     // level 1: the rows of this warp's Gaussians, end to end, the Gaussians ordered by their widest
@@ -358,9 +514,10 @@ __global__ void __launch_bounds__(kBlock, 4) st_scatter_kernel(const AccumulateP
     }
     __syncwarp();
     int prev = -1;
-    for (uint32_t base = 0; base < total_rows; base += 32) {
+    for (uint32_t base = sub * 32u; base < total_rows; base += 32u << log_split) {
         const uint32_t rel = row_first - base;
         const uint32_t bits = __reduce_or_sync(kFullMask, (has_rows && rel < 32u) ? (1u << rel) : 0u);
+        if (kSplit) prev = __popc(__ballot_sync(kFullMask, has_rows && row_first < base)) - 1;
         const int owner = prev + __popc(bits & upto_mask);
         prev += __popc(bits);
         const uint32_t r = base + lane;
@@ -385,59 +542,191 @@ __global__ void __launch_bounds__(kBlock, 4) st_scatter_kernel(const AccumulateP
     }
 }
 
-// Persistent consumer of the large-Gaussian queue: each warp steals one chunk of rows at a time.
-template <bool kBlue, bool kHybrid, bool kMulti>
-__global__ void __launch_bounds__(kBlock) st_queue_kernel(const AccumulateParams a) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const unsigned long long packed = a.queue->packed;
-    const FrameRng rng = frame_rng(a);
-    const uint32_t n_entries =
-        static_cast<uint32_t>(min(packed >> kQueueEntryShift, static_cast<unsigned long long>(a.q.capacity)));
-    if (n_entries == 0) return;
-    uint32_t last_entry = n_entries - 1;  // the last used entry; entry 0 starts at chunk 0 and always is
-    if (a.q.meta[last_entry].w == kUnusedQueueEntry)
-        last_entry = queue_entry_of_chunk(a.q.meta, n_entries, kUnusedQueueEntry - 1u, lane);
-    const uint4 last = a.q.meta[last_entry];
-    const uint32_t last_log_rpc = last.z & ~kGatherFormFlag;
-    const uint32_t n_chunks = last.w + ((last.y + (1u << last_log_rpc) - 1u) >> last_log_rpc);
-    for (;;) {
-        uint32_t c = 0;
-        if (lane == 0) c = atomicAdd(&a.queue->next_chunk, 1u);
-        c = __shfl_sync(kFullMask, c, 0);
-        if (c >= n_chunks) break;
-        const uint32_t lo = queue_entry_of_chunk(a.q.meta, n_entries, c, lane);
-        const uint4 m = a.q.meta[lo];
-        const float4 gm = a.q.geom[lo];
-        const float4 gm2 = a.q.geom2[lo];
-        const unsigned long long key = a.q.key[lo];
-        RowGaussian G;
-        G.mx = gm.x;
-        G.my = gm.y;
-        G.cx = gm.z;
-        G.cy = gm.w;
-        G.cz = gm2.x;
-        G.opacity = gm2.y;
-        G.key_lo = static_cast<uint32_t>(key);
-        G.key_hi = static_cast<uint32_t>(key >> 32);
-        G.x_min = __float_as_uint(gm2.z);
-        G.w = __float_as_uint(gm2.w);
-        G.y_min = m.x;
-        G.row_first = 0;
-        G.flags = m.z & kGatherFormFlag;
-        G.span = span_constants(G.cx, G.cy, G.cz, G.opacity);
-        const uint32_t log_rpc = m.z & ~kGatherFormFlag;
-        const uint32_t r0 = (c - m.w) << log_rpc;
-        if (r0 >= m.y || G.w == 0 || log_rpc > 5u) {
-            if (lane == 0) atomicOr(&a.queue->error, 1u);
-            continue;
-        }
-        walk_chunk<kBlue, kHybrid, kMulti>(a, rng, lane, G, r0, log_rpc, m.y);
+// Lists the queue's items in depth order (buckets of 1/32 octave). Every block sums the producers'
+// histogram itself, counts its own slice of the entries per bucket in shared memory, takes each
+// bucket's share with one atomic and places its items there.
+__global__ void __launch_bounds__(kOrderBlock) st_order_kernel(const AccumulateParams a) {
+    constexpr uint32_t kPerThread = kDepthBuckets / kOrderBlock;
+    __shared__ uint32_t s_first[kDepthBuckets], s_count[kDepthBuckets];
+    __shared__ uint32_t s_warp[kOrderBlock / 32];
+    if (!dense_scene(a)) return;  // the producers have listed the items as they came
+    const uint32_t n = min(a.queue->st_entries, a.stq.capacity);
+    const uint32_t per_block = max(kOrderBlock, (n + gridDim.x - 1u) / gridDim.x);
+    const uint32_t begin = min(blockIdx.x * per_block, n), end = min(begin + per_block, n);
+    if (begin >= end) return;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t v[kPerThread], sum = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < kPerThread; ++i) {
+        v[i] = a.stq.histogram[threadIdx.x * kPerThread + i];
+        sum += v[i];
+        s_count[threadIdx.x * kPerThread + i] = 0u;
+    }
+    const uint32_t incl = warp_inclusive_sum(sum, lane);
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t first = incl - sum;
+    for (uint32_t w = 0; w < warp; ++w) first += s_warp[w];
+#pragma unroll
+    for (uint32_t i = 0; i < kPerThread; ++i) {
+        s_first[threadIdx.x * kPerThread + i] = first;
+        first += v[i];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == kOrderBlock - 1u) a.queue->st_listed = first;
+    auto parts_of = [&](const uint32_t e, uint32_t& bucket) {
+        const RowGaussian* const G = queue_entry(a.stq, e);
+        const uint32_t h = G->row_first;
+        bucket = depth_bucket(G->key_hi);
+        return h != 0 ? part_count(quad_rect(G->x_min, G->w, G->y_min, h)) : 0u;
+    };
+    for (uint32_t e = begin + threadIdx.x; e < end; e += kOrderBlock) {
+        uint32_t bucket;
+        const uint32_t parts = parts_of(e, bucket);
+        atomicAdd(&s_count[bucket], parts);
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t i = 0; i < kPerThread; ++i) {
+        const uint32_t bucket = threadIdx.x * kPerThread + i;
+        if (s_count[bucket] != 0)
+            s_first[bucket] += atomicAdd(a.stq.histogram + kDepthBuckets + bucket, s_count[bucket]);
+    }
+    __syncthreads();
+    for (uint32_t e = begin + threadIdx.x; e < end; e += kOrderBlock) {
+        uint32_t bucket;
+        const uint32_t parts = parts_of(e, bucket);
+        const uint32_t at = atomicAdd(&s_first[bucket], parts);
+        for (uint32_t i = 0; i < parts; ++i) a.stq.list[at + i] = i << kItemEntryBits | e;
     }
 }
 
-__global__ void clear_kernel(unsigned long long* __restrict__ fb, const size_t n_fb, WorkQueue* __restrict__ queue) {
-    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-    const size_t tid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+// Persistent consumer of the queue, front to back: a warp takes some items at a time, lays their quads
+// end to end and compares 32 quads of tile bounds at a time, one 16-byte load per lane; the tiles in
+// front of their bounds are tested against the ellipse, one per lane, and those that remain are
+// walked, the next tile's keys read ahead. Short queues are dealt out in pieces of items.
+template <bool kBlue, bool kHybrid, bool kMulti>
+__global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) st_queue_kernel(const AccumulateParams a) {
+    __shared__ RowGaussian s_gauss[kWarpsPerBlock][32];
+    __shared__ uint2 s_part[kWarpsPerBlock][32];     // first quad of the part, minus its place in the claim; quad columns
+    __shared__ uint8_t s_tiles[kWarpsPerBlock][128];  // tiles in front of their bounds: lane << 2 | tile of its quad
+    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    const uint32_t upto_mask = kFullMask >> (31u - lane);
+    const uint32_t n_items =
+        dense_scene(a) ? a.queue->st_listed : min(a.queue->st_items, a.stq.list_capacity);
+    if (n_items == 0) return;
+    const FrameRng rng = frame_rng(a);
+    const uint32_t n_warps = kWarpsPerBlock * gridDim.x;
+    uint32_t log_split = 0;
+    while (log_split < 4u && (n_items << log_split) < 4u * n_warps) ++log_split;
+    const uint32_t n_parts = n_items << log_split;
+    // The first claim is the warp's number; each next one is taken while the current is walked. Claims
+    // grow with the depth taken: most of what lies there is culled, and long claims in front of the
+    // queue would take items out of their order.
+    uint32_t c0 = blockIdx.x + wib * gridDim.x, claim = 1;
+    while (c0 < n_parts) {
+        const uint32_t next_claim = log_split == 0 ? min(1u + c0 / n_warps, kMaxClaim) : 1u;
+        uint32_t next = 0;
+        if (lane == 0) next = atomicAdd(&a.queue->next_chunk, next_claim);
+        const uint32_t item = lane < claim && c0 + lane < n_parts ? a.stq.list[(c0 + lane) >> log_split] : kNoItem;
+        RowGaussian G;
+        uint32_t quads = 0, first = 0, columns = 1;
+        if (item != kNoItem) {
+            G = *queue_entry(a.stq, item & kItemEntryMask);
+            const QuadRect r = quad_rect(G.x_min, G.w, G.y_min, G.row_first);
+            const uint32_t all = r.w * r.h, parts = part_count(r);
+            const uint32_t size = (all + parts - 1u) / parts;
+            first = min((item >> kItemEntryBits) * size, all);
+            quads = min(size, all - first);
+            columns = r.w;
+            // a short queue's items are dealt out in pieces
+            const uint32_t piece = (quads + (1u << log_split) - 1u) >> log_split;
+            const uint32_t skip = min(piece * ((c0 + lane) & ((1u << log_split) - 1u)), quads);
+            first += skip;
+            quads = min(piece, quads - skip);
+        }
+        const uint32_t incl = warp_inclusive_sum(quads, lane);
+        const uint32_t start = incl - quads;
+        const uint32_t total = __shfl_sync(kFullMask, incl, 31);
+        const uint32_t slot = __popc(__ballot_sync(kFullMask, quads != 0) & lt_mask);
+        __syncwarp();
+        if (quads != 0) {
+            s_gauss[wib][slot] = G;
+            s_part[wib][slot] = make_uint2(first - start, columns);
+        }
+        __syncwarp();
+        int prev = -1;
+        for (uint32_t base = 0; base < total; base += 32) {
+            const uint32_t rel = start - base;
+            const uint32_t bits = __reduce_or_sync(kFullMask, (quads != 0 && rel < 32u) ? (1u << rel) : 0u);
+            uint32_t owner = static_cast<uint32_t>(prev + __popc(bits & upto_mask));
+            prev += __popc(bits);
+            const bool valid = base + lane < total;
+            if (!valid) owner = 0;
+            const uint2 part = s_part[wib][owner];
+            const uint32_t t = base + lane + part.x;
+            const uint32_t row = t / part.y;
+            const uint32_t x_min = s_gauss[wib][owner].x_min;
+            const uint32_t qx = x_min / (4u * kBoundTile) + (t - row * part.y);
+            const uint32_t ty = s_gauss[wib][owner].y_min / kBoundTile + row;
+            uint32_t front = 0;
+            if (valid) {
+                const uint4 bound = __ldcg(reinterpret_cast<const uint4*>(
+                    a.stq.tile_bound + static_cast<size_t>(ty) * a.stq.bound_pitch + 4u * qx));
+                const uint32_t key_hi = s_gauss[wib][owner].key_hi;
+                front = (bound.x >= key_hi ? 1u : 0u) | (bound.y >= key_hi ? 2u : 0u) | (bound.z >= key_hi ? 4u : 0u) |
+                        (bound.w >= key_hi ? 8u : 0u);
+                // the AABB's tiles of the quad
+                const uint32_t lo = x_min / kBoundTile, hi = (x_min + s_gauss[wib][owner].w - 1u) / kBoundTile;
+                if (lo > 4u * qx) front &= 0xfu << (lo - 4u * qx);
+                if (hi < 4u * qx + 3u) front &= 0xfu >> (4u * qx + 3u - hi);
+            }
+            if (!__any_sync(kFullMask, front != 0)) continue;
+            const uint32_t n_front = __popc(front);
+            const uint32_t place = warp_inclusive_sum(n_front, lane);
+            const uint32_t n_tiles = __shfl_sync(kFullMask, place, 31);
+            uint8_t* at = s_tiles[wib] + (place - n_front);
+            for (uint32_t i = 0; i < 4u; ++i)
+                if (front & (1u << i)) *at++ = static_cast<uint8_t>(lane << 2 | i);
+            __syncwarp();
+            for (uint32_t j = 0; j < n_tiles; j += 32) {
+                const uint32_t tile = s_tiles[wib][min(j + lane, n_tiles - 1u)];
+                const uint32_t tx = 4u * __shfl_sync(kFullMask, qx, tile >> 2) + (tile & 3u);
+                const uint32_t tyy = __shfl_sync(kFullMask, ty, tile >> 2);
+                const uint32_t own = __shfl_sync(kFullMask, owner, tile >> 2);
+                uint32_t todo =
+                    __ballot_sync(kFullMask, j + lane < n_tiles && tile_on_ellipse(s_gauss[wib][own], tx, tyy));
+                if (todo == 0) continue;
+                uint32_t src = __ffs(todo) - 1;
+                uint32_t wx = __shfl_sync(kFullMask, tx, src), wy = __shfl_sync(kFullMask, tyy, src);
+                const size_t below = 4u * static_cast<size_t>(a.cam.width_int);
+                TilePixels px = tile_pixels(a, wx, wy, lane);
+                TileKeys keys = tile_keys(px, 0, below);
+                for (;;) {
+                    const uint32_t gauss = __shfl_sync(kFullMask, own, src);
+                    todo &= todo - 1;
+                    src = todo != 0 ? __ffs(todo) - 1 : src;
+                    const uint32_t nx = __shfl_sync(kFullMask, tx, src), ny = __shfl_sync(kFullMask, tyy, src);
+                    const TilePixels npx = tile_pixels(a, nx, ny, lane);
+                    TileKeys ahead = keys;
+                    if (todo != 0) ahead = tile_keys(npx, 0, below);
+                    walk_tile<kBlue, kHybrid, kMulti>(a, rng, s_gauss[wib][gauss], wx, wy, lane, px, keys);
+                    if (todo == 0) break;
+                    px = npx;
+                    wx = nx;
+                    wy = ny;
+                    keys = ahead;
+                }
+            }
+            __syncwarp();
+        }
+        c0 = n_warps + __shfl_sync(kFullMask, next, 0);
+        claim = next_claim;
+    }
+}
+
+__device__ __forceinline__ void clear_keys(unsigned long long* __restrict__ fb, const size_t n_fb,
+                                           WorkQueue* __restrict__ queue, const size_t tid, const size_t stride) {
     ulonglong2* fb2 = reinterpret_cast<ulonglong2*>(fb);
     const size_t n2 = n_fb / 2;
     for (size_t i = tid; i < n2; i += stride) fb2[i] = make_ulonglong2(kEmptyFragment, kEmptyFragment);
@@ -449,43 +738,98 @@ __global__ void clear_kernel(unsigned long long* __restrict__ fb, const size_t n
             queue->overflow = 0;
             queue->error = 0;
             queue->binned = 0;
+            queue->st_entries = 0;
+            queue->st_items = 0;
+            queue->st_listed = 0;
         }
     }
 }
 
+__global__ void clear_kernel(unsigned long long* __restrict__ fb, const size_t n_fb, WorkQueue* __restrict__ queue) {
+    clear_keys(fb, n_fb, queue, static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x,
+               static_cast<size_t>(gridDim.x) * blockDim.x);
+}
+
+// The clear of a stochastic-transparency pass: also the tile bounds and the depth histogram, and, in
+// the first kSampleBlocks blocks, the AABB pixels of one Gaussian per thread evenly over the scene, from
+// which dense_scene tells how often the larger ones cover the framebuffer.
+__global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams a, const size_t n_fb) {
+    if (blockIdx.x < kSampleBlocks) {
+        __shared__ float s_sum[kWarpsPerBlock];
+        const uint32_t t = blockIdx.x * kBlock + threadIdx.x;
+        const uint32_t step = max(a.n / (kSampleBlocks * kBlock), 1u);
+        bool active = t < a.n;
+        const uint32_t g = active ? t * step : a.n - 1u;
+        Projected p;
+        float pixels = 0.0f;
+        if (project_gaussian(active, g, a.means, a.scales, a.rotations, a.opacities, a.w2c, a.cam, p, a.pre, a.quant) &&
+            active) {
+            const PixelRect rect = pixel_rect(p.bounds, a.cam);
+            pixels = static_cast<float>(rect.width) * static_cast<float>(rect.height);
+            pixels = pixels > static_cast<float>(kDenseMinPixels) ? fminf(pixels, kSampleMaxPixels) * static_cast<float>(step)
+                                                                  : 0.0f;
+        }
+        for (uint32_t o = 16; o > 0; o >>= 1) pixels += __shfl_xor_sync(kFullMask, pixels, o);
+        if ((threadIdx.x & 31u) == 0) s_sum[threadIdx.x >> 5] = pixels;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (uint32_t w = 1; w < kWarpsPerBlock; ++w) pixels += s_sum[w];
+            a.queue->covered[blockIdx.x] = pixels;
+        }
+        return;
+    }
+    const size_t stride = static_cast<size_t>(gridDim.x - kSampleBlocks) * kBlock;
+    const size_t tid = static_cast<size_t>(blockIdx.x - kSampleBlocks) * kBlock + threadIdx.x;
+    clear_keys(a.framebuffer, n_fb, a.queue, tid, stride);
+    for (size_t i = tid; i < static_cast<size_t>(a.stq.bound_pitch) * a.stq.tiles_y; i += stride)
+        a.stq.tile_bound[i] = 0xffffffffu;
+    for (size_t i = tid; i < 2u * kDepthBuckets; i += stride) a.stq.histogram[i] = 0u;
+}
+
 template <bool kBlue, bool kHybrid, bool kMulti>
-void launch_st(const AccumulateParams& p, const unsigned grid, const unsigned queue_grid, cudaStream_t stream) {
-    st_scatter_kernel<kBlue, kHybrid, kMulti><<<grid, kBlock, 0, stream>>>(p);
-    st_queue_kernel<kBlue, kHybrid, kMulti><<<queue_grid, kBlock, 0, stream>>>(p);
+void launch_st(const AccumulateParams& p, const unsigned grid, const int num_sms, cudaStream_t stream) {
+    if (p.stq.log_row_split != 0) st_scatter_kernel<kBlue, kHybrid, kMulti, true><<<grid, kBlock, 0, stream>>>(p);
+    else st_scatter_kernel<kBlue, kHybrid, kMulti, false><<<grid, kBlock, 0, stream>>>(p);
+    if (!isinf(p.stq.dense_pixels)) st_order_kernel<<<static_cast<unsigned>(num_sms), kOrderBlock, 0, stream>>>(p);
+    st_queue_kernel<kBlue, kHybrid, kMulti>
+        <<<static_cast<unsigned>(num_sms) * kQueueBlocksPerSM, kBlock, 0, stream>>>(p);
 }
 
 template <bool kMulti>
-void launch_st_variant(const AccumulateParams& p, const unsigned grid, const unsigned queue_grid, cudaStream_t stream) {
+void launch_st_variant(const AccumulateParams& p, const unsigned grid, const int num_sms, cudaStream_t stream) {
     const bool blue = p.blue_noise != nullptr;
-    if (blue && p.hybrid) launch_st<true, true, kMulti>(p, grid, queue_grid, stream);
-    else if (blue) launch_st<true, false, kMulti>(p, grid, queue_grid, stream);
-    else if (p.hybrid) launch_st<false, true, kMulti>(p, grid, queue_grid, stream);
-    else launch_st<false, false, kMulti>(p, grid, queue_grid, stream);
+    if (blue && p.hybrid) launch_st<true, true, kMulti>(p, grid, num_sms, stream);
+    else if (blue) launch_st<true, false, kMulti>(p, grid, num_sms, stream);
+    else if (p.hybrid) launch_st<false, true, kMulti>(p, grid, num_sms, stream);
+    else launch_st<false, false, kMulti>(p, grid, num_sms, stream);
 }
 
 }  // namespace
 
+namespace {
+unsigned clear_blocks(const size_t n_fb, const int num_sms) {
+    const size_t need = (n_fb / 2 + kBlock - 1) / kBlock;
+    const size_t cap = static_cast<size_t>(num_sms) * 16;
+    return static_cast<unsigned>(need > cap ? cap : (need < 1 ? 1 : need));
+}
+}  // namespace
+
 cudaError_t launch_clear(unsigned long long* framebuffer, const size_t n_fb, WorkQueue* queue, const int num_sms,
                          cudaStream_t stream) {
-    size_t need = (n_fb / 2 + 255) / 256;
-    const size_t cap = static_cast<size_t>(num_sms) * 16;
-    if (need > cap) need = cap;
-    if (need < 1) need = 1;
-    clear_kernel<<<static_cast<unsigned>(need), 256, 0, stream>>>(framebuffer, n_fb, queue);
+    clear_kernel<<<clear_blocks(n_fb, num_sms), kBlock, 0, stream>>>(framebuffer, n_fb, queue);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_clear_st(const AccumulateParams& p, const size_t n_fb, const int num_sms, cudaStream_t stream) {
+    st_clear_kernel<<<kSampleBlocks + clear_blocks(n_fb, num_sms), kBlock, 0, stream>>>(p, n_fb);
     return cudaGetLastError();
 }
 
 cudaError_t launch_accumulate_st(const AccumulateParams& p, const int num_sms, cudaStream_t stream) {
     if (p.n == 0) return cudaSuccess;
-    const unsigned grid = (p.n + kBlock - 1) / kBlock;
-    const unsigned queue_grid = static_cast<unsigned>(num_sms) * kQueueBlocksPerSM;
-    if (p.n_samples > 1) launch_st_variant<true>(p, grid, queue_grid, stream);
-    else launch_st_variant<false>(p, grid, queue_grid, stream);
+    const unsigned grid = (((p.n + 31u) / 32u << p.stq.log_row_split) + kWarpsPerBlock - 1u) / kWarpsPerBlock;
+    if (p.n_samples > 1) launch_st_variant<true>(p, grid, num_sms, stream);
+    else launch_st_variant<false>(p, grid, num_sms, stream);
     return cudaGetLastError();
 }
 

@@ -6,10 +6,12 @@
 // design: outputs and scratch come from the caller (no allocation inside), the frame counter is
 // atomic and settable, all inputs are validated, and no path synchronises with the host (the
 // reference's hybrid paths read device counts back twice per call).
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <cuda_runtime.h>
 #include "../../include/sgs_b200.h"
@@ -29,7 +31,13 @@ std::atomic<uint32_t> g_queue_limit{0};
 
 constexpr size_t kAlign = 256;
 constexpr uint32_t kDefaultMaxBinned = 1u << 20;     // accumulate_hybrid_gps.cu:22
-constexpr uint32_t kStQueueCapacity = 1u << 18;       // large ST Gaussians held by the queue
+constexpr uint32_t kStQueueCapacity = 1u << 18;       // ST queue entries with space of their own
+// Coverage by larger Gaussians (AABB pixels over framebuffer pixels) above which a scene counts as dense
+// (accumulate_st.cu). Either way, in us: the 100k scene at 640x480 (64) 93 sparse, 138 dense; its 400k
+// variant (258) 233, 214; the training scene at 800x800 with 60k (170) 278, 230, with 8 samples 1566, 1131;
+// 40k heavy-tailed at 1279x719 (129) 398, 353; the 6M scene (0 at 640x360) 370, 381.
+constexpr float kDenseCoverage = 128.0f;
+constexpr uint32_t kMinOrdered = 8192;                // Gaussians of a scene that may count as dense
 constexpr uint32_t kMaxSamplesPerCall = 1024;         // sgs_render_samples
 constexpr int kMaxDevices = 64;
 std::atomic<int> g_sm_count[kMaxDevices];
@@ -54,8 +62,11 @@ struct Derived {
     uint32_t ss;
     uint64_t n_fb;
     uint64_t n_pixels;
-    uint32_t queue_capacity;
+    uint32_t queue_capacity;  // GPS queue entries
     uint32_t max_binned;
+    bool st_queue;            // the queue is stochastic transparency's
+    uint32_t st_wanted;       // ST entries the queue would hold with room for all
+    uint32_t tiles_x, tiles_y;
 };
 
 // Validates the arguments that determine sizes; fills the derived sizes.
@@ -72,6 +83,8 @@ int derive(const sgs_gaussians* g, const sgs_camera* c, const sgs_settings* s, D
     d.n_pixels = static_cast<uint64_t>(c->width) * c->height;
     d.queue_capacity = 0;
     d.max_binned = 0;
+    d.st_queue = false;
+    d.st_wanted = d.tiles_x = d.tiles_y = 0;
     if (g->n_gaussians > 0) {
         if (s->use_gps) {
             if (s->hybrid_scheduling) {
@@ -86,11 +99,12 @@ int derive(const sgs_gaussians* g, const sgs_camera* c, const sgs_settings* s, D
             // the Gaussians the reference's hybrid pass gathers (accumulate_hybrid.cu:27,345)
             if (s->hybrid_scheduling)
                 d.max_binned = std::min(s->max_binned != 0 ? s->max_binned : kDefaultMaxBinned, g->n_gaussians);
-            d.queue_capacity = std::min(g->n_gaussians, kStQueueCapacity);
+            d.st_queue = true;
+            d.tiles_x = static_cast<uint32_t>((fbw + 4 * kBoundTile - 1) / (4 * kBoundTile)) * 4;
+            d.tiles_y = static_cast<uint32_t>((fbh + kBoundTile - 1) / kBoundTile);
+            d.st_wanted = std::min(g->n_gaussians, kMaxStEntries);
             const uint32_t cap = g_queue_limit.load(std::memory_order_relaxed);
-            if (cap != 0) d.queue_capacity = std::min(d.queue_capacity, cap);
-            const uint64_t limit = 0xffffffffull / std::max<uint64_t>(fbh, 1);
-            if (d.queue_capacity > limit) d.queue_capacity = static_cast<uint32_t>(limit);
+            if (cap != 0) d.st_wanted = std::min(d.st_wanted, cap);
         }
     }
     return SGS_OK;
@@ -99,6 +113,11 @@ int derive(const sgs_gaussians* g, const sgs_camera* c, const sgs_settings* s, D
 struct FullLayout {
     sgs_workspace_layout pub;
     size_t q_key, q_geom, q_geom2, q_meta, q_count;
+    // stochastic transparency: the queue's own entries at q_key; tile bounds, depth histogram, list and
+    // further entries (st_b) borrow the samples section, which the accumulate passes leave unused, or
+    // lie in a section of their own where it is too small
+    size_t tile_bound, histogram, list, st_b;
+    uint32_t st_own, st_capacity;
 };
 
 FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n_samples = 1) {
@@ -113,8 +132,39 @@ FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n
     off = align_up(off + d.n_fb * sizeof(float4));
     L.reuse_weights = off;
     if (s->spatial_reuse) off = align_up(off + d.n_fb * sizeof(float4));
-    const size_t q = d.queue_capacity;
     F.q_key = off;
+    if (d.st_queue) {
+        // 60 bytes for each of min(N, 2^18) entries in any case; more where the workspace stays within the
+        // scratch of the allocation-free render (several samples per call never run there)
+        const size_t bounds = align_up(static_cast<size_t>(d.tiles_x) * d.tiles_y * sizeof(uint32_t));
+        const size_t fixed = bounds + align_up(2 * kDepthBuckets * sizeof(uint32_t));
+        constexpr size_t kListBytes = kItemsPerEntry * sizeof(uint32_t);
+        const size_t room = d.n_fb * sizeof(float4);
+        size_t own = std::max<size_t>(std::min(d.st_wanted, kStQueueCapacity) * size_t(60) / kStEntryBytes, 1);
+        const bool borrow = fixed + align_up(own * kListBytes) <= room;
+        if (borrow) {
+            const size_t listed = (room - fixed) / kListBytes - kAlign / kListBytes;
+            const size_t spare =
+                n_samples > 1 ? d.st_wanted : (kNoAllocScratchBytes - std::min(off, kNoAllocScratchBytes)) / kStEntryBytes;
+            own = std::max(own, std::min({static_cast<size_t>(d.st_wanted), spare, listed}));
+        }
+        F.st_own = static_cast<uint32_t>(own);
+        off = align_up(off + own * kStEntryBytes);
+        F.tile_bound = borrow ? L.samples : off;
+        F.histogram = F.tile_bound + bounds;
+        F.list = F.tile_bound + fixed;
+        F.st_capacity = F.st_own;
+        if (borrow && d.st_wanted > own) {
+            const size_t used = fixed + align_up(own * kListBytes) + kAlign;
+            const size_t more = room > used ? (room - used) / (kStEntryBytes + kListBytes) : 0;
+            F.st_capacity += static_cast<uint32_t>(std::min<size_t>(d.st_wanted - own, more));
+        }
+        F.st_b = F.list + align_up(F.st_capacity * kListBytes);
+        if (!borrow) off = F.st_b;
+        L.total = off;
+        return F;
+    }
+    const size_t q = d.queue_capacity;
     off = align_up(off + q * sizeof(unsigned long long));
     F.q_geom = off;
     off = align_up(off + q * sizeof(float4));
@@ -277,6 +327,30 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
     w.q.meta = reinterpret_cast<uint4*>(ws + F.q_meta);
     w.q.count = reinterpret_cast<uint32_t*>(ws + F.q_count);
     w.q.capacity = d.queue_capacity;
+    StQueue stq{};
+    if (d.st_queue) {
+        stq.a = ws + F.q_key;
+        stq.b = ws + F.st_b;
+        stq.entries_a = F.st_own;
+        stq.capacity = F.st_capacity;
+        // a queue of a few thousand entries is not worth the order pass's launch
+        stq.dense_pixels = g->n_gaussians < kMinOrdered ? std::numeric_limits<float>::infinity()
+                                                        : kDenseCoverage * static_cast<float>(d.n_fb);
+        // Few Gaussians leave the chip idle while single warps walk the rows of 32 large ones: 2^split
+        // warps share them (640x480, 100k: 117 to 93 us; 640x480 training scene of 30k, 8 samples: 1012 to
+        // 785 us). From 256k up the repeated projections cost more than that gains. Hybrid scheduling
+        // counts the first max_binned large Gaussians, which must not be counted twice.
+        stq.log_row_split = g->n_gaussians < (1u << 16) ? 3u : g->n_gaussians < (1u << 18) ? 2u : 0u;
+        if (s->hybrid_scheduling && static_cast<uint64_t>(g->n_gaussians) << stq.log_row_split > d.max_binned)
+            stq.log_row_split = 0;
+        stq.list = reinterpret_cast<uint32_t*>(ws + F.list);
+        stq.list_capacity = kItemsPerEntry * F.st_capacity;
+        stq.histogram = reinterpret_cast<uint32_t*>(ws + F.histogram);
+        stq.tile_bound = reinterpret_cast<uint32_t*>(ws + F.tile_bound);
+        stq.bound_pitch = d.tiles_x;
+        stq.tiles_y = d.tiles_y;
+        stq.height = c->height * d.ss;
+    }
 
     const PassCamera cam = pass_camera(c, s, d.ss);
     AccumulateParams ap{};
@@ -297,6 +371,7 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
     ap.hybrid = s->hybrid_scheduling != 0;
     ap.queue = w.queue;
     ap.q = w.q;
+    ap.stq = stq;
     ap.n_samples = n_samples;
     ap.fb_stride = d.n_fb;
     ap.pre = reinterpret_cast<const float4*>(g->preactivated);
@@ -348,7 +423,8 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
 
     // the clear and accumulate passes of one framebuffer (or, with p.n_samples > 1, of all of them)
     auto accumulate = [&](const AccumulateParams& p, const size_t n_clear) -> int {
-        cudaError_t err = launch_clear(p.framebuffer, n_clear, w.queue, sms, acc_stream);
+        cudaError_t err = d.st_queue ? launch_clear_st(p, n_clear, sms, acc_stream)
+                                    : launch_clear(p.framebuffer, n_clear, w.queue, sms, acc_stream);
         if (err != cudaSuccess) return fail(SGS_ERROR_CUDA, "clear: %s", cudaGetErrorString(err));
         if (g->n_gaussians == 0) return SGS_OK;
         if (t_stage_start != nullptr) cudaEventRecord(t_stage_start, acc_stream);

@@ -17,8 +17,12 @@ struct WorkQueue {
     unsigned int overflow;       // producers that found the queue full (processed in place)
     unsigned int error;          // nonzero when a consumer met an inconsistent entry
     unsigned int binned;         // hybrid ST: Gaussians the reference would gather, in arrival order
-    unsigned int pad[2];
+    unsigned int st_entries;     // ST: entries and list items reserved by producers
+    unsigned int st_items;
+    unsigned int st_listed;      // ST: items the order pass has listed
+    alignas(16) float covered[4];  // ST: AABB pixels of the scene, estimated by kSampleBlocks blocks of the clear pass
 };
+static_assert(offsetof(WorkQueue, covered) % 16 == 0, "read as one float4");
 constexpr unsigned long long kQueueEntryShift = 40;
 constexpr unsigned long long kQueueChunkMask = (1ull << kQueueEntryShift) - 1;
 // Producers queue chunk indices below this, so the consumers' cursor (which overshoots the last chunk
@@ -28,13 +32,52 @@ constexpr unsigned long long kMaxQueueChunks = 0xffffffffull - (1ull << 24);
 // kMaxQueueChunks (above every chunk index, so the entry search never returns it).
 constexpr uint32_t kUnusedQueueEntry = 0xffffffffu;
 
-// Per-entry arrays of the large-Gaussian queue (structure of arrays, 16-byte aligned).
+// Scratch of the allocation-free render (render_no_alloc.cu). The stochastic-transparency queue takes
+// more than its 2^18 entries only while a one-sample workspace stays within it.
+constexpr size_t kNoAllocScratchBytes = size_t(64) << 20;
+
+// ---- stochastic-transparency queue: entries in depth order, depth bounds per tile ----
+constexpr uint32_t kStEntryBytes = 64;
+constexpr uint32_t kBoundTile = 8;        // pixels per side of a tile with a depth bound
+constexpr uint32_t kDepthBuckets = 1024;  // 1/32 octave each over view depths of 2^-16 .. 2^16
+constexpr uint32_t kSampleBlocks = 4;
+// A list item is a part (32 quads of tiles, at most kMaxParts parts) of an entry: part << kItemEntryBits | entry.
+constexpr uint32_t kItemEntryBits = 20;
+constexpr uint32_t kItemEntryMask = (1u << kItemEntryBits) - 1u;
+constexpr uint32_t kMaxParts = 1u << (32u - kItemEntryBits);
+constexpr uint32_t kNoItem = 0xffffffffu;  // an unused list place (the last entry has no such part: kMaxStEntries)
+constexpr uint32_t kMaxStEntries = kItemEntryMask;
+constexpr uint32_t kItemsPerEntry = 4;     // list places per entry
+
+struct StQueue {
+    void* a;                        // the first entries_a entries, kStEntryBytes each
+    void* b;                        // the others
+    uint32_t entries_a;
+    uint32_t capacity;              // entries in all, at most kMaxStEntries
+    float dense_pixels;             // covered pixels above which the scene counts as dense
+    uint32_t log_row_split;         // warps sharing 32 Gaussians in the scatter pass
+    uint32_t* list;                 // items in the consumers' order
+    uint32_t list_capacity;
+    uint32_t* histogram;            // items per depth bucket, then the order pass's cursors
+    uint32_t* tile_bound;           // per tile, an upper bound of its keys' depth bits; null: not kept
+    uint32_t bound_pitch, tiles_y;  // tiles per row (a multiple of 4) and rows
+    uint32_t height;                // framebuffer rows
+};
+
+// Depth bucket of a key's high word; depths off the range share the end buckets (the order only
+// decides how much is culled, never the winners).
+__device__ __forceinline__ uint32_t depth_bucket(const uint32_t depth_bits) {
+    const int b = static_cast<int>(depth_bits >> 18) - ((127 - 16) << 5);
+    return static_cast<uint32_t>(min(max(b, 0), static_cast<int>(kDepthBuckets) - 1));
+}
+
+// Per-entry arrays of the GPS large-Gaussian queue (structure of arrays, 16-byte aligned).
 struct QueueArrays {
     unsigned long long* key;  // packed fragment key
-    float4* geom;             // ST: mean2d - 0.5 (x, y), exp2-scaled conic (x, y); GPS: mean2d, L.x, L.y
-    float4* geom2;            // ST: conic z, opacity, x_min, width (bit casts); GPS: L.z, power threshold, opacity_rcp, dilog
-    uint4* meta;              // ST: y_min, height, rows per chunk, first chunk; GPS: conic x/y/z bits, first chunk
-    uint32_t* count;          // GPS: number of points
+    float4* geom;             // mean2d, L.x, L.y
+    float4* geom2;            // L.z, power threshold, opacity_rcp, dilog
+    uint4* meta;              // conic x/y/z bits, first chunk
+    uint32_t* count;          // number of points
     uint32_t capacity;
 };
 
@@ -85,6 +128,7 @@ struct AccumulateParams {
     bool hybrid;                      // hybrid scheduling
     WorkQueue* queue;
     QueueArrays q;
+    StQueue stq;
     uint32_t n_samples;               // samples of one call (frames frame .. frame + n_samples - 1)
     size_t fb_stride;                 // framebuffer elements between consecutive samples' framebuffers
     const float4* pre;                // preactivated layout (2 float4 per Gaussian) or null
@@ -116,6 +160,7 @@ __device__ __forceinline__ FrameRng frame_rng(const AccumulateParams& a) {
 
 cudaError_t launch_clear(unsigned long long* framebuffer, size_t n_fb, WorkQueue* queue, int num_sms,
                          cudaStream_t stream);
+cudaError_t launch_clear_st(const AccumulateParams& p, size_t n_fb, int num_sms, cudaStream_t stream);
 cudaError_t launch_accumulate_st(const AccumulateParams& p, int num_sms, cudaStream_t stream);
 cudaError_t launch_accumulate_gps(const AccumulateParams& p, int num_sms, cudaStream_t stream);
 cudaError_t launch_quantize(const float* means, const float* scales, const float4* rotations, const float* opacities,
