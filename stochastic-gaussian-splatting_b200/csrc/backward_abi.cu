@@ -46,6 +46,7 @@ int setup(const sgs_gaussians* g, const sgs_camera* c, const sgs_settings* s, Ba
     p.cam_position = c->cam_position;
     p.n = g->n_gaussians;
     p.sh_bases = g->sh_bases;
+    p.sh_vec4 = g->sh_bases == 16 && (reinterpret_cast<uintptr_t>(g->sh_coefficients) & 15u) == 0;
     p.cam.width = static_cast<float>(c->width * ss);
     p.cam.height = static_cast<float>(c->height * ss);
     p.cam.focal_x = c->focal_x * ssf;
@@ -60,6 +61,8 @@ int setup(const sgs_gaussians* g, const sgs_camera* c, const sgs_settings* s, Ba
     p.width = c->width;
     p.ss = ss;
     p.n_fb = c->width * ss * c->height * ss;
+    p.tiles_x = (c->width * ss + kBoundTile - 1) / kBoundTile;
+    p.tiles_y = (c->height * ss + kBoundTile - 1) / kBoundTile;
     out.gps = s->use_gps != 0;
     out.gps_law = nullptr;
     return SGS_OK;
@@ -69,17 +72,19 @@ constexpr uint32_t kMaxFusedSamples = 1024;
 
 size_t align256(const size_t v) { return (v + 255) & ~size_t(255); }
 
-// Interleaved per-pixel sample table of the fused backward: keys, then terms, the per-pixel largest
-// key, and for GPS the count-law table (returned; null without GPS).
+// Interleaved per-pixel sample table of the fused backward: keys, then terms, 8 bytes per pixel for the
+// pixels' and the tiles' largest depths (4 each; there are no more tiles than pixels), and for GPS the
+// count-law table (returned; null without GPS).
 float2* set_sample_table(BackwardParams& p, void* scratch, const uint32_t n_samples, const bool gps) {
     p.n_samples = n_samples;
     p.pix_keys = static_cast<unsigned long long*>(scratch);
     const size_t keys = align256(sizeof(unsigned long long) * p.n_fb * static_cast<size_t>(n_samples));
     const size_t terms = align256(sizeof(float) * p.n_fb * static_cast<size_t>(n_samples));
-    const size_t max_keys = align256(sizeof(unsigned long long) * p.n_fb);
+    const size_t depths = align256(2 * sizeof(uint32_t) * static_cast<size_t>(p.n_fb));
     p.pix_terms = reinterpret_cast<float*>(static_cast<char*>(scratch) + keys);
-    p.pix_max_key = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) + keys + terms);
-    return gps ? reinterpret_cast<float2*>(static_cast<char*>(scratch) + keys + terms + max_keys) : nullptr;
+    p.pix_far = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + keys + terms);
+    p.tile_far = p.pix_far + p.n_fb;
+    return gps ? reinterpret_cast<float2*>(static_cast<char*>(scratch) + keys + terms + depths) : nullptr;
 }
 
 cudaError_t launch_walk(const BackwardSetup& S, cudaStream_t stream) {
@@ -168,7 +173,7 @@ size_t sgs_backward_samples_scratch_size(const sgs_camera* camera, const sgs_set
     const uint32_t ss = settings->supersampling_factor < 1 ? 1u : static_cast<uint32_t>(settings->supersampling_factor);
     const size_t n_fb = static_cast<size_t>(camera->width) * ss * camera->height * ss;
     return align256(sizeof(unsigned long long) * n_fb * n_samples) + align256(sizeof(float) * n_fb * n_samples) +
-           align256(sizeof(unsigned long long) * n_fb) + (settings->use_gps ? align256(gps_count_law_bytes()) : 0);
+           align256(2 * sizeof(uint32_t) * n_fb) + (settings->use_gps ? align256(gps_count_law_bytes()) : 0);
 }
 
 size_t sgs_gps_count_law_size(void) { return gps_count_law_bytes(); }

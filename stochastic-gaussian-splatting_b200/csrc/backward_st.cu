@@ -26,9 +26,11 @@ namespace {
 
 constexpr uint32_t kBlock = 256;
 constexpr uint32_t kWarpsPerBlock = kBlock / 32;
+constexpr uint32_t kProjectionBlock = 128;
 constexpr uint32_t kFullMask = 0xffffffffu;
 constexpr uint32_t kCoopFragments = 64;  // larger AABBs are processed by the whole warp
-constexpr uint32_t kBigFragments = 2048;  // fused walk: larger AABBs go to the row-chunk queue
+constexpr uint32_t kBigFragments = 256;   // fused walk: larger AABBs go to the row-chunk queue
+constexpr uint32_t kMaxLaneTiles = 16;    // AABBs of at most this many tiles are tested by their lane
 constexpr uint32_t kChunkPixels = 2048;   // pixels per stolen chunk (whole rows, at most 32)
 constexpr uint32_t kQueueBlocksPerSM = 8;
 constexpr int kAccum = 10;               // op, conic x/y/z, mean2d x/y, depth, colour r/g/b
@@ -252,7 +254,27 @@ __device__ __forceinline__ GpsFragment gps_fragment(const float cx, const float 
     return f;
 }
 
+// The SH coefficients of Gaussian g, degree 3 as twelve 16-byte loads where the array allows it.
+template <int kBases>
+__device__ __forceinline__ void load_sh(const BackwardParams& b, const uint32_t g, float c[kBases * 3]) {
+    const float* const src = b.sh + static_cast<size_t>(g) * (kBases * 3);
+    if (kBases == 16 && b.sh_vec4) {
+#pragma unroll
+        for (int i = 0; i < 12; ++i) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(src) + i);
+            c[4 * i + 0] = v.x;
+            c[4 * i + 1] = v.y;
+            c[4 * i + 2] = v.z;
+            c[4 * i + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kBases * 3; ++i) c[i] = src[i];
+    }
+}
+
 // View-dependent colour of every Gaussian (the colour its fragments would give a pixel).
+template <int kBases>
 __global__ void __launch_bounds__(kBlock) colors_kernel(const BackwardParams b) {
     const uint32_t g = blockIdx.x * kBlock + threadIdx.x;
     if (g >= b.n) return;
@@ -260,8 +282,9 @@ __global__ void __launch_bounds__(kBlock) colors_kernel(const BackwardParams b) 
     const float vy = b.means[3 * g + 1] - b.cam_position[1];
     const float vz = b.means[3 * g + 2] - b.cam_position[2];
     const float inv_len = rsqrtf(vx * vx + vy * vy + vz * vz);
-    const float3 c = eval_sh(b.sh + static_cast<size_t>(g) * b.sh_bases * 3, vx * inv_len, vy * inv_len, vz * inv_len,
-                             b.sh_bases);
+    float sh[kBases * 3];
+    load_sh<kBases>(b, g, sh);
+    const float3 c = eval_sh(sh, vx * inv_len, vy * inv_len, vz * inv_len, kBases);
     b.colors[3 * g + 0] = c.x;
     b.colors[3 * g + 1] = c.y;
     b.colors[3 * g + 2] = c.z;
@@ -375,9 +398,10 @@ __global__ void __launch_bounds__(kBlock) fragments_backward_kernel(const Backwa
 // geometric factors once and sums the S samples' contributions:
 //   dL/da_k = ge (g . c_k + g_d z_k) - sum_{key_w > key_k} T / (1 - a_k) + g_a n_none / (1 - a_k)
 // with ge = #samples whose winner is not in front of k and n_none = #samples with no winner.
-// A fragment behind every sample's winner (key_k > the pixel's largest winner key, an empty pixel
-// counting as the largest key) contributes exactly zero; the walk tests that first, so the per-sample
-// table is read only for the fragments in front of some winner.
+// A fragment behind every sample's winner (its depth larger than the pixel's largest winner depth, an
+// empty pixel counting as the largest) contributes exactly zero; the walk tests that first, for whole
+// Gaussians and chunks by the tiles' largest depths, so the per-sample table is read only for the
+// fragments in front of some winner.
 
 __global__ void __launch_bounds__(kBlock) sample_terms_kernel(const BackwardParams b) {
     const uint32_t pix = blockIdx.x * kBlock + threadIdx.x;
@@ -392,7 +416,8 @@ __global__ void __launch_bounds__(kBlock) sample_terms_kernel(const BackwardPara
     b.pix_keys[slot] = key;
     b.pix_terms[slot] = t * b.grad_scale;
     // the farthest winner of the samples so far (launches are ordered: sample 0 starts the maximum)
-    b.pix_max_key[pix] = b.sample == 0 ? key : max(b.pix_max_key[pix], key);
+    const uint32_t far = static_cast<uint32_t>(key >> 32);
+    b.pix_far[pix] = b.sample == 0 ? far : max(b.pix_far[pix], far);
 }
 
 // The same table from the framebuffers of all S samples at once (consecutive, b.n_fb apart): the
@@ -405,7 +430,7 @@ __global__ void __launch_bounds__(kBlock) framebuffer_terms_kernel(const Backwar
     const uint32_t ip = (py / b.ss) * b.width + px / b.ss;
     const float g0 = b.grad_image[3 * ip + 0], g1 = b.grad_image[3 * ip + 1], g2 = b.grad_image[3 * ip + 2];
     const float gd = b.grad_depth != nullptr ? b.grad_depth[ip] : 0.0f;
-    unsigned long long max_key = 0;
+    uint32_t far = 0;
     const size_t row = static_cast<size_t>(pix) * b.n_samples;
     for (uint32_t s = 0; s < b.n_samples; ++s) {
         const unsigned long long key = b.framebuffer[static_cast<size_t>(s) * b.n_fb + pix];
@@ -417,9 +442,27 @@ __global__ void __launch_bounds__(kBlock) framebuffer_terms_kernel(const Backwar
         }
         b.pix_keys[row + s] = key;
         b.pix_terms[row + s] = t * b.grad_scale;
-        max_key = max(max_key, key);
+        far = max(far, static_cast<uint32_t>(key >> 32));
     }
-    b.pix_max_key[pix] = max_key;
+    b.pix_far[pix] = far;
+}
+
+// Per 8 x 8 tile of the framebuffer, the largest depth bits of its pixels' farthest winners (all ones
+// where a pixel of some sample is empty): a Gaussian behind that adds exactly zero in the tile. One
+// warp per tile, two pixels per lane.
+__global__ void __launch_bounds__(kBlock) tile_far_kernel(const BackwardParams b) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t tile = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    if (tile >= b.tiles_x * b.tiles_y) return;
+    const uint32_t width = b.cam.width_int, height = b.n_fb / width;
+    const uint32_t x = tile % b.tiles_x * kBoundTile + (lane & 7u);
+    const uint32_t y = tile / b.tiles_x * kBoundTile + (lane >> 3);
+    const uint32_t* const p = b.pix_far + (static_cast<size_t>(y) * width + x);
+    uint32_t far = 0;
+    if (x < width && y < height) far = p[0];
+    if (x < width && y + 4u < height) far = max(far, p[4u * static_cast<size_t>(width)]);
+    far = __reduce_max_sync(kFullMask, far);
+    if (lane == 0) b.tile_far[tile] = far;
 }
 
 // Rows per chunk of a queued Gaussian of AABB width w (log2): about kChunkPixels pixels, a power of
@@ -487,7 +530,7 @@ __device__ __forceinline__ void walk_row_gradients(const BackwardParams& b, cons
     uint32_t ix = xs / b.ss, sub = xs - ix * b.ss;
     float fx = static_cast<float>(xs);
     for (uint32_t i = 0; i < steps; ++i) {
-        if (i < len && key_k <= b.pix_max_key[pix0 + i]) {
+        if (i < len && q.key_hi <= b.pix_far[pix0 + i]) {
             const float dx = fx - q.mx;
             const float e = dx * (q.cx * dx + cydy) + czdy * dy;
             const float alpha = q.opacity * exp2f(fminf(e, 0.0f));
@@ -580,6 +623,47 @@ __global__ void __launch_bounds__(kBlock) fragments_samples_kernel(const Backwar
     if (!project_gaussian(active, g, b.means, b.scales, b.rotations, b.opacities, b.w2c, b.cam, p)) return;
     const PixelRect rect = pixel_rect(p.bounds, b.cam);
     bool has_rows = active && rect.width > 0 && rect.height > 0;
+    // behind every winner of its tiles: all gradients are zero. Few tiles are tested by the Gaussian's lane,
+    // more by the whole warp.
+    const uint32_t tx0 = rect.x_min / kBoundTile, tw = (rect.x_min + rect.width - 1u) / kBoundTile - tx0 + 1u;
+    const uint32_t ty0 = rect.y_min / kBoundTile, th = (rect.y_min + rect.height - 1u) / kBoundTile - ty0 + 1u;
+    const uint32_t depth = __float_as_uint(p.depth);
+    const bool many_tiles = has_rows && tw * th > kMaxLaneTiles;
+    if (has_rows && !many_tiles) {
+        has_rows = false;
+        for (uint32_t ty = 0; ty < th && !has_rows; ++ty)
+            for (uint32_t tx = 0; tx < tw && !has_rows; ++tx)
+                has_rows = __ldg(b.tile_far + (ty0 + ty) * b.tiles_x + tx0 + tx) >= depth;
+    }
+    for (uint32_t pending = __ballot_sync(kFullMask, many_tiles); pending != 0; pending &= pending - 1) {
+        const uint32_t src = __ffs(pending) - 1;
+        const uint32_t sx = __shfl_sync(kFullMask, tx0, src), sy = __shfl_sync(kFullMask, ty0, src);
+        const uint32_t sw = __shfl_sync(kFullMask, tw, src), n = sw * __shfl_sync(kFullMask, th, src);
+        const uint32_t sd = __shfl_sync(kFullMask, depth, src);
+        bool front = false;
+        for (uint32_t t = 0; t < n && !front; t += 32u) {
+            const uint32_t row = (t + lane) / sw;
+            front = __any_sync(kFullMask, t + lane < n && __ldg(b.tile_far + (sy + row) * b.tiles_x + sx + t + lane -
+                                                                row * sw) >= sd);
+        }
+        if (lane == src && !front) has_rows = false;
+    }
+    // large footprints go to the queue (walked in row chunks across all SMs) unless it is full; one atomic per warp
+    const bool large = has_rows && rect.width * rect.height > kBigFragments;
+    const uint32_t log_rpc = log_chunk_rows(rect.width);
+    const uint32_t chunks = large ? (rect.height + (1u << log_rpc) - 1u) >> log_rpc : 0u;
+    const uint32_t larges = __ballot_sync(kFullMask, large);
+    uint32_t entry_at = 0xffffffffu;
+    unsigned long long first_chunk = 0;
+    if (larges != 0) {
+        const uint32_t incl = warp_inclusive_sum(chunks, lane);
+        unsigned long long old = 0;
+        if (lane == 31)
+            old = atomicAdd(&b.bw_queue->packed, (static_cast<unsigned long long>(__popc(larges)) << kQueueEntryShift) | incl);
+        old = __shfl_sync(kFullMask, old, 31);
+        if (large) entry_at = static_cast<uint32_t>(old >> kQueueEntryShift) + __popc(larges & lt_mask);
+        first_chunk = (old & kQueueChunkMask) + (incl - chunks);
+    }
     WalkGaussian q;
     GpsConstants c{};
     if (kGps && has_rows) c = gps_constants(p);
@@ -606,23 +690,17 @@ __global__ void __launch_bounds__(kBlock) fragments_samples_kernel(const Backwar
         q.y_min = rect.y_min;
         q.w = rect.width;
         q.row_first = 0;
-        // large footprints go to the queue (walked in row chunks across all SMs) unless it is full
-        if (rect.width * rect.height > kBigFragments) {
-            const uint32_t log_rpc = log_chunk_rows(rect.width);
-            const uint32_t chunks = (rect.height + (1u << log_rpc) - 1u) >> log_rpc;
-            const unsigned long long old = atomicAdd(&b.bw_queue->packed, (1ull << kQueueEntryShift) | chunks);
-            const uint32_t e = static_cast<uint32_t>(old >> kQueueEntryShift);
-            const unsigned long long first_chunk = old & kQueueChunkMask;
-            if (e < b.bw_capacity && first_chunk + chunks <= kMaxQueueChunks) {
-                WalkEntry* entry = static_cast<WalkEntry*>(b.bw_entries) + e;
+        if (entry_at < b.bw_capacity) {
+            if (first_chunk + chunks <= kMaxQueueChunks) {
+                WalkEntry* entry = static_cast<WalkEntry*>(b.bw_entries) + entry_at;
                 entry->g = q;
                 if (kGps) entry->c = c;
-                b.bw_meta[e] = make_uint4(rect.y_min, rect.height, log_rpc, static_cast<uint32_t>(first_chunk));
-                b.bw_index[e] = g;
+                b.bw_meta[entry_at] = make_uint4(rect.y_min, rect.height, log_rpc, static_cast<uint32_t>(first_chunk));
+                b.bw_index[entry_at] = g;
                 has_rows = false;
-            } else if (e < b.bw_capacity) {
+            } else {
                 // past 32-bit chunk indices: marked unused (the marked entries are the last ones), walked here
-                b.bw_meta[e] = make_uint4(0u, 0u, 0u, kUnusedQueueEntry);
+                b.bw_meta[entry_at] = make_uint4(0u, 0u, 0u, kUnusedQueueEntry);
             }
         }
     }
@@ -689,12 +767,7 @@ __global__ void __launch_bounds__(kBlock) fragments_samples_queue_kernel(const B
         if (lane == 0) c = atomicAdd(&b.bw_queue->next_chunk, 1u);
         c = __shfl_sync(kFullMask, c, 0);
         if (c >= n_chunks) break;
-        uint32_t lo = 0, hi = n_entries - 1;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (b.bw_meta[mid].w <= c) lo = mid;
-            else hi = mid - 1;
-        }
+        const uint32_t lo = queue_entry_of_chunk(b.bw_meta, n_entries, c, lane);
         const uint4 m = b.bw_meta[lo];
         const uint32_t log_rows = m.z;
         const uint32_t r0 = (c - m.w) << log_rows;
@@ -703,6 +776,16 @@ __global__ void __launch_bounds__(kBlock) fragments_samples_queue_kernel(const B
             continue;
         }
         const WalkGaussian q = entries[lo].g;
+        // the chunk's tiles, one per lane: behind the winners of all of them nothing is added
+        const uint32_t rows = min(1u << log_rows, m.y - r0);
+        const uint32_t tx0 = q.x_min / kBoundTile, tw = (q.x_min + q.w - 1u) / kBoundTile - tx0 + 1u;
+        const uint32_t ty0 = (q.y_min + r0) / kBoundTile, th = (q.y_min + r0 + rows - 1u) / kBoundTile - ty0 + 1u;
+        bool front = false;
+        for (uint32_t t = lane; t < tw * th && !front; t += 32u) {
+            const uint32_t ty = t / tw;
+            front = __ldg(b.tile_far + (ty0 + ty) * b.tiles_x + tx0 + (t - ty * tw)) >= q.key_hi;
+        }
+        if (!__any_sync(kFullMask, front)) continue;
         const GpsConstants gc = kGps ? entries[lo].c : GpsConstants{};
         const uint32_t r = r0 + (lane & ((1u << log_rows) - 1u));
         FragAccum acc;
@@ -741,24 +824,32 @@ __device__ __forceinline__ void sh_basis(const float x, const float y, const flo
     Y[15] = x * (kSH3b * yy - kSH3a * xx); dY[15][0] = kSH3b * yy - 3.0f * kSH3a * xx; dY[15][1] = 2.0f * kSH3b * x * y; dY[15][2] = 0;
 }
 
-// Projection backward (gs_utils.h:38-193 differentiated): accumulated projected-quantity gradients to
-// the parameters. Culled Gaussians receive zero gradients.
-__global__ void __launch_bounds__(kBlock) projection_backward_kernel(const BackwardParams b) {
-    const uint32_t g = blockIdx.x * kBlock + threadIdx.x;
-    if (g >= b.n) return;
-    const float* acc = b.accum + static_cast<size_t>(g) * kAccum;
-    float* dm = b.d_means + 3 * g;
-    float* ds = b.d_scales + 3 * g;
-    float* dq = b.d_rotations + 4 * g;
-    float* dsh = b.d_sh + static_cast<size_t>(g) * b.sh_bases * 3;
-    dm[0] = dm[1] = dm[2] = 0.0f;
-    ds[0] = ds[1] = ds[2] = 0.0f;
-    dq[0] = dq[1] = dq[2] = dq[3] = 0.0f;
-    b.d_opacities[g] = 0.0f;
-    for (uint32_t i = 0; i < b.sh_bases * 3; ++i) dsh[i] = 0.0f;
+// Gradients of one Gaussian's mean, log-scales, quaternion and opacity logit from its accumulated
+// projected-quantity gradients (gs_utils.h:38-193 differentiated), and the factors of its SH gradients
+// (coefficient k, channel ch: Y[k] gc[ch]). A culled Gaussian has zero gradients.
+template <int kBases>
+__device__ __forceinline__ void gaussian_gradients(const BackwardParams& b, const uint32_t g, float Y[kBases],
+                                                   float gc[3]) {
+    float acc[kAccum];
     bool any = false;
-    for (int i = 0; i < kAccum; ++i) any |= acc[i] != 0.0f;
-    if (!any) return;
+#pragma unroll
+    for (int i = 0; i < kAccum; ++i) {
+        acc[i] = b.accum[static_cast<size_t>(g) * kAccum + i];
+        any |= acc[i] != 0.0f;
+    }
+    float* dm = b.d_means + 3 * static_cast<size_t>(g);
+    float* ds = b.d_scales + 3 * static_cast<size_t>(g);
+    float* dq = b.d_rotations + 4 * static_cast<size_t>(g);
+    if (!any) {
+        dm[0] = dm[1] = dm[2] = 0.0f;
+        ds[0] = ds[1] = ds[2] = 0.0f;
+        dq[0] = dq[1] = dq[2] = dq[3] = 0.0f;
+        b.d_opacities[g] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < kBases; ++k) Y[k] = 0.0f;
+        gc[0] = gc[1] = gc[2] = 0.0f;
+        return;
+    }
 
     const float mx = b.means[3 * g], my = b.means[3 * g + 1], mz = b.means[3 * g + 2];
     const float4 r1 = b.w2c[0], r2 = b.w2c[1], r3 = b.w2c[2];
@@ -883,29 +974,68 @@ __global__ void __launch_bounds__(kBlock) projection_backward_kernel(const Backw
     const float dvx = mx - b.cam_position[0], dvy = my - b.cam_position[1], dvz = mz - b.cam_position[2];
     const float len = sqrtf(dvx * dvx + dvy * dvy + dvz * dvz);
     const float dir[3] = {dvx / len, dvy / len, dvz / len};
-    float Y[16], dY[16][3];
-    sh_basis(dir[0], dir[1], dir[2], Y, dY);
-    const float* shg = b.sh + static_cast<size_t>(g) * b.sh_bases * 3;
-    const float* col = b.colors + 3 * g;
+    float Y16[16], dY[16][3];
+    sh_basis(dir[0], dir[1], dir[2], Y16, dY);
+    float sh[kBases * 3];
+    load_sh<kBases>(b, g, sh);
+    const float* col = b.colors + 3 * static_cast<size_t>(g);
     float ddir[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int k = 0; k < kBases; ++k) Y[k] = Y16[k];
+#pragma unroll
     for (int ch = 0; ch < 3; ++ch) {
-        const float gc = col[ch] > 0.0f ? acc[7 + ch] : 0.0f;
-        for (uint32_t k = 0; k < b.sh_bases; ++k) {
-            dsh[3 * k + ch] = gc * Y[k];
-            ddir[0] += gc * shg[3 * k + ch] * dY[k][0];
-            ddir[1] += gc * shg[3 * k + ch] * dY[k][1];
-            ddir[2] += gc * shg[3 * k + ch] * dY[k][2];
+        gc[ch] = col[ch] > 0.0f ? acc[7 + ch] : 0.0f;
+#pragma unroll
+        for (int k = 0; k < kBases; ++k) {
+            ddir[0] += gc[ch] * sh[3 * k + ch] * dY[k][0];
+            ddir[1] += gc[ch] * sh[3 * k + ch] * dY[k][1];
+            ddir[2] += gc[ch] * sh[3 * k + ch] * dY[k][2];
         }
     }
     const float dd = ddir[0] * dir[0] + ddir[1] * dir[1] + ddir[2] * dir[2];
     for (int k = 0; k < 3; ++k) dm[k] = gm[k] + (ddir[k] - dir[k] * dd) / len;
 }
 
+// One thread per Gaussian; the SH gradients, 4/5 of the bytes, are then written by whole warps (a
+// thread's own 48 floats lie 192 bytes from its neighbour's).
+template <int kBases>
+__global__ void __launch_bounds__(kProjectionBlock) projection_backward_kernel(const BackwardParams b) {
+    constexpr int kFloats = 3 * kBases;
+    constexpr int kStride = (kBases + 3) | 1;  // odd: conflict-free over the threads
+    __shared__ float s_factor[kProjectionBlock][kStride];
+    const uint32_t g = blockIdx.x * kProjectionBlock + threadIdx.x;
+    if (g < b.n) {
+        float Y[kBases], gc[3];
+        gaussian_gradients<kBases>(b, g, Y, gc);
+#pragma unroll
+        for (int k = 0; k < kBases; ++k) s_factor[threadIdx.x][k] = Y[k];
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) s_factor[threadIdx.x][kBases + ch] = gc[ch];
+    }
+    __syncwarp();
+    const uint32_t warp0 = threadIdx.x & ~31u, lane = threadIdx.x & 31u;
+    const uint32_t first = blockIdx.x * kProjectionBlock + warp0;
+    if (first >= b.n) return;
+    const uint32_t n = min(32u, b.n - first) * kFloats;
+    float* const out = b.d_sh + static_cast<size_t>(first) * kFloats;
+    for (uint32_t i = lane; i < n; i += 32u) {
+        const float* const f = s_factor[warp0 + i / kFloats];
+        const uint32_t r = i % kFloats;
+        out[i] = f[kBases + r % 3u] * f[r / 3u];
+    }
+}
+
 }  // namespace
 
 cudaError_t launch_backward_colors(const BackwardParams& p, cudaStream_t stream) {
     if (p.n == 0) return cudaSuccess;
-    colors_kernel<<<(p.n + kBlock - 1) / kBlock, kBlock, 0, stream>>>(p);
+    const unsigned grid = (p.n + kBlock - 1) / kBlock;
+    switch (p.sh_bases) {
+        case 1: colors_kernel<1><<<grid, kBlock, 0, stream>>>(p); break;
+        case 4: colors_kernel<4><<<grid, kBlock, 0, stream>>>(p); break;
+        case 9: colors_kernel<9><<<grid, kBlock, 0, stream>>>(p); break;
+        default: colors_kernel<16><<<grid, kBlock, 0, stream>>>(p); break;
+    }
     return cudaGetLastError();
 }
 
@@ -931,6 +1061,7 @@ cudaError_t launch_backward_fragments_samples(const BackwardParams& p, cudaStrea
     if (p.n == 0) return cudaSuccess;
     const unsigned grid = (p.n + kBlock - 1) / kBlock;
     const unsigned queue_grid = static_cast<unsigned>(max(p.num_sms, 1)) * kQueueBlocksPerSM;
+    tile_far_kernel<<<(p.tiles_x * p.tiles_y + kWarpsPerBlock - 1) / kWarpsPerBlock, kBlock, 0, stream>>>(p);
     fragments_samples_kernel<false><<<grid, kBlock, 0, stream>>>(p, nullptr);
     fragments_samples_queue_kernel<false><<<queue_grid, kBlock, 0, stream>>>(p, nullptr);
     return cudaGetLastError();
@@ -942,6 +1073,7 @@ cudaError_t launch_backward_fragments_samples_gps(const BackwardParams& p, float
     const unsigned grid = (p.n + kBlock - 1) / kBlock;
     const unsigned queue_grid = static_cast<unsigned>(max(p.num_sms, 1)) * kQueueBlocksPerSM;
     gps_count_law_kernel<<<kLawRows, 32, 0, stream>>>(law);
+    tile_far_kernel<<<(p.tiles_x * p.tiles_y + kWarpsPerBlock - 1) / kWarpsPerBlock, kBlock, 0, stream>>>(p);
     fragments_samples_kernel<true><<<grid, kBlock, 0, stream>>>(p, law);
     fragments_samples_queue_kernel<true><<<queue_grid, kBlock, 0, stream>>>(p, law);
     return cudaGetLastError();
@@ -956,7 +1088,13 @@ cudaError_t launch_gps_count_law(float2* law, cudaStream_t stream) {
 
 cudaError_t launch_backward_projection(const BackwardParams& p, cudaStream_t stream) {
     if (p.n == 0) return cudaSuccess;
-    projection_backward_kernel<<<(p.n + kBlock - 1) / kBlock, kBlock, 0, stream>>>(p);
+    const unsigned grid = (p.n + kProjectionBlock - 1) / kProjectionBlock;
+    switch (p.sh_bases) {
+        case 1: projection_backward_kernel<1><<<grid, kProjectionBlock, 0, stream>>>(p); break;
+        case 4: projection_backward_kernel<4><<<grid, kProjectionBlock, 0, stream>>>(p); break;
+        case 9: projection_backward_kernel<9><<<grid, kProjectionBlock, 0, stream>>>(p); break;
+        default: projection_backward_kernel<16><<<grid, kProjectionBlock, 0, stream>>>(p); break;
+    }
     return cudaGetLastError();
 }
 

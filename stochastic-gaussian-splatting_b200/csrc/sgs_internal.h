@@ -223,6 +223,7 @@ struct BackwardParams {
     const float* cam_position;
     uint32_t n;
     uint32_t sh_bases;
+    bool sh_vec4;                            // degree-3 SH at a 16-byte aligned base
     PassCamera cam;                          // framebuffer camera
     uint32_t width;                          // image width (pixels)
     uint32_t ss;
@@ -243,7 +244,9 @@ struct BackwardParams {
     // T = grad_scale (g . c_w + g_d z_w), interleaved [pixel][sample]
     unsigned long long* pix_keys;
     float* pix_terms;
-    unsigned long long* pix_max_key;         // per pixel, the largest winner key of the samples
+    uint32_t* pix_far;                       // per pixel, the largest depth bits of the samples' winners
+    uint32_t* tile_far;                      // per 8 x 8 tile, the largest of those
+    uint32_t tiles_x, tiles_y;
     // queue of Gaussians with large footprints, walked in row chunks by a persistent kernel
     WorkQueue* bw_queue;
     void* bw_entries;                        // WalkGaussian per entry (backward_st.cu)
