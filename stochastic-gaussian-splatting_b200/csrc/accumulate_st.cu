@@ -15,9 +15,10 @@
 //    packed FP32x2 instructions (fma/mul/sub .f32x2 of sm_100a, each element rounded like the scalar
 //    instruction), with no per-pixel owner lookup or shared-memory traffic; the warp steps as often
 //    as its longest row needs, and each accepted pixel issues one predicated RED;
-//  * a device-side work queue for the Gaussians with larger AABBs (dense_scene): st_order_kernel
-//    puts a long queue in depth order and a persistent kernel takes its tiles of 8 x 8 pixels front to
-//    back (no cross-warp tail, no host synchronisation). Every tile has an upper bound of
+//  * a device-side work queue for the Gaussians with larger AABBs, which a persistent kernel takes in
+//    parts (no cross-warp tail, no host synchronisation). In sparse scenes a part is a chunk of rows.
+//    In dense ones (dense_scene) st_order_kernel lists the parts in depth order and a part is some
+//    tiles of 8 x 8 pixels. Every tile has an upper bound of
 //    its keys' depths (tile_bound); one lane per tile drops the tiles that lie behind their bound or
 //    off the ellipse, and the warp walks the rest, two pixels per lane, lowering the bounds with the
 //    keys it reads. Keys only decrease during a pass, so a dropped fragment could not have won;
@@ -48,7 +49,8 @@ constexpr uint32_t kQueueBlocksPerSM = 4;
 // framebuffer many times over, kMinPixels elsewhere (dense_scene).
 constexpr uint32_t kMinPixels = 2048;
 constexpr uint32_t kDenseMinPixels = 256;
-constexpr float kSampleMaxPixels = 4096.0f;  // a sampled Gaussian counts for at most this many pixels
+constexpr uint32_t kChunkPixels = 2048;   // pixels per chunk of rows of a queued Gaussian in a sparse scene
+constexpr float kSampleMaxCover = 32.0f;  // a sampled Gaussian counts for at most this many framebuffers
 constexpr uint32_t kOrderBlock = 512;
 constexpr uint32_t kMaxClaim = 16;     // items a consumer warp takes per atomic on the cursor
 constexpr uint32_t kPartQuads = 32;    // quads of four tiles in an item (a part of a queued Gaussian)
@@ -187,16 +189,24 @@ __device__ __forceinline__ void red_min_if(unsigned long long* address, const un
         : "memory");
 }
 
-// Each lane walks the span of its row y (when valid), two pixels per step; the warp takes as many
-// steps as its longest row needs (scatter_utils.cuh:35-46 per pixel).
+// Each lane walks segment `seg` of `1 << log_segs` equal parts of the span of its row y (when
+// valid), two pixels per step; the warp takes as many steps as its longest segment needs
+// (scatter_utils.cuh:35-46 per pixel).
 template <bool kBlue, bool kHybrid, bool kMulti>
 __device__ __forceinline__ void walk_rows(const AccumulateParams& a, const FrameRng& rng, const bool valid,
-                                          const RowGaussian& G, const uint32_t y) {
+                                          const RowGaussian& G, const uint32_t y, const uint32_t seg = 0,
+                                          const uint32_t log_segs = 0) {
     uint32_t xs = 0, len = 0;
     float dy = 0.0f;
     if (valid) {
         dy = __fsub_rn(static_cast<float>(y), G.my);
         row_span(G.x_min, G.w, G.mx, G.span, dy, xs, len);
+        if (log_segs > 0) {
+            const uint32_t part = (len + (1u << log_segs) - 1u) >> log_segs;
+            const uint32_t skip = min(seg * part, len);
+            xs += skip;
+            len = min(len - skip, part);
+        }
     }
     const uint32_t steps = __reduce_max_sync(kFullMask, len);
     if (steps == 0) return;
@@ -279,6 +289,25 @@ __device__ __forceinline__ bool tile_on_ellipse(const RowGaussian& G, const uint
     const float eps = 0.1f + 1.0e-4f * (fabsf(right) + fabsf(left) + fabsf(x0));
     // written so that a non-finite bound keeps the tile
     return !(right + eps < x0) && !(left - eps > x0 + kSide);
+}
+
+// Sparse scenes: rows per chunk of a queued Gaussian of AABB width w (about kChunkPixels pixels, a power
+// of two between 1 and 32; each row is walked in 32 / rows segments, so wide footprints keep every lane
+// walking) and chunks per item (one, but for AABBs of more than kMaxParts chunks).
+__device__ __forceinline__ uint32_t log_chunk_rows(const uint32_t w) {
+    const uint32_t rows = max(1u, min(32u, kChunkPixels / max(w, 1u)));
+    return 31u - __clz(rows);
+}
+struct RowParts {
+    uint32_t log_rows, chunks, per_part, parts;
+};
+__device__ __forceinline__ RowParts row_parts(const uint32_t w, const uint32_t h) {
+    RowParts r;
+    r.log_rows = log_chunk_rows(w);
+    r.chunks = (h + (1u << r.log_rows) - 1u) >> r.log_rows;
+    r.per_part = (r.chunks + kMaxParts - 1u) / kMaxParts;
+    r.parts = (r.chunks + r.per_part - 1u) / r.per_part;
+    return r;
 }
 
 // A lane's two pixels of tile (tx, ty), (lane & 7, lane / 8) and four rows below, and their keys: 0 (which
@@ -464,7 +493,9 @@ __global__ void __launch_bounds__(kBlock, 4) st_scatter_kernel(const AccumulateP
         e = __shfl_sync(kFullMask, e, leader) + __popc(big & lt_mask);
         const bool fits = want && e < a.stq.capacity;
         const uint32_t parts =
-            fits ? part_count(quad_rect(rect.x_min, rect.width, rect.y_min, rect.height)) : 0u;
+            !fits   ? 0u
+            : dense ? part_count(quad_rect(rect.x_min, rect.width, rect.y_min, rect.height))
+                    : row_parts(rect.width, rect.height).parts;
         const uint32_t incl = warp_inclusive_sum(parts, lane);
         uint32_t item = 0;
         if (lane == 31 && incl != 0) item = atomicAdd(&a.queue->st_items, incl);
@@ -612,11 +643,33 @@ __global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) st_queue_kernel(con
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
     const uint32_t upto_mask = kFullMask >> (31u - lane);
-    const uint32_t n_items =
-        dense_scene(a) ? a.queue->st_listed : min(a.queue->st_items, a.stq.list_capacity);
+    const bool dense = dense_scene(a);
+    const uint32_t n_items = dense ? a.queue->st_listed : min(a.queue->st_items, a.stq.list_capacity);
     if (n_items == 0) return;
     const FrameRng rng = frame_rng(a);
     const uint32_t n_warps = kWarpsPerBlock * gridDim.x;
+    if (!dense) {
+        // row chunks as they came, each lane a segment of a row, without a look at the keys
+        uint32_t c = blockIdx.x + wib * gridDim.x;
+        while (c < n_items) {
+            uint32_t next = 0;
+            if (lane == 0) next = atomicAdd(&a.queue->next_chunk, 1u);
+            const uint32_t item = a.stq.list[c];
+            if (item != kNoItem) {
+                const RowGaussian G = *queue_entry(a.stq, item & kItemEntryMask);
+                const RowParts r = row_parts(G.w, G.row_first);
+                const uint32_t chunk = (item >> kItemEntryBits) * r.per_part;
+                const uint32_t end = min(chunk + r.per_part, r.chunks);
+                for (uint32_t k = chunk; k < end; ++k) {
+                    const uint32_t row = (k << r.log_rows) + (lane & ((1u << r.log_rows) - 1u));
+                    walk_rows<kBlue, kHybrid, kMulti>(a, rng, row < G.row_first, G, G.y_min + row, lane >> r.log_rows,
+                                                      5u - r.log_rows);
+                }
+            }
+            c = n_warps + __shfl_sync(kFullMask, next, 0);
+        }
+        return;
+    }
     uint32_t log_split = 0;
     while (log_split < 4u && (n_items << log_split) < 4u * n_warps) ++log_split;
     const uint32_t n_parts = n_items << log_split;
@@ -766,8 +819,9 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
             active) {
             const PixelRect rect = pixel_rect(p.bounds, a.cam);
             pixels = static_cast<float>(rect.width) * static_cast<float>(rect.height);
-            pixels = pixels > static_cast<float>(kDenseMinPixels) ? fminf(pixels, kSampleMaxPixels) * static_cast<float>(step)
-                                                                  : 0.0f;
+            pixels = pixels > static_cast<float>(kDenseMinPixels)
+                         ? fminf(pixels * static_cast<float>(step), kSampleMaxCover * a.cam.width * a.cam.height)
+                         : 0.0f;
         }
         for (uint32_t o = 16; o > 0; o >>= 1) pixels += __shfl_xor_sync(kFullMask, pixels, o);
         if ((threadIdx.x & 31u) == 0) s_sum[threadIdx.x >> 5] = pixels;

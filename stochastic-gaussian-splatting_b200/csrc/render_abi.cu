@@ -33,10 +33,11 @@ constexpr size_t kAlign = 256;
 constexpr uint32_t kDefaultMaxBinned = 1u << 20;     // accumulate_hybrid_gps.cu:22
 constexpr uint32_t kStQueueCapacity = 1u << 18;       // ST queue entries with space of their own
 // Coverage by larger Gaussians (AABB pixels over framebuffer pixels) above which a scene counts as dense
-// (accumulate_st.cu). Either way, in us: the 100k scene at 640x480 (64) 93 sparse, 138 dense; its 400k
-// variant (258) 233, 214; the training scene at 800x800 with 60k (170) 278, 230, with 8 samples 1566, 1131;
-// 40k heavy-tailed at 1279x719 (129) 398, 353; the 6M scene (0 at 640x360) 370, 381.
-constexpr float kDenseCoverage = 128.0f;
+// (accumulate_st.cu). Sparse against dense, in us: the training scene at 800x800 with 60k Gaussians
+// (coverage 255) 197, 223, with 120k (514) 339, 252; the 100k scene at 640x480 (64) 82, 129, with 400k (259)
+// 193, 213, with 800k (484) 312, 287; heavy-tailed at 1279x719 with 20k (277) 257, 292, with 40k (550) 415,
+// 364; the 6M scene at 1280x720 (6) 455, 481.
+constexpr float kDenseCoverage = 420.0f;
 constexpr uint32_t kMinOrdered = 8192;                // Gaussians of a scene that may count as dense
 constexpr uint32_t kMaxSamplesPerCall = 1024;         // sgs_render_samples
 constexpr int kMaxDevices = 64;
@@ -117,7 +118,7 @@ struct FullLayout {
     // further entries (st_b) borrow the samples section, which the accumulate passes leave unused, or
     // lie in a section of their own where it is too small
     size_t tile_bound, histogram, list, st_b;
-    uint32_t st_own, st_capacity;
+    uint32_t st_own, st_capacity, st_items;
 };
 
 FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n_samples = 1) {
@@ -153,13 +154,19 @@ FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n
         F.tile_bound = borrow ? L.samples : off;
         F.histogram = F.tile_bound + bounds;
         F.list = F.tile_bound + fixed;
+        // the list: kItemsPerEntry places for each entry, or half of the borrowed section (two items per
+        // framebuffer pixel, more than a scene that covers it 10,000 times needs); further entries behind it
         F.st_capacity = F.st_own;
-        if (borrow && d.st_wanted > own) {
-            const size_t used = fixed + align_up(own * kListBytes) + kAlign;
-            const size_t more = room > used ? (room - used) / (kStEntryBytes + kListBytes) : 0;
-            F.st_capacity += static_cast<uint32_t>(std::min<size_t>(d.st_wanted - own, more));
+        size_t items = own * kItemsPerEntry;
+        if (borrow) {
+            const size_t left = room - fixed - kAlign;
+            items = std::max(items, std::min<size_t>(left / 2 / sizeof(uint32_t), kMaxItems));
+            const size_t used = align_up(items * sizeof(uint32_t));
+            const size_t more = left > used ? (left - used) / kStEntryBytes : 0;
+            if (d.st_wanted > own) F.st_capacity += static_cast<uint32_t>(std::min<size_t>(d.st_wanted - own, more));
         }
-        F.st_b = F.list + align_up(F.st_capacity * kListBytes);
+        F.st_items = static_cast<uint32_t>(items);
+        F.st_b = F.list + align_up(items * sizeof(uint32_t));
         if (!borrow) off = F.st_b;
         L.total = off;
         return F;
@@ -344,7 +351,7 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
         if (s->hybrid_scheduling && static_cast<uint64_t>(g->n_gaussians) << stq.log_row_split > d.max_binned)
             stq.log_row_split = 0;
         stq.list = reinterpret_cast<uint32_t*>(ws + F.list);
-        stq.list_capacity = kItemsPerEntry * F.st_capacity;
+        stq.list_capacity = F.st_items;
         stq.histogram = reinterpret_cast<uint32_t*>(ws + F.histogram);
         stq.tile_bound = reinterpret_cast<uint32_t*>(ws + F.tile_bound);
         stq.bound_pitch = d.tiles_x;

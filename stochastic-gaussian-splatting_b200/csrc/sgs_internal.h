@@ -47,7 +47,8 @@ constexpr uint32_t kItemEntryMask = (1u << kItemEntryBits) - 1u;
 constexpr uint32_t kMaxParts = 1u << (32u - kItemEntryBits);
 constexpr uint32_t kNoItem = 0xffffffffu;  // an unused list place (the last entry has no such part: kMaxStEntries)
 constexpr uint32_t kMaxStEntries = kItemEntryMask;
-constexpr uint32_t kItemsPerEntry = 4;     // list places per entry
+constexpr uint32_t kItemsPerEntry = 4;     // list places per entry, at least
+constexpr uint32_t kMaxItems = 1u << 23;
 
 struct StQueue {
     void* a;                        // the first entries_a entries, kStEntryBytes each
