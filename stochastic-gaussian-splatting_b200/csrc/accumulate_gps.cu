@@ -29,8 +29,10 @@ constexpr uint32_t kBlock = 256;
 constexpr uint32_t kFullMask = 0xffffffffu;
 constexpr uint32_t kBinningPointThreshold = 512;  // accumulate_hybrid_gps.cu:21
 constexpr uint32_t kChunkPoints = 256;             // accumulate_hybrid_gps.cu:19
-constexpr uint32_t kQueueBlocksPerSM = 8;
+constexpr uint32_t kChunkBlocksPerSM = 8;
+constexpr uint32_t kQueueBlocksPerSM = 4;
 constexpr uint32_t kItemsPerWarp = 128;  // parked cooperative points per warp (multiple of 32)
+constexpr uint32_t kMaxClaim = 8;         // items a consumer warp takes per atomic on the cursor
 constexpr uint32_t kChunksPerClaim = 8;  // chunks a consumer warp takes per atomic on the cursor
 
 struct PointSource {
@@ -216,6 +218,7 @@ __device__ __forceinline__ void gps_scatter(const AccumulateParams& a) {
                 base = __shfl_sync(kFullMask, base, leader);
                 const uint32_t e = static_cast<uint32_t>(base >> kQueueEntryShift) + __popc(ballot & ((1u << lane) - 1u));
                 const unsigned long long first_chunk = (base & kQueueChunkMask) + (incl - chunks);
+                bool queued = false;
                 if (want && e < a.max_binned && e < a.q.capacity) {
                     if (first_chunk + chunks <= kMaxQueueChunks) {
                         a.q.key[e] = s.key;
@@ -225,6 +228,7 @@ __device__ __forceinline__ void gps_scatter(const AccumulateParams& a) {
                                                  __float_as_uint(s.conic.z), static_cast<uint32_t>(first_chunk));
                         a.q.count[e] = count;
                         act = false;
+                        queued = true;
                     } else {
                         // past 32-bit chunk indices (where the reference's own chunk offsets wrap): the
                         // entry is marked unused and the Gaussian scattered. Entries and chunks are
@@ -232,6 +236,10 @@ __device__ __forceinline__ void gps_scatter(const AccumulateParams& a) {
                         a.q.meta[e] = make_uint4(0u, 0u, 0u, kUnusedQueueEntry);
                         a.q.count[e] = 0u;
                     }
+                }
+                if (a.stq.list != nullptr) {
+                    count_at_depth(a.stq.histogram, static_cast<uint32_t>(s.key >> 32),
+                                   queued ? gps_parts(count).parts : 0u, lane);
                 }
             }
         }
@@ -298,10 +306,10 @@ __global__ void __launch_bounds__(kBlock, 5) gps_scatter_hybrid_kernel(const Acc
     gps_scatter<true, false>(a);
 }
 
-// Persistent consumer of the binned Gaussians: each warp steals kChunksPerClaim 256-point chunks at
-// a time (accumulate_hybrid_gps.cu:126-181 with per-point counter-based seeds, so which warp draws
+// Consumer of the binned Gaussians as they came (short queues, and items that do not fit the list): each warp
+// steals kChunksPerClaim 256-point chunks at a time (accumulate_hybrid_gps.cu:126-181 with per-point counter-based seeds, so which warp draws
 // which chunk does not change the winners).
-__global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) gps_queue_kernel(const AccumulateParams a) {
+__device__ __forceinline__ void consume_chunks(const AccumulateParams& a) {
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned long long packed = a.queue->packed;
     const uint32_t cap = min(a.max_binned, a.q.capacity);
@@ -355,6 +363,152 @@ __global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) gps_queue_kernel(co
     }
 }
 
+__global__ void __launch_bounds__(kBlock, kChunkBlocksPerSM) gps_chunks_kernel(const AccumulateParams a) {
+    consume_chunks(a);
+}
+
+// An item of the warp's claim, staged in shared memory.
+struct GpsItem {
+    float4 geom, geom2;  // as in the queue arrays
+    uint4 meta;
+    unsigned long long key;
+    uint32_t first, end;  // points of the item
+};
+
+// Whether every pixel the Gaussian can reach is nearer than it. Its points register only in pixels whose
+// centres pass the power test, which lie within the ellipse's extents of the mean; where the ellipse is
+// so thin that rounding decides that test (1 / (1 - rho^2) above 1000), the radius of the draw itself,
+// at most sqrt(-2 ln 1e-37) = 13.06, bounds them. Blocks of tiles whose bound does not decide it take
+// their tiles' largest bound, and tiles whose bound does not, the largest depth of their keys.
+__device__ __forceinline__ bool occluded(const AccumulateParams& a, const GpsItem& G, const uint32_t lane) {
+    const float var_x = G.geom.z * G.geom.z, var_y = G.geom.w * G.geom.w + G.geom2.x * G.geom2.x;
+    const float radius =
+        __uint_as_float(G.meta.x) * var_x <= 1000.0f ? 1.01f * sqrtf(2.0f * fmaxf(G.geom2.y, 0.0f)) : 13.2f;
+    const float ex = 1.0f + radius * sqrtf(var_x), ey = 1.0f + radius * sqrtf(var_y);
+    const float x_lo = fmaxf(G.geom.x - ex, 0.0f), x_hi = fminf(G.geom.x + ex, a.cam.width - 1.0f);
+    const float y_lo = fmaxf(G.geom.y - ey, 0.0f), y_hi = fminf(G.geom.y + ey, a.cam.height - 1.0f);
+    if (!(x_lo <= x_hi && y_lo <= y_hi)) return false;  // (also for a non-finite extent)
+    const uint32_t tx0 = static_cast<uint32_t>(x_lo) / kBoundTile, tx1 = static_cast<uint32_t>(x_hi) / kBoundTile;
+    const uint32_t ty0 = static_cast<uint32_t>(y_lo) / kBoundTile, ty1 = static_cast<uint32_t>(y_hi) / kBoundTile;
+    const uint32_t bx0 = tx0 / kBlockTiles, by0 = ty0 / kBlockTiles, bw = tx1 / kBlockTiles - bx0 + 1u;
+    const uint32_t n = bw * (ty1 / kBlockTiles - by0 + 1u);
+    const uint32_t depth = static_cast<uint32_t>(G.key >> 32);
+    // one block of 8 x 8 tiles per lane
+    for (uint32_t base = 0; base < n; base += 32u) {
+        const uint32_t row = (base + lane) / bw;
+        const uint32_t bx = bx0 + (base + lane - row * bw), by = by0 + row;
+        const bool open = base + lane < n && __ldcg(a.stq.block_bound + by * a.stq.blocks_x + bx) >= depth;
+        for (uint32_t todo = __ballot_sync(kFullMask, open); todo != 0; todo &= todo - 1) {
+            // an open block: its tiles, two per lane
+            const uint32_t src = __ffs(todo) - 1;
+            const uint32_t ox = __shfl_sync(kFullMask, bx, src), oy = __shfl_sync(kFullMask, by, src);
+            const uint32_t tx = ox * kBlockTiles + (lane & 7u), ty = oy * kBlockTiles + (lane >> 3);
+            const uint32_t* const t = a.stq.tile_bound + static_cast<size_t>(ty) * a.stq.bound_pitch + tx;
+            const bool column = tx * kBoundTile < a.cam.width_int;
+            const uint32_t far0 = column && ty < a.stq.tiles_y ? __ldcg(t) : 0u;
+            const uint32_t far1 = column && ty + 4u < a.stq.tiles_y ? __ldcg(t + 4u * a.stq.bound_pitch) : 0u;
+            const uint32_t block = __reduce_max_sync(kFullMask, max(far0, far1));
+            if (lane == 0 && block != 0xffffffffu) atomicMin(a.stq.block_bound + oy * a.stq.blocks_x + ox, block);
+            const bool in = tx >= tx0 && tx <= tx1;
+            uint32_t upper = __ballot_sync(kFullMask, in && far0 >= depth && ty >= ty0 && ty <= ty1);
+            uint32_t lower = __ballot_sync(kFullMask, in && far1 >= depth && ty + 4u >= ty0 && ty + 4u <= ty1);
+            while ((upper | lower) != 0) {
+                // an open tile: its keys, two per lane
+                const uint32_t i = upper != 0 ? __ffs(upper) - 1 : __ffs(lower) + 31u;
+                if (upper != 0) upper &= upper - 1;
+                else lower &= lower - 1;
+                const uint32_t px = ox * kBlockTiles + (i & 7u), py = oy * kBlockTiles + (i >> 3);
+                const uint32_t x = px * kBoundTile + (lane & 7u), y = py * kBoundTile + (lane >> 3);
+                const unsigned long long* const p = a.framebuffer + (static_cast<size_t>(y) * a.cam.width_int + x);
+                uint32_t far = 0;
+                if (x < a.cam.width_int && y < a.stq.height) far = static_cast<uint32_t>(__ldcg(p) >> 32);
+                if (x < a.cam.width_int && y + 4u < a.stq.height)
+                    far = max(far, static_cast<uint32_t>(__ldcg(p + 4u * static_cast<size_t>(a.cam.width_int)) >> 32));
+                far = __reduce_max_sync(kFullMask, far);
+                if (lane == 0 && far != 0xffffffffu)
+                    atomicMin(a.stq.tile_bound + static_cast<size_t>(py) * a.stq.bound_pitch + px, far);
+                if (far >= depth) return false;
+            }
+        }
+    }
+    return true;
+}
+
+// Persistent consumer of the binned Gaussians, front to back (accumulate_hybrid_gps.cu:126-181 with
+// per-point counter-based seeds, so neither the order nor the warp that draws a point changes the
+// winners): a warp takes some items at a time and skips those whose Gaussian lies behind every pixel it can
+// reach, for keys only decrease during a pass.
+__global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) gps_queue_kernel(const AccumulateParams a) {
+    __shared__ GpsItem s_item[kBlock / 32][kMaxClaim];
+    if (a.queue->st_listed == kNotListed) {
+        consume_chunks(a);
+        return;
+    }
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t n_items = a.queue->st_listed;
+    const uint32_t frame = frame_rng(a).frame;
+    const uint32_t n_warps = gridDim.x * (kBlock / 32u);
+    uint32_t c0 = blockIdx.x + warp * gridDim.x, claim = 1;
+    while (c0 < n_items) {
+        // claims grow with the depth taken, as most of what lies there is skipped
+        const uint32_t next_claim = min(1u + c0 / n_warps, kMaxClaim);
+        uint32_t next = 0;
+        if (lane == 0) next = atomicAdd(&a.queue->next_chunk, next_claim);
+        const uint32_t n = min(claim, n_items - c0);
+        __syncwarp();
+        if (lane < n) {
+            const uint32_t item = a.stq.list[c0 + lane];
+            const uint32_t e = item & kItemEntryMask;
+            const uint32_t count = a.q.count[e];
+            GpsItem G;
+            G.geom = a.q.geom[e];
+            G.geom2 = a.q.geom2[e];
+            G.meta = a.q.meta[e];
+            G.key = a.q.key[e];
+            const uint32_t points = gps_parts(count).points;
+            G.first = (item >> kItemEntryBits) * points;
+            G.end = min(G.first + points, count);
+            s_item[warp][lane] = G;
+        }
+        __syncwarp();
+        for (uint32_t i = 0; i < n; ++i) {
+            const GpsItem& G = s_item[warp][i];
+            if (occluded(a, G, lane)) continue;
+            PointSource s;
+            s.key = G.key;
+            s.mean2d = make_float2(G.geom.x, G.geom.y);
+            s.L = make_float3(G.geom.z, G.geom.w, G.geom2.x);
+            s.power_threshold = G.geom2.y;
+            s.opacity_rcp = G.geom2.z;
+            s.opacity_dilog = G.geom2.w;
+            s.conic = make_float3(__uint_as_float(G.meta.x), __uint_as_float(G.meta.y), __uint_as_float(G.meta.z));
+            const uint2 base_seed = gps_seed(static_cast<uint32_t>(s.key), frame);
+            // a group's pixels first, then their keys, read together, then the atomics the keys leave
+            for (uint32_t point = G.first + lane; point < G.end; point += 32u * kFilterGroup) {
+                unsigned long long* pixel[kFilterGroup];
+                unsigned long long current[kFilterGroup];
+#pragma unroll
+                for (uint32_t k = 0; k < kFilterGroup; ++k) {
+                    uint2 seed = base_seed;
+                    seed.x ^= (point + 32u * k) * 0x9E3779B9u;
+                    pixel[k] = point + 32u * k < G.end ? gps_point_pixel(a, a.framebuffer, pcg2d_uniform(seed), s) : nullptr;
+                }
+#pragma unroll
+                for (uint32_t k = 0; k < kFilterGroup; ++k) {
+                    current[k] = 0ull;
+                    if (pixel[k] != nullptr)
+                        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(current[k]) : "l"(pixel[k]));
+                }
+#pragma unroll
+                for (uint32_t k = 0; k < kFilterGroup; ++k)
+                    if (pixel[k] != nullptr && current[k] > s.key) atomicMin(pixel[k], s.key);
+            }
+        }
+        c0 = n_warps + __shfl_sync(kFullMask, next, 0);
+        claim = next_claim;
+    }
+}
+
 }  // namespace
 
 cudaError_t launch_accumulate_gps(const AccumulateParams& p, const int num_sms, cudaStream_t stream) {
@@ -363,7 +517,13 @@ cudaError_t launch_accumulate_gps(const AccumulateParams& p, const int num_sms, 
     if (p.hybrid) gps_scatter_hybrid_kernel<<<grid, kBlock, 0, stream>>>(p);
     else if (p.n_samples > 1) gps_scatter_kernel<true><<<grid, kBlock, 0, stream>>>(p);
     else gps_scatter_kernel<false><<<grid, kBlock, 0, stream>>>(p);
-    if (p.hybrid) gps_queue_kernel<<<static_cast<unsigned>(num_sms) * kQueueBlocksPerSM, kBlock, 0, stream>>>(p);
+    if (p.hybrid && p.stq.list != nullptr) {
+        const cudaError_t err = launch_order_gps(p, num_sms, stream);
+        if (err != cudaSuccess) return err;
+        gps_queue_kernel<<<static_cast<unsigned>(num_sms) * kQueueBlocksPerSM, kBlock, 0, stream>>>(p);
+    } else if (p.hybrid) {
+        gps_chunks_kernel<<<static_cast<unsigned>(num_sms) * kChunkBlocksPerSM, kBlock, 0, stream>>>(p);
+    }
     return cudaGetLastError();
 }
 

@@ -17,7 +17,7 @@
 //    as its longest row needs, and each accepted pixel issues one predicated RED;
 //  * a device-side work queue for the Gaussians with larger AABBs, which a persistent kernel takes in
 //    parts (no cross-warp tail, no host synchronisation). In sparse scenes a part is a chunk of rows.
-//    In dense ones (dense_scene) st_order_kernel lists the parts in depth order and a part is some
+//    In dense ones (dense_scene) order_kernel lists the parts in depth order and a part is some
 //    tiles of 8 x 8 pixels. Every tile has an upper bound of
 //    its keys' depths (tile_bound); one lane per tile drops the tiles that lie behind their bound or
 //    off the ellipse, and the warp walks the rest, two pixels per lane, lowering the bounds with the
@@ -509,8 +509,8 @@ __global__ void __launch_bounds__(kBlock, 4) st_scatter_kernel(const AccumulateP
         if (!dense) {
             for (uint32_t i = 0; i < parts && item + i < a.stq.list_capacity; ++i)
                 a.stq.list[item + i] = listed ? i << kItemEntryBits | e : kNoItem;
-        } else if (listed) {
-            atomicAdd(a.stq.histogram + depth_bucket(G.key_hi), parts);
+        } else {
+            count_at_depth(a.stq.histogram, G.key_hi, listed ? parts : 0u, lane);
         }
         keep_big = want && !listed;
         if (keep_big) atomicAdd(&a.queue->overflow, 1u);
@@ -576,12 +576,16 @@ __global__ void __launch_bounds__(kBlock, 4) st_scatter_kernel(const AccumulateP
 // Lists the queue's items in depth order (buckets of 1/32 octave). Every block sums the producers'
 // histogram itself, counts its own slice of the entries per bucket in shared memory, takes each
 // bucket's share with one atomic and places its items there.
-__global__ void __launch_bounds__(kOrderBlock) st_order_kernel(const AccumulateParams a) {
+// kGps: the entries of GPS hybrid scheduling (accumulate_gps.cu), when the list has room for all of them.
+template <bool kGps>
+__global__ void __launch_bounds__(kOrderBlock) order_kernel(const AccumulateParams a) {
     constexpr uint32_t kPerThread = kDepthBuckets / kOrderBlock;
     __shared__ uint32_t s_first[kDepthBuckets], s_count[kDepthBuckets];
     __shared__ uint32_t s_warp[kOrderBlock / 32];
-    if (!dense_scene(a)) return;  // the producers have listed the items as they came
-    const uint32_t n = min(a.queue->st_entries, a.stq.capacity);
+    if (!kGps && !dense_scene(a)) return;  // the producers have listed the items as they came
+    const uint32_t n = kGps ? static_cast<uint32_t>(min(a.queue->packed >> kQueueEntryShift,
+                                                        static_cast<unsigned long long>(min(a.max_binned, a.q.capacity))))
+                            : min(a.queue->st_entries, a.stq.capacity);
     const uint32_t per_block = max(kOrderBlock, (n + gridDim.x - 1u) / gridDim.x);
     const uint32_t begin = min(blockIdx.x * per_block, n), end = min(begin + per_block, n);
     if (begin >= end) return;
@@ -603,8 +607,17 @@ __global__ void __launch_bounds__(kOrderBlock) st_order_kernel(const AccumulateP
         s_first[threadIdx.x * kPerThread + i] = first;
         first += v[i];
     }
-    if (blockIdx.x == 0 && threadIdx.x == kOrderBlock - 1u) a.queue->st_listed = first;
+    __shared__ uint32_t s_total;
+    if (threadIdx.x == kOrderBlock - 1u) s_total = first;
+    __syncthreads();
+    const bool fits = s_total <= a.stq.list_capacity;  // ST: always
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.queue->st_listed = fits ? s_total : kNotListed;
+    if (!fits) return;
     auto parts_of = [&](const uint32_t e, uint32_t& bucket) {
+        if (kGps) {
+            bucket = depth_bucket(static_cast<uint32_t>(a.q.key[e] >> 32));
+            return gps_parts(a.q.count[e]).parts;
+        }
         const RowGaussian* const G = queue_entry(a.stq, e);
         const uint32_t h = G->row_first;
         bucket = depth_bucket(G->key_hi);
@@ -798,9 +811,19 @@ __device__ __forceinline__ void clear_keys(unsigned long long* __restrict__ fb, 
     }
 }
 
-__global__ void clear_kernel(unsigned long long* __restrict__ fb, const size_t n_fb, WorkQueue* __restrict__ queue) {
-    clear_keys(fb, n_fb, queue, static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x,
-               static_cast<size_t>(gridDim.x) * blockDim.x);
+__device__ __forceinline__ void clear_bounds(const StQueue& q, const size_t tid, const size_t stride) {
+    for (size_t i = tid; i < static_cast<size_t>(q.bound_pitch) * q.tiles_y + q.n_blocks; i += stride)
+        q.tile_bound[i] = 0xffffffffu;
+    for (size_t i = tid; i < 2u * kDepthBuckets; i += stride) q.histogram[i] = 0u;
+}
+
+// q.tile_bound null: no tile bounds and no depth histogram.
+__global__ void clear_kernel(unsigned long long* __restrict__ fb, const size_t n_fb, WorkQueue* __restrict__ queue,
+                             const StQueue q) {
+    const size_t tid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+    clear_keys(fb, n_fb, queue, tid, stride);
+    if (q.tile_bound != nullptr) clear_bounds(q, tid, stride);
 }
 
 // The clear of a stochastic-transparency pass: also the tile bounds and the depth histogram, and, in
@@ -835,16 +858,15 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
     const size_t stride = static_cast<size_t>(gridDim.x - kSampleBlocks) * kBlock;
     const size_t tid = static_cast<size_t>(blockIdx.x - kSampleBlocks) * kBlock + threadIdx.x;
     clear_keys(a.framebuffer, n_fb, a.queue, tid, stride);
-    for (size_t i = tid; i < static_cast<size_t>(a.stq.bound_pitch) * a.stq.tiles_y; i += stride)
-        a.stq.tile_bound[i] = 0xffffffffu;
-    for (size_t i = tid; i < 2u * kDepthBuckets; i += stride) a.stq.histogram[i] = 0u;
+    clear_bounds(a.stq, tid, stride);
 }
 
 template <bool kBlue, bool kHybrid, bool kMulti>
 void launch_st(const AccumulateParams& p, const unsigned grid, const int num_sms, cudaStream_t stream) {
     if (p.stq.log_row_split != 0) st_scatter_kernel<kBlue, kHybrid, kMulti, true><<<grid, kBlock, 0, stream>>>(p);
     else st_scatter_kernel<kBlue, kHybrid, kMulti, false><<<grid, kBlock, 0, stream>>>(p);
-    if (!isinf(p.stq.dense_pixels)) st_order_kernel<<<static_cast<unsigned>(num_sms), kOrderBlock, 0, stream>>>(p);
+    if (!isinf(p.stq.dense_pixels))
+        order_kernel<false><<<static_cast<unsigned>(num_sms), kOrderBlock, 0, stream>>>(p);
     st_queue_kernel<kBlue, kHybrid, kMulti>
         <<<static_cast<unsigned>(num_sms) * kQueueBlocksPerSM, kBlock, 0, stream>>>(p);
 }
@@ -868,9 +890,15 @@ unsigned clear_blocks(const size_t n_fb, const int num_sms) {
 }
 }  // namespace
 
-cudaError_t launch_clear(unsigned long long* framebuffer, const size_t n_fb, WorkQueue* queue, const int num_sms,
-                         cudaStream_t stream) {
-    clear_kernel<<<clear_blocks(n_fb, num_sms), kBlock, 0, stream>>>(framebuffer, n_fb, queue);
+cudaError_t launch_clear(unsigned long long* framebuffer, const size_t n_fb, WorkQueue* queue, const StQueue& stq,
+                         const int num_sms, cudaStream_t stream) {
+    const size_t n = n_fb + static_cast<size_t>(stq.bound_pitch) * stq.tiles_y / 2;
+    clear_kernel<<<clear_blocks(n, num_sms), kBlock, 0, stream>>>(framebuffer, n_fb, queue, stq);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_order_gps(const AccumulateParams& p, const int num_sms, cudaStream_t stream) {
+    order_kernel<true><<<static_cast<unsigned>(num_sms), kOrderBlock, 0, stream>>>(p);
     return cudaGetLastError();
 }
 

@@ -38,7 +38,7 @@ constexpr uint32_t kStQueueCapacity = 1u << 18;       // ST queue entries with s
 // 193, 213, with 800k (484) 312, 287; heavy-tailed at 1279x719 with 20k (277) 257, 292, with 40k (550) 415,
 // 364; the 6M scene at 1280x720 (6) 455, 481.
 constexpr float kDenseCoverage = 420.0f;
-constexpr uint32_t kMinOrdered = 8192;                // Gaussians of a scene that may count as dense
+constexpr uint32_t kMinOrdered = 8192;                // Gaussians of a scene whose queue may be ordered
 constexpr uint32_t kMaxSamplesPerCall = 1024;         // sgs_render_samples
 constexpr int kMaxDevices = 64;
 std::atomic<int> g_sm_count[kMaxDevices];
@@ -85,7 +85,10 @@ int derive(const sgs_gaussians* g, const sgs_camera* c, const sgs_settings* s, D
     d.queue_capacity = 0;
     d.max_binned = 0;
     d.st_queue = false;
-    d.st_wanted = d.tiles_x = d.tiles_y = 0;
+    d.st_wanted = 0;
+    // tiles per row padded to whole quads
+    d.tiles_x = static_cast<uint32_t>((fbw + 4 * kBoundTile - 1) / (4 * kBoundTile)) * 4;
+    d.tiles_y = static_cast<uint32_t>((fbh + kBoundTile - 1) / kBoundTile);
     if (g->n_gaussians > 0) {
         if (s->use_gps) {
             if (s->hybrid_scheduling) {
@@ -101,14 +104,16 @@ int derive(const sgs_gaussians* g, const sgs_camera* c, const sgs_settings* s, D
             if (s->hybrid_scheduling)
                 d.max_binned = std::min(s->max_binned != 0 ? s->max_binned : kDefaultMaxBinned, g->n_gaussians);
             d.st_queue = true;
-            d.tiles_x = static_cast<uint32_t>((fbw + 4 * kBoundTile - 1) / (4 * kBoundTile)) * 4;
-            d.tiles_y = static_cast<uint32_t>((fbh + kBoundTile - 1) / kBoundTile);
             d.st_wanted = std::min(g->n_gaussians, kMaxStEntries);
             const uint32_t cap = g_queue_limit.load(std::memory_order_relaxed);
             if (cap != 0) d.st_wanted = std::min(d.st_wanted, cap);
         }
     }
     return SGS_OK;
+}
+
+size_t bound_blocks(const Derived& d) {
+    return static_cast<size_t>((d.tiles_x + kBlockTiles - 1) / kBlockTiles) * ((d.tiles_y + kBlockTiles - 1) / kBlockTiles);
 }
 
 struct FullLayout {
@@ -137,7 +142,7 @@ FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n
     if (d.st_queue) {
         // 60 bytes for each of min(N, 2^18) entries in any case; more where the workspace stays within the
         // scratch of the allocation-free render (several samples per call never run there)
-        const size_t bounds = align_up(static_cast<size_t>(d.tiles_x) * d.tiles_y * sizeof(uint32_t));
+        const size_t bounds = align_up((static_cast<size_t>(d.tiles_x) * d.tiles_y + bound_blocks(d)) * sizeof(uint32_t));
         const size_t fixed = bounds + align_up(2 * kDepthBuckets * sizeof(uint32_t));
         constexpr size_t kListBytes = kItemsPerEntry * sizeof(uint32_t);
         const size_t room = d.n_fb * sizeof(float4);
@@ -170,6 +175,19 @@ FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n
         if (!borrow) off = F.st_b;
         L.total = off;
         return F;
+    }
+    // hybrid GPS: tile bounds, depth histogram and item list borrow the samples section; a short queue, or
+    // one whose items turn out not to fit the list, is taken as it came
+    if (d.queue_capacity >= kMinOrdered && d.queue_capacity <= kItemEntryMask + 1u) {
+        const size_t bounds = align_up((static_cast<size_t>(d.tiles_x) * d.tiles_y + bound_blocks(d)) * sizeof(uint32_t));
+        const size_t fixed = bounds + align_up(2 * kDepthBuckets * sizeof(uint32_t));
+        const size_t room = d.n_fb * sizeof(float4);
+        if (fixed + kMinOrdered * sizeof(uint32_t) <= room) {
+            F.tile_bound = L.samples;
+            F.histogram = L.samples + bounds;
+            F.list = L.samples + fixed;
+            F.st_items = static_cast<uint32_t>(std::min<size_t>((room - fixed) / sizeof(uint32_t), kMaxItems));
+        }
     }
     const size_t q = d.queue_capacity;
     off = align_up(off + q * sizeof(unsigned long long));
@@ -335,6 +353,18 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
     w.q.count = reinterpret_cast<uint32_t*>(ws + F.q_count);
     w.q.capacity = d.queue_capacity;
     StQueue stq{};
+    if (F.st_items != 0) {
+        stq.list = reinterpret_cast<uint32_t*>(ws + F.list);
+        stq.list_capacity = F.st_items;
+        stq.histogram = reinterpret_cast<uint32_t*>(ws + F.histogram);
+        stq.tile_bound = reinterpret_cast<uint32_t*>(ws + F.tile_bound);
+        stq.block_bound = stq.tile_bound + static_cast<size_t>(d.tiles_x) * d.tiles_y;
+        stq.blocks_x = (d.tiles_x + kBlockTiles - 1) / kBlockTiles;
+        stq.n_blocks = static_cast<uint32_t>(bound_blocks(d));
+        stq.bound_pitch = d.tiles_x;
+        stq.tiles_y = d.tiles_y;
+        stq.height = c->height * d.ss;
+    }
     if (d.st_queue) {
         stq.a = ws + F.q_key;
         stq.b = ws + F.st_b;
@@ -350,13 +380,6 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
         stq.log_row_split = g->n_gaussians < (1u << 16) ? 3u : g->n_gaussians < (1u << 18) ? 2u : 0u;
         if (s->hybrid_scheduling && static_cast<uint64_t>(g->n_gaussians) << stq.log_row_split > d.max_binned)
             stq.log_row_split = 0;
-        stq.list = reinterpret_cast<uint32_t*>(ws + F.list);
-        stq.list_capacity = F.st_items;
-        stq.histogram = reinterpret_cast<uint32_t*>(ws + F.histogram);
-        stq.tile_bound = reinterpret_cast<uint32_t*>(ws + F.tile_bound);
-        stq.bound_pitch = d.tiles_x;
-        stq.tiles_y = d.tiles_y;
-        stq.height = c->height * d.ss;
     }
 
     const PassCamera cam = pass_camera(c, s, d.ss);
@@ -431,7 +454,7 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
     // the clear and accumulate passes of one framebuffer (or, with p.n_samples > 1, of all of them)
     auto accumulate = [&](const AccumulateParams& p, const size_t n_clear) -> int {
         cudaError_t err = d.st_queue ? launch_clear_st(p, n_clear, sms, acc_stream)
-                                    : launch_clear(p.framebuffer, n_clear, w.queue, sms, acc_stream);
+                                    : launch_clear(p.framebuffer, n_clear, w.queue, p.stq, sms, acc_stream);
         if (err != cudaSuccess) return fail(SGS_ERROR_CUDA, "clear: %s", cudaGetErrorString(err));
         if (g->n_gaussians == 0) return SGS_OK;
         if (t_stage_start != nullptr) cudaEventRecord(t_stage_start, acc_stream);
@@ -474,7 +497,7 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
         // Several GPS samples with hybrid scheduling: each frame's points are drawn by its own scatter
         // and queue passes into its own framebuffer (the work queue is reused in stream order), then one
         // resolve pass merges the n framebuffers in frame order.
-        cudaError_t err = launch_clear(w.framebuffer, d.n_fb * n_samples, w.queue, sms, acc_stream);
+        cudaError_t err = launch_clear(w.framebuffer, d.n_fb * n_samples, w.queue, stq, sms, acc_stream);
         if (err != cudaSuccess) return fail(SGS_ERROR_CUDA, "clear: %s", cudaGetErrorString(err));
         if (t_stage_start != nullptr) cudaEventRecord(t_stage_start, acc_stream);
         for (uint32_t sm = 0; sm < n_samples && g->n_gaussians > 0; ++sm) {
@@ -483,7 +506,7 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
             pa.framebuffer = w.framebuffer + static_cast<size_t>(sm) * d.n_fb;
             pa.frame_offset = sm;
             if (sm > 0) {
-                err = launch_clear(pa.framebuffer, 0, w.queue, sms, acc_stream);  // the queue header only
+                err = launch_clear(pa.framebuffer, 0, w.queue, stq, sms, acc_stream);  // the queue only
                 if (err != cudaSuccess) return fail(SGS_ERROR_CUDA, "clear: %s", cudaGetErrorString(err));
             }
             err = launch_accumulate_gps(pa, sms, acc_stream);

@@ -19,7 +19,7 @@ struct WorkQueue {
     unsigned int binned;         // hybrid ST: Gaussians the reference would gather, in arrival order
     unsigned int st_entries;     // ST: entries and list items reserved by producers
     unsigned int st_items;
-    unsigned int st_listed;      // ST: items the order pass has listed
+    unsigned int st_listed;      // items the order pass has listed (GPS: or kNotListed)
     alignas(16) float covered[4];  // ST: AABB pixels of the scene, estimated by kSampleBlocks blocks of the clear pass
 };
 static_assert(offsetof(WorkQueue, covered) % 16 == 0, "read as one float4");
@@ -36,9 +36,10 @@ constexpr uint32_t kUnusedQueueEntry = 0xffffffffu;
 // more than its 2^18 entries only while a one-sample workspace stays within it.
 constexpr size_t kNoAllocScratchBytes = size_t(64) << 20;
 
-// ---- stochastic-transparency queue: entries in depth order, depth bounds per tile ----
+// ---- queues in depth order, depth bounds per tile (stochastic transparency; binned GPS Gaussians) ----
 constexpr uint32_t kStEntryBytes = 64;
 constexpr uint32_t kBoundTile = 8;        // pixels per side of a tile with a depth bound
+constexpr uint32_t kBlockTiles = 8;       // tiles per side of a block with a depth bound
 constexpr uint32_t kDepthBuckets = 1024;  // 1/32 octave each over view depths of 2^-16 .. 2^16
 constexpr uint32_t kSampleBlocks = 4;
 // A list item is a part (32 quads of tiles, at most kMaxParts parts) of an entry: part << kItemEntryBits | entry.
@@ -61,6 +62,8 @@ struct StQueue {
     uint32_t list_capacity;
     uint32_t* histogram;            // items per depth bucket, then the order pass's cursors
     uint32_t* tile_bound;           // per tile, an upper bound of its keys' depth bits; null: not kept
+    uint32_t* block_bound;          // the same per block of 8 x 8 tiles, behind the tiles' bounds (GPS; ST leaves it)
+    uint32_t blocks_x, n_blocks;
     uint32_t bound_pitch, tiles_y;  // tiles per row (a multiple of 4) and rows
     uint32_t height;                // framebuffer rows
 };
@@ -70,6 +73,32 @@ struct StQueue {
 __device__ __forceinline__ uint32_t depth_bucket(const uint32_t depth_bits) {
     const int b = static_cast<int>(depth_bits >> 18) - ((127 - 16) << 5);
     return static_cast<uint32_t>(min(max(b, 0), static_cast<int>(kDepthBuckets) - 1));
+}
+
+// Adds `items` (0: none) to the histogram at the depth of `key_hi`, one atomic per bucket of the warp
+// (neighbours in Morton order mostly share theirs; a dense scene's Gaussians have some 60 in all).
+__device__ __forceinline__ void count_at_depth(uint32_t* __restrict__ histogram, const uint32_t key_hi,
+                                               const uint32_t items, const uint32_t lane) {
+    const uint32_t bucket = items != 0 ? depth_bucket(key_hi) : 0xffffffffu;
+    const uint32_t peers = __match_any_sync(0xffffffffu, bucket);
+    const uint32_t sum = __reduce_add_sync(peers, items);
+    if (sum != 0 && lane == __ffs(peers) - 1u) atomicAdd(histogram + bucket, sum);
+}
+
+// Items of a binned GPS Gaussian of `count` points: kGpsItemPoints points each (more where it would have
+// more than kMaxGpsParts items, so that the items of 2^20 entries stay below 2^31); an unused entry has none.
+constexpr uint32_t kGpsItemPoints = 2048;
+constexpr uint32_t kMaxGpsParts = 1024;
+constexpr uint32_t kNotListed = 0xffffffffu;  // WorkQueue::st_listed: the items do not fit the list
+struct GpsParts {
+    uint32_t parts, points;
+};
+__device__ __forceinline__ GpsParts gps_parts(const uint32_t count) {
+    GpsParts p;
+    const uint32_t items = (count + kGpsItemPoints - 1u) / kGpsItemPoints;
+    p.points = (items + kMaxGpsParts - 1u) / kMaxGpsParts * kGpsItemPoints;
+    p.parts = count != 0 ? (count + p.points - 1u) / p.points : 0u;
+    return p;
 }
 
 // Per-entry arrays of the GPS large-Gaussian queue (structure of arrays, 16-byte aligned).
@@ -159,8 +188,9 @@ __device__ __forceinline__ FrameRng frame_rng(const AccumulateParams& a) {
     return frame_rng_at(a, (a.frame_ptr != nullptr ? *a.frame_ptr : a.frame_idx) + a.frame_offset);
 }
 
-cudaError_t launch_clear(unsigned long long* framebuffer, size_t n_fb, WorkQueue* queue, int num_sms,
-                         cudaStream_t stream);
+cudaError_t launch_clear(unsigned long long* framebuffer, size_t n_fb, WorkQueue* queue, const StQueue& stq,
+                         int num_sms, cudaStream_t stream);
+cudaError_t launch_order_gps(const AccumulateParams& p, int num_sms, cudaStream_t stream);
 cudaError_t launch_clear_st(const AccumulateParams& p, size_t n_fb, int num_sms, cudaStream_t stream);
 cudaError_t launch_accumulate_st(const AccumulateParams& p, int num_sms, cudaStream_t stream);
 cudaError_t launch_accumulate_gps(const AccumulateParams& p, int num_sms, cudaStream_t stream);
