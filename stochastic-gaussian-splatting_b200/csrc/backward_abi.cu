@@ -10,7 +10,7 @@ namespace {
 
 using namespace sgs;
 
-constexpr size_t kAccumFloats = 10;
+constexpr size_t kAccumSums = 10;
 
 struct BackwardSetup {
     BackwardParams p;
@@ -107,7 +107,7 @@ BackwardLayout backward_layout(const uint32_t n) {
     const size_t cap = queue_capacity(n);
     L.colors = 0;
     L.accum = align256(sizeof(float) * ((3 * static_cast<size_t>(n) + 3) & ~size_t(3)));
-    L.queue = L.accum + align256(sizeof(float) * kAccumFloats * n);
+    L.queue = L.accum + align256(sizeof(double) * kAccumSums * n);
     L.entries = L.queue + align256(sizeof(WorkQueue));
     L.meta = L.entries + align256(kWalkGaussianBytes * cap);
     L.index = L.meta + align256(sizeof(uint4) * cap);
@@ -119,7 +119,7 @@ void set_backward_buffers(BackwardParams& p, void* backward_workspace) {
     char* base = static_cast<char*>(backward_workspace);
     const BackwardLayout L = backward_layout(p.n);
     p.colors = reinterpret_cast<float*>(base + L.colors);
-    p.accum = reinterpret_cast<float*>(base + L.accum);
+    p.accum = reinterpret_cast<double*>(base + L.accum);
     p.bw_queue = reinterpret_cast<WorkQueue*>(base + L.queue);
     p.bw_entries = base + L.entries;
     p.bw_meta = reinterpret_cast<uint4*>(base + L.meta);
@@ -159,7 +159,7 @@ int sgs_backward_accumulate(const sgs_gaussians* gaussians, const sgs_camera* ca
     set_backward_buffers(p, backward_workspace);
     cudaError_t err = cudaSuccess;
     if (first) {
-        err = cudaMemsetAsync(p.accum, 0, kAccumFloats * p.n * sizeof(float), stream);
+        err = cudaMemsetAsync(p.accum, 0, kAccumSums * p.n * sizeof(double), stream);
         if (err == cudaSuccess) err = launch_backward_colors(p, stream);
     }
     if (err == cudaSuccess) err = launch_backward_fragments(p, stream);
@@ -238,7 +238,7 @@ int sgs_backward_accumulate_samples(const sgs_gaussians* gaussians, const sgs_ca
     set_backward_buffers(p, backward_workspace);
     cudaError_t err = cudaSuccess;
     if (first) {
-        err = cudaMemsetAsync(p.accum, 0, kAccumFloats * p.n * sizeof(float), stream);
+        err = cudaMemsetAsync(p.accum, 0, kAccumSums * p.n * sizeof(double), stream);
         if (err == cudaSuccess) err = launch_backward_colors(p, stream);
     }
     if (err == cudaSuccess) err = cudaMemsetAsync(p.bw_queue, 0, sizeof(WorkQueue), stream);
@@ -277,7 +277,7 @@ int sgs_backward_accumulate_framebuffers(const sgs_gaussians* gaussians, const s
     S.gps_law = set_sample_table(p, scratch, n_samples, S.gps);
     set_backward_buffers(p, backward_workspace);
     cudaError_t err = cudaSuccess;
-    if (first) err = cudaMemsetAsync(p.accum, 0, kAccumFloats * p.n * sizeof(float), stream);
+    if (first) err = cudaMemsetAsync(p.accum, 0, kAccumSums * p.n * sizeof(double), stream);
     if (err == cudaSuccess) err = launch_backward_colors(p, stream);
     if (err == cudaSuccess) err = launch_backward_framebuffer_terms(p, stream);
     if (err == cudaSuccess) err = cudaMemsetAsync(p.bw_queue, 0, sizeof(WorkQueue), stream);

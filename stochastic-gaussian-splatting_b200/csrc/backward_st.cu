@@ -290,8 +290,11 @@ __global__ void __launch_bounds__(kBlock) colors_kernel(const BackwardParams b) 
     b.colors[3 * g + 2] = c.z;
 }
 
+// A fragment's contributions are float, their sums double: the parameters' gradients, the quaternions'
+// above all, amplify the rounding of these sums some 100 times, and with float sums the order of the
+// atomics alone moved them by up to 4e-5 from run to run (5 % of the walk's time).
 struct FragAccum {
-    float v[kAccum];
+    double v[kAccum];
 };
 
 // Contribution of one fragment of Gaussian k at framebuffer pixel (px, py) to k's accumulators.
@@ -351,7 +354,7 @@ __global__ void __launch_bounds__(kBlock) fragments_backward_kernel(const Backwa
     const float3 ck = make_float3(b.colors[3 * g + 0], b.colors[3 * g + 1], b.colors[3 * g + 2]);
     FragAccum acc;
 #pragma unroll
-    for (int i = 0; i < kAccum; ++i) acc.v[i] = 0.0f;
+    for (int i = 0; i < kAccum; ++i) acc.v[i] = 0.0;
     if (count <= kCoopFragments) {
         for (uint32_t f = 0; f < count; ++f)
             fragment_grad(b, p, ce, key, ck, rect.x_min + f % rect.width, rect.y_min + f / rect.width, acc);
@@ -374,20 +377,20 @@ __global__ void __launch_bounds__(kBlock) fragments_backward_kernel(const Backwa
         const uint32_t w = __shfl_sync(kFullMask, rect.width, src), n = __shfl_sync(kFullMask, count, src);
         FragAccum part;
 #pragma unroll
-        for (int i = 0; i < kAccum; ++i) part.v[i] = 0.0f;
+        for (int i = 0; i < kAccum; ++i) part.v[i] = 0.0;
         for (uint32_t f = lane; f < n; f += 32) fragment_grad(b, q, qce, qkey, qck, x0 + f % w, y0 + f / w, part);
 #pragma unroll
         for (int i = 0; i < kAccum; ++i) {
-            float v = part.v[i];
+            double v = part.v[i];
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
             if (lane == src) acc.v[i] += v;
         }
     }
     if (!active) return;
-    float* out = b.accum + static_cast<size_t>(g) * kAccum;
+    double* out = b.accum + static_cast<size_t>(g) * kAccum;
 #pragma unroll
     for (int i = 0; i < kAccum; ++i)
-        if (acc.v[i] != 0.0f) out[i] += acc.v[i];
+        if (acc.v[i] != 0.0) out[i] += acc.v[i];
 }
 
 
@@ -603,22 +606,26 @@ __device__ __forceinline__ void walk_row_gradients(const BackwardParams& b, cons
     }
 }
 
+// Threads of a walk block (at most 48 KB of shared memory).
+constexpr uint32_t walk_block(const bool gps) { return gps ? 128u : 256u; }
+
 // One thread per Gaussian: the rows of a warp's 32 Gaussians are laid end to end, 32 per step, and
 // each lane walks one row; the row sums go to per-Gaussian accumulators in shared memory.
 template <bool kGps>
-__global__ void __launch_bounds__(kBlock) fragments_samples_kernel(const BackwardParams b, const float2* __restrict__ law) {
-    __shared__ WalkGaussian s_g[kWarpsPerBlock][32];
-    __shared__ GpsConstants s_c[kGps ? kWarpsPerBlock : 1][32];
-    __shared__ float s_acc[kWarpsPerBlock][32][kAccum];
+__global__ void __launch_bounds__(walk_block(kGps)) fragments_samples_kernel(const BackwardParams b, const float2* __restrict__ law) {
+    constexpr uint32_t kWarps = walk_block(kGps) / 32u;
+    __shared__ WalkGaussian s_g[kWarps][32];
+    __shared__ GpsConstants s_c[kGps ? kWarps : 1][32];
+    __shared__ double s_acc[kWarps][32][kAccum];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t wib = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
     const uint32_t upto_mask = kFullMask >> (31u - lane);
-    const uint32_t idx = blockIdx.x * kBlock + threadIdx.x;
+    const uint32_t idx = blockIdx.x * walk_block(kGps) + threadIdx.x;
     bool active = idx < b.n;
     const uint32_t g = active ? idx : b.n - 1;
 #pragma unroll
-    for (int i = 0; i < kAccum; ++i) s_acc[wib][lane][i] = 0.0f;
+    for (int i = 0; i < kAccum; ++i) s_acc[wib][lane][i] = 0.0;
     Projected p;
     if (!project_gaussian(active, g, b.means, b.scales, b.rotations, b.opacities, b.w2c, b.cam, p)) return;
     const PixelRect rect = pixel_rect(p.bounds, b.cam);
@@ -727,21 +734,21 @@ __global__ void __launch_bounds__(kBlock) fragments_samples_kernel(const Backwar
         const GpsConstants rc = kGps ? s_c[wib][valid ? owner : 0] : GpsConstants{};
         FragAccum acc;
 #pragma unroll
-        for (int i = 0; i < kAccum; ++i) acc.v[i] = 0.0f;
+        for (int i = 0; i < kAccum; ++i) acc.v[i] = 0.0;
         walk_row_gradients<kGps>(b, rq, rc, law, valid, rq.y_min + (r - rq.row_first), acc);
         if (valid) {
 #pragma unroll
             for (int i = 0; i < kAccum; ++i)
-                if (acc.v[i] != 0.0f) atomicAdd(&s_acc[wib][owner][i], acc.v[i]);
+                if (acc.v[i] != 0.0) atomicAdd(&s_acc[wib][owner][i], acc.v[i]);
         }
     }
     __syncwarp();
     if (!has_rows) return;
-    float* out = b.accum + static_cast<size_t>(g) * kAccum;
+    double* out = b.accum + static_cast<size_t>(g) * kAccum;
 #pragma unroll
     for (int i = 0; i < kAccum; ++i) {
-        const float v = s_acc[wib][slot][i];
-        if (v != 0.0f) out[i] += v;
+        const double v = s_acc[wib][slot][i];
+        if (v != 0.0) out[i] += v;
     }
 }
 
@@ -790,15 +797,15 @@ __global__ void __launch_bounds__(kBlock) fragments_samples_queue_kernel(const B
         const uint32_t r = r0 + (lane & ((1u << log_rows) - 1u));
         FragAccum acc;
 #pragma unroll
-        for (int i = 0; i < kAccum; ++i) acc.v[i] = 0.0f;
+        for (int i = 0; i < kAccum; ++i) acc.v[i] = 0.0;
         walk_row_gradients<kGps>(b, q, gc, law, r < m.y, q.y_min + r, acc, lane >> log_rows, 5u - log_rows);
-        float* out = b.accum + static_cast<size_t>(b.bw_index[lo]) * kAccum;
+        double* out = b.accum + static_cast<size_t>(b.bw_index[lo]) * kAccum;
 #pragma unroll
         for (int i = 0; i < kAccum; ++i) {
-            float v = acc.v[i];
+            double v = acc.v[i];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
-            if (lane == 0 && v != 0.0f) atomicAdd(out + i, v);
+            if (lane == 0 && v != 0.0) atomicAdd(out + i, v);
         }
     }
 }
@@ -834,7 +841,7 @@ __device__ __forceinline__ void gaussian_gradients(const BackwardParams& b, cons
     bool any = false;
 #pragma unroll
     for (int i = 0; i < kAccum; ++i) {
-        acc[i] = b.accum[static_cast<size_t>(g) * kAccum + i];
+        acc[i] = static_cast<float>(b.accum[static_cast<size_t>(g) * kAccum + i]);
         any |= acc[i] != 0.0f;
     }
     float* dm = b.d_means + 3 * static_cast<size_t>(g);
@@ -1059,10 +1066,9 @@ cudaError_t launch_backward_sample_terms(const BackwardParams& p, cudaStream_t s
 
 cudaError_t launch_backward_fragments_samples(const BackwardParams& p, cudaStream_t stream) {
     if (p.n == 0) return cudaSuccess;
-    const unsigned grid = (p.n + kBlock - 1) / kBlock;
     const unsigned queue_grid = static_cast<unsigned>(max(p.num_sms, 1)) * kQueueBlocksPerSM;
     tile_far_kernel<<<(p.tiles_x * p.tiles_y + kWarpsPerBlock - 1) / kWarpsPerBlock, kBlock, 0, stream>>>(p);
-    fragments_samples_kernel<false><<<grid, kBlock, 0, stream>>>(p, nullptr);
+    fragments_samples_kernel<false><<<(p.n + walk_block(false) - 1) / walk_block(false), walk_block(false), 0, stream>>>(p, nullptr);
     fragments_samples_queue_kernel<false><<<queue_grid, kBlock, 0, stream>>>(p, nullptr);
     return cudaGetLastError();
 }
@@ -1070,11 +1076,10 @@ cudaError_t launch_backward_fragments_samples(const BackwardParams& p, cudaStrea
 cudaError_t launch_backward_fragments_samples_gps(const BackwardParams& p, float2* law, cudaStream_t stream) {
     if (p.n == 0) return cudaSuccess;
     if (law == nullptr) return cudaErrorInvalidValue;
-    const unsigned grid = (p.n + kBlock - 1) / kBlock;
     const unsigned queue_grid = static_cast<unsigned>(max(p.num_sms, 1)) * kQueueBlocksPerSM;
     gps_count_law_kernel<<<kLawRows, 32, 0, stream>>>(law);
     tile_far_kernel<<<(p.tiles_x * p.tiles_y + kWarpsPerBlock - 1) / kWarpsPerBlock, kBlock, 0, stream>>>(p);
-    fragments_samples_kernel<true><<<grid, kBlock, 0, stream>>>(p, law);
+    fragments_samples_kernel<true><<<(p.n + walk_block(true) - 1) / walk_block(true), walk_block(true), 0, stream>>>(p, law);
     fragments_samples_queue_kernel<true><<<queue_grid, kBlock, 0, stream>>>(p, law);
     return cudaGetLastError();
 }

@@ -265,7 +265,7 @@ struct BackwardParams {
     const float* grad_depth;                 // (H, W) or null
     float grad_scale;                        // weight of this sample in the output / ss^2
     float* colors;                           // (N, 3) per-Gaussian colour
-    float* accum;                            // (N, 10) projected-quantity gradients
+    double* accum;                           // (N, 10) projected-quantity gradients
     float* d_means;
     float* d_scales;
     float* d_rotations;
