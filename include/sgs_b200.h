@@ -327,6 +327,21 @@ size_t sgs_denoise_scratch_size(int32_t batch, int32_t height, int32_t width);
 int sgs_denoise(const void* features, int32_t batch, int32_t height, int32_t width, const void* weights,
                 const float* biases, void* scratch, size_t scratch_bytes, float* output, void* stream);
 
+/* A training step of the denoiser in two calls. Forward: `params` holds 12 device pointers, FP32
+ * W1[co][ci][3][3], b1[co], ..., W6, b6 with the model's channel counts (7 -> 32 -> ... -> 3); the features
+ * (FP16 [batch][height][width][8]) give `output` (FP32 [batch][height][width][3]), and `saved` keeps what the
+ * backward needs. Backward: `weights` holds the 6 device pointers of the weights; `grads` receives
+ * sgs_denoise_train_params() floats, the gradients of W1, b1, ..., W6, b6 back to back. Buffers are
+ * 16-byte aligned; the same bits as the layers through sgs_conv3x3. */
+size_t sgs_denoise_train_params(void);
+size_t sgs_denoise_train_saved_size(int32_t batch, int32_t height, int32_t width);
+size_t sgs_denoise_train_scratch_size(int32_t batch, int32_t height, int32_t width);
+int sgs_denoise_train_forward(const void* features, int32_t batch, int32_t height, int32_t width,
+                              const float* const* params, void* saved, size_t saved_bytes, float* output, void* stream);
+int sgs_denoise_train_backward(const float* grad_output, int32_t batch, int32_t height, int32_t width,
+                               const float* const* weights, const void* saved, void* scratch, size_t scratch_bytes,
+                               float* grads, void* stream);
+
 /* Synchronises `stream` and reports whether a denoiser kernel gave up a bounded tensor-core wait
  * (SGS_ERROR_CUDA), clearing the flag. */
 int sgs_denoise_status(void* stream);

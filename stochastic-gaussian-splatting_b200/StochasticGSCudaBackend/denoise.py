@@ -129,37 +129,58 @@ def _padded_bias(b: torch.Tensor, n: int) -> torch.Tensor:
     return out
 
 
+def _pointers(tensors) -> ctypes.Array:
+    return (ctypes.c_void_p * len(tensors))(*(t.data_ptr() for t in tensors))
+
+
+def _master(p: torch.Tensor, shape: tuple, device: torch.device) -> torch.Tensor:
+    if tuple(p.shape) != shape or p.device != device:
+        raise RuntimeError(f"denoiser parameters must have the model's shapes on {device}, got {tuple(p.shape)} on {p.device}")
+    return p.detach().to(torch.float32).contiguous()
+
+
 class _DenoiseTrain(torch.autograd.Function):
+    """Forward and backward as one C-ABI call each (sgs_denoise_train_forward / _backward): the weights are
+    packed, the gradients staged and unpacked by kernels, not by tensor operations per layer."""
+
     @staticmethod
     def forward(ctx, features, *params):
-        ws = [pack_forward(params[2 * l].detach(), STAGED_IN[l], STAGED_OUT[l]) for l in range(6)]
-        bs = [_padded_bias(params[2 * l + 1].detach(), STAGED_OUT[l]) for l in range(6)]
-        acts = [features]
-        x = features
-        for l in range(5):
-            x = conv3x3(x, ws[l], bs[l], ABI_IN[l], STAGED_OUT[l], _abi.SGS_CONV_RELU)
-            acts.append(x)
-        out = conv3x3(x, ws[5], bs[5], ABI_IN[5], STAGED_OUT[5], _abi.SGS_CONV_FINAL, residual=features)
-        ctx.acts = acts
-        ctx.save_for_backward(*[p.detach() for p in params[0::2]])
+        b, h, w = features.shape[:3]
+        dev = features.device
+        if features.dtype != torch.float16 or features.dim() != 4 or features.shape[3] != FEATURES:
+            raise RuntimeError("features must be a float16 (B, H, W, 8) tensor")
+        if len(params) != 12:
+            raise RuntimeError(f"denoise_train takes 12 parameters, got {len(params)}")
+        features = features.contiguous()
+        masters = [_master(p, ((LAYERS[i // 2][1], LAYERS[i // 2][0], 3, 3) if i % 2 == 0 else (LAYERS[i // 2][1],)), dev)
+                   for i, p in enumerate(params)]
+        saved = torch.empty(_lib.sgs_denoise_train_saved_size(b, h, w), dtype=torch.uint8, device=dev)
+        out = torch.empty((b, h, w, 3), dtype=torch.float32, device=dev)
+        _check(_lib.sgs_denoise_train_forward(features.data_ptr(), b, h, w, _pointers(masters), saved.data_ptr(),
+                                              saved.numel(), out.data_ptr(), _stream(dev)),
+               "sgs_denoise_train_forward")
+        ctx.saved = saved
+        ctx.save_for_backward(*masters[0::2])
         return out
 
     @staticmethod
     def backward(ctx, g_out):
-        weights = ctx.saved_tensors
-        acts = ctx.acts
+        weights = [w.contiguous() for w in ctx.saved_tensors]
         b, h, w = g_out.shape[:3]
-        gz = torch.zeros((b, h, w, STAGED_OUT[5]), dtype=torch.bfloat16, device=g_out.device)
-        gz[..., :3] = g_out
-        grads = [None] * 12
-        for l in range(5, -1, -1):
-            gw, gb = conv3x3_wgrad(acts[l], ABI_IN[l], gz, STAGED_OUT[l])
-            grads[2 * l] = unpack_wgrad(gw, l)
-            grads[2 * l + 1] = gb[:LAYERS[l][1]].clone()
-            if l > 0:
-                wd = pack_dgrad(weights[l], STAGED_IN[l], STAGED_OUT[l])
-                gz = conv3x3(gz, wd, None, STAGED_OUT[l], STAGED_IN[l], _abi.SGS_CONV_MASK, mask=acts[l])
-        ctx.acts = None
+        dev = g_out.device
+        g_out = g_out.to(torch.float32).contiguous()
+        scratch = torch.empty(_lib.sgs_denoise_train_scratch_size(b, h, w), dtype=torch.uint8, device=dev)
+        flat = torch.empty(_lib.sgs_denoise_train_params(), dtype=torch.float32, device=dev)
+        _check(_lib.sgs_denoise_train_backward(g_out.data_ptr(), b, h, w, _pointers(weights), ctx.saved.data_ptr(),
+                                               scratch.data_ptr(), scratch.numel(), flat.data_ptr(), _stream(dev)),
+               "sgs_denoise_train_backward")
+        ctx.saved = None
+        grads, at = [], 0
+        for ci, co in LAYERS:
+            grads.append(flat[at:at + 9 * ci * co].view(co, ci, 3, 3))
+            at += 9 * ci * co
+            grads.append(flat[at:at + co])
+            at += co
         # the residual path gives the features a gradient too; the input is data, not trained
         return (None, *grads)
 

@@ -6,6 +6,8 @@
 //                         (bias + ReLU, or bias + residual for the last layer) and data gradients
 //                         (flipped, transposed weights; the ReLU mask of the layer below fused).
 //   conv3x3_wgrad_kernel  weight and bias gradients of one layer, summed over all pixels.
+//   conv3x3_wgrad_tma_kernel the same for BF16 inputs, loaded by TMA.
+//   train_*               one training step's weight packing, gradient staging and unpacking.
 //   features_*            the 8-channel FP16 input built from the per-sample renders.
 //
 // Activations are NHWC BF16 [batch][height][width][channels], channels 16 or 32. One CTA of 128
@@ -557,6 +559,250 @@ __global__ void __launch_bounds__(kThreads) conv3x3_wgrad_kernel(const WgradArgs
     }
 }
 
+// Weight and bias gradients of a layer with BF16 input, persistent and warp-specialised. Warp 4 loads,
+// per tile, the input halo with TMA three times, shifted by the taps' dx (one box of 8 channels x 8 x 18
+// pixels each, zero fill outside the image), and the tile's output gradient; warp 5 multiplies them,
+// pixels as K. A row of 8 pixels is one core matrix, so the taps' dy are row offsets, and one MMA of
+// M = 128 holds the rows (dx, input channel) of one dy, then the bias row (a constant group of ones)
+// and rows that nothing reads. No im2col copy: with it a tile took 7.9 us, loads, copies and MMAs in
+// turn (55 us per 16 x 128 x 128 layer). The accumulators stay in TMEM over all of a CTA's tiles.
+template <int CIN, int COUT>
+struct WgradTma {
+    static constexpr int KC = CIN / 8;
+    static constexpr int KCO = COUT / 8;
+    static constexpr int kStages = 4;
+    static constexpr uint32_t kGroup = kTileW * kHaloH * 16;  // one 8-channel group of a shifted halo
+    static constexpr int kOnes = 3 * KC;                      // the group after the three shifts
+    static constexpr uint32_t kGradOffset = (kOnes + 1) * kGroup;
+    static constexpr uint32_t kGradGroup = kTilePx * 16;
+    static constexpr uint32_t kStage = kGradOffset + KCO * kGradGroup;
+    static constexpr uint32_t kTxBytes = kOnes * kGroup + KCO * kGradGroup;
+    // the rows that nothing reads lie in 16 groups from a stage's start, at most 16 tile rows further
+    static constexpr uint32_t kReach = 15 * kGroup + 18 * kTileW * 16;
+    static constexpr uint32_t kPad = kReach > kStage ? kReach - kStage : 0;
+    static constexpr int kCols = 3 * COUT <= 64 ? 64 : 128;
+    static constexpr int kBars = 2 * kStages + 1;
+    static constexpr size_t kSmem = static_cast<size_t>(kStages) * kStage + kPad + kBars * 8 + 16 + 128;
+    static_assert(kGroup % 128 == 0 && kGradOffset % 128 == 0 && kStage % 128 == 0, "128-byte TMA destinations");
+    static_assert(kOnes < 16, "the bias group is a row group of the MMA");
+};
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kTmaThreads) conv3x3_wgrad_tma_kernel(const __grid_constant__ CUtensorMap in_map,
+                                                                       const __grid_constant__ CUtensorMap grad_map,
+                                                                       const WgradArgs a) {
+    using G = WgradTma<CIN, COUT>;
+    constexpr uint32_t kIdesc = tc::instr_desc_bf16(kTilePx, COUT, true, true);
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char* const base = smem_raw + ((128u - (tc::smem_u32(smem_raw) & 127u)) & 127u);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + G::kStages * G::kStage + G::kPad);
+    uint32_t* slot = reinterpret_cast<uint32_t*>(bars + G::kBars);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t bar0 = tc::smem_u32(bars);
+    const uint32_t done = bar0 + 8u * (2 * G::kStages);
+#define SGS_FULL(st) (bar0 + 8u * (st))
+#define SGS_EMPTY(st) (bar0 + 8u * (G::kStages + (st)))
+    for (int st = 0; st < G::kStages; ++st)
+        for (uint32_t i = tid; i < G::kGroup / 16; i += kTmaThreads)
+            reinterpret_cast<uint4*>(base + st * G::kStage + G::kOnes * G::kGroup)[i] = make_uint4(0x3F80u, 0u, 0u, 0u);
+    tc::fence_async_smem();
+    if (warp == 0) tc::tmem_alloc(tc::smem_u32(slot), G::kCols);
+    if (tid == 0)
+        for (int i = 0; i < G::kBars; ++i) tc::mbar_init(bar0 + 8u * i, 1);
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = *slot;
+    const uint32_t smem0 = tc::smem_u32(base);
+    bool failed = false;
+    int issued = 0;  // producer: tiles whose loads were issued; MMA: tiles whose MMAs were committed
+
+    if (warp == 4) {
+        if (lane == 0) {
+            for (int t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++issued) {
+                const int st = issued % G::kStages;
+                if (issued >= G::kStages &&
+                    !tc::mbar_wait(SGS_EMPTY(st), ((issued / G::kStages) & 1u) ^ 1u, kWaitLimit)) {
+                    failed = true;
+                    break;
+                }
+                const TileXY tile = tile_xy(t, a.tiles_x, a.tiles_y);
+                const uint32_t dst = smem0 + st * G::kStage;
+                tc::mbar_arrive_expect_tx(SGS_FULL(st), G::kTxBytes);
+#pragma unroll
+                for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+                    for (int c = 0; c < G::KC; ++c)
+                        tc::tma_load_4d(dst + (dx * G::KC + c) * G::kGroup, &in_map, SGS_FULL(st), c * 8,
+                                        tile.x0 - 1 + dx, tile.y0 - 1, tile.b);
+#pragma unroll
+                for (int c = 0; c < G::KCO; ++c)
+                    tc::tma_load_4d(dst + G::kGradOffset + c * G::kGradGroup, &grad_map, SGS_FULL(st), c * 8, tile.x0,
+                                    tile.y0, tile.b);
+            }
+        }
+    } else if (warp == 5) {
+        if (lane == 0) {
+            for (int t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++issued) {
+                const int st = issued % G::kStages;
+                if (!tc::mbar_wait(SGS_FULL(st), (issued / G::kStages) & 1u, kWaitLimit)) {
+                    failed = true;
+                    break;
+                }
+                tc::fence_after_sync();
+                const uint32_t in = smem0 + st * G::kStage, grad = in + G::kGradOffset;
+#pragma unroll
+                for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                    for (int kk = 0; kk < kTilePx / 16; ++kk)
+                        tc::mma_bf16(tmem + dy * COUT, tc::smem_desc(in + (dy + 2 * kk) * (kTileW * 16), 128, G::kGroup),
+                                     tc::smem_desc(grad + kk * 256, 128, G::kGradGroup), kIdesc,
+                                     (issued | kk) != 0 ? 1u : 0u);
+                tc::commit(SGS_EMPTY(st));
+            }
+            if (!failed) tc::commit(done);
+        }
+    } else {
+        // the CTA's sums, once its last tile's MMAs are through
+        const uint32_t tiles = (a.n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;  // one wait's limit for each
+        const bool ok = __all_sync(0xFFFFFFFFu, tc::mbar_wait(done, 0, kWaitLimit * min(tiles, 4000u)));
+        failed = !ok;
+        if (ok) {
+            tc::fence_after_sync();
+            const int group = tid >> 3, ch = tid & 7;
+#pragma unroll
+            for (int dy = 0; dy < 3; ++dy) {
+                float acc[COUT];
+                load_accumulator<COUT>(tmem + (static_cast<uint32_t>(warp * 32) << 16) + dy * COUT, acc);
+                if (group < G::kOnes) {
+                    const int tap = dy * 3 + group / G::KC, ci = group % G::KC * 8 + ch;
+#pragma unroll
+                    for (int n = 0; n < COUT; ++n) atomicAdd(a.grad_w + (tap * COUT + n) * CIN + ci, acc[n]);
+                } else if (group == G::kOnes && ch == 0 && dy == 0) {
+#pragma unroll
+                    for (int n = 0; n < COUT; ++n) atomicAdd(a.grad_b + n, acc[n]);
+                }
+            }
+        }
+    }
+    if (__syncthreads_or(failed)) {
+        if (tid == 0) atomicExch(&g_error, 1u);
+        // let this CTA's own copies and MMAs in flight finish (bounded) before its memory goes away
+        if (warp == 4 && lane == 0)
+            for (int q = issued - 1; q >= 0 && q >= issued - G::kStages; --q)
+                tc::mbar_wait(SGS_FULL(q % G::kStages), (q / G::kStages) & 1u, kWaitLimit);
+        if (warp == 5 && lane == 0 && issued > 0)
+            tc::mbar_wait(SGS_EMPTY((issued - 1) % G::kStages), ((issued - 1) / G::kStages) & 1u, kWaitLimit);
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) {
+        tc::fence_after_sync();
+        tc::tmem_dealloc(tmem, G::kCols);
+    }
+#undef SGS_FULL
+#undef SGS_EMPTY
+}
+
+// ---- training step: packing, staging, unpacking ------------------------------------------------
+
+constexpr int kTrainLayers = SGS_DENOISE_LAYERS;
+__host__ __device__ constexpr int model_in(int l) { return l == 0 ? 7 : 32; }
+__host__ __device__ constexpr int model_out(int l) { return l == kTrainLayers - 1 ? 3 : 32; }
+__host__ __device__ constexpr int staged_in(int l) { return l == 0 ? 16 : 32; }
+__host__ __device__ constexpr int staged_out(int l) { return l == kTrainLayers - 1 ? 16 : 32; }
+// elements of the forward weights, of the weight-gradient sums (8 input channels in the first layer) and
+// of the parameters before layer l
+__host__ __device__ constexpr int packed_before(int l) {
+    int n = 0;
+    for (int i = 0; i < l; ++i) n += 9 * staged_in(i) * staged_out(i);
+    return n;
+}
+__host__ __device__ constexpr int sums_before(int l) {
+    int n = 0;
+    for (int i = 0; i < l; ++i) n += 9 * (i == 0 ? 8 : 32) * staged_out(i);
+    return n;
+}
+__host__ __device__ constexpr int params_before(int l) {
+    int n = 0;
+    for (int i = 0; i < l; ++i) n += (9 * model_in(i) + 1) * model_out(i);
+    return n;
+}
+__host__ __device__ constexpr int bias_before(int l) { return 32 * l; }
+constexpr int kPacked = packed_before(kTrainLayers), kSums = sums_before(kTrainLayers);
+constexpr int kParams = params_before(kTrainLayers), kBiases = 32 * (kTrainLayers - 1) + 16;
+
+struct TrainParams {
+    const float* weights[kTrainLayers];  // W[co][ci][3][3]
+    const float* biases[kTrainLayers];
+};
+
+// Forward weights of all layers as BF16 [tap][ci / 8][co][ci % 8] and FP32 biases, zero-padded to the staged
+// channels, and (the blocks behind them) the FP16 features as BF16.
+constexpr int kPackBlocks = (kPacked + kBiases + 255) / 256;
+__global__ void __launch_bounds__(256) train_pack_kernel(const TrainParams p, __nv_bfloat16* __restrict__ weights,
+                                                         float* __restrict__ biases, const uint4* __restrict__ features,
+                                                         uint4* __restrict__ features_bf16, const uint32_t n_px) {
+    if (blockIdx.x >= kPackBlocks) {
+        const uint32_t i = (blockIdx.x - kPackBlocks) * 256u + threadIdx.x;
+        if (i < n_px) features_bf16[i] = half8_to_bf16x8(__ldg(features + i));
+        return;
+    }
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < kPacked) {
+        int l = 0;
+        while (l + 1 < kTrainLayers && i >= packed_before(l + 1)) ++l;
+        const int si = staged_in(l), so = staged_out(l), mi = model_in(l), mo = model_out(l);
+        const int r = i - packed_before(l);
+        const int ci = r / (so * 8) % (si / 8) * 8 + r % 8, co = r / 8 % so, tap = r / (si * so);
+        weights[i] = __float2bfloat16_rn(ci < mi && co < mo ? p.weights[l][(co * mi + ci) * 9 + tap] : 0.0f);
+    } else if (i < kPacked + kBiases) {
+        const int r = i - kPacked, l = r / 32;
+        biases[r] = r % 32 < model_out(l) ? p.biases[l][r % 32] : 0.0f;
+    }
+}
+
+// Data-gradient weights of the layers above the first, BF16 [tap][co / 8][ci][co % 8] = W[co][ci][8 - tap], and
+// (the blocks behind them) the output gradient as BF16 with 16 channels.
+constexpr int kDgradBlocks = (kPacked - packed_before(1) + 255) / 256;
+__global__ void __launch_bounds__(256) train_stage_kernel(const TrainParams p, __nv_bfloat16* __restrict__ weights,
+                                                          const float* __restrict__ grad, uint4* __restrict__ staged,
+                                                          const uint32_t n_px) {
+    if (blockIdx.x >= kDgradBlocks) {
+        const uint32_t i = (blockIdx.x - kDgradBlocks) * 256u + threadIdx.x;
+        if (i >= n_px) return;
+        const float* const g = grad + 3 * static_cast<size_t>(i);
+        staged[2 * static_cast<size_t>(i)] = make_uint4(pack_bf16(g[0], g[1]), pack_bf16(g[2], 0.0f), 0u, 0u);
+        staged[2 * static_cast<size_t>(i) + 1] = make_uint4(0u, 0u, 0u, 0u);
+        return;
+    }
+    const int i = packed_before(1) + blockIdx.x * 256 + threadIdx.x;
+    if (i >= kPacked) return;
+    int l = 1;
+    while (l + 1 < kTrainLayers && i >= packed_before(l + 1)) ++l;
+    const int si = staged_in(l), so = staged_out(l), mi = model_in(l), mo = model_out(l);
+    const int r = i - packed_before(l);
+    const int co = r / (si * 8) % (so / 8) * 8 + r % 8, ci = r / 8 % si, tap = r / (si * so);
+    weights[i - packed_before(1)] =
+        __float2bfloat16_rn(ci < mi && co < mo ? p.weights[l][(co * mi + ci) * 9 + 8 - tap] : 0.0f);
+}
+
+// Parameter gradients W1[co][ci][3][3], b1, ..., back to back from the sums [tap][co][ci] and bias sums.
+__global__ void __launch_bounds__(256) train_unpack_kernel(const float* __restrict__ sums, float* __restrict__ grads) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= kParams) return;
+    int l = 0;
+    while (l + 1 < kTrainLayers && i >= params_before(l + 1)) ++l;
+    const int mi = model_in(l), mo = model_out(l), so = staged_out(l), si = l == 0 ? 8 : 32;
+    const int r = i - params_before(l);
+    if (r < 9 * mi * mo) {
+        const int tap = r % 9, ci = r / 9 % mi, co = r / (9 * mi);
+        grads[i] = sums[sums_before(l) + (tap * so + co) * si + ci];
+    } else {
+        grads[i] = sums[kSums + bias_before(l) + (r - 9 * mi * mo)];
+    }
+}
+
 // ---- input features -----------------------------------------------------------------------
 
 // accum per pixel: float4 (sum r, sum g, sum b, sum alpha), float4 (sum depth, sum lum^2,
@@ -663,9 +909,9 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_tiled() {
     return fn;
 }
 
-// 4-D map over a BF16 NHWC tensor [batch][height][width][channels] with a box of 8 channels x the
-// 10 x 18 halo x 1 image.
-bool nhwc_halo_map(CUtensorMap* map, const void* base, int batch, int height, int width, int channels) {
+// 4-D map over a BF16 NHWC tensor [batch][height][width][channels] with a box of 8 channels x
+// box_w x box_h pixels x 1 image.
+bool nhwc_map(CUtensorMap* map, const void* base, int batch, int height, int width, int channels, int box_w, int box_h) {
     const auto fn = encode_tiled();
     if (fn == nullptr) return false;
     const cuuint64_t dims[4] = {static_cast<cuuint64_t>(channels), static_cast<cuuint64_t>(width),
@@ -673,7 +919,7 @@ bool nhwc_halo_map(CUtensorMap* map, const void* base, int batch, int height, in
     const cuuint64_t strides[3] = {static_cast<cuuint64_t>(channels) * 2,
                                    static_cast<cuuint64_t>(width) * channels * 2,
                                    static_cast<cuuint64_t>(height) * width * channels * 2};
-    const cuuint32_t box[4] = {8, kHaloW, kHaloH, 1};
+    const cuuint32_t box[4] = {8, static_cast<cuuint32_t>(box_w), static_cast<cuuint32_t>(box_h), 1};
     const cuuint32_t elem[4] = {1, 1, 1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, elem,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -697,15 +943,16 @@ bool planar_halo_map(CUtensorMap* map, const void* base, int batch, int height, 
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// in_channels: the tensor's channels where fewer than CIN (the others read zeros).
 template <int CIN, int COUT, int EPI, bool kPlanar = false>
-cudaError_t launch_conv_tma(const ConvArgs& a, cudaStream_t stream) {
+cudaError_t launch_conv_tma(const ConvArgs& a, cudaStream_t stream, int in_channels = CIN) {
     using S = TmaConv<CIN, COUT>;
     auto kernel = conv3x3_tma_kernel<CIN, COUT, EPI, kPlanar>;
     static const int per_sm = resident_ctas(kernel, S::kSmem, 512 / kTmaCols, kTmaThreads);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
     CUtensorMap map;
     const bool mapped = kPlanar ? planar_halo_map(&map, a.in, a.batch, a.height, a.width, CIN)
-                                : nhwc_halo_map(&map, a.in, a.batch, a.height, a.width, CIN);
+                                : nhwc_map(&map, a.in, a.batch, a.height, a.width, in_channels, kHaloW, kHaloH);
     if (!mapped) return cudaErrorInvalidValue;
     const int grid = a.n_tiles < sm_count() * per_sm ? a.n_tiles : sm_count() * per_sm;
     kernel<<<grid, kTmaThreads, S::kSmem, stream>>>(map, a);
@@ -724,6 +971,21 @@ cudaError_t launch_wgrad(const WgradArgs& a, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
+template <int CIN, int COUT>
+cudaError_t launch_wgrad_tma(const WgradArgs& a, cudaStream_t stream) {
+    using G = WgradTma<CIN, COUT>;
+    auto kernel = conv3x3_wgrad_tma_kernel<CIN, COUT>;
+    static const int per_sm = resident_ctas(kernel, G::kSmem, 512 / G::kCols, kTmaThreads);
+    if (per_sm <= 0) return cudaErrorInvalidConfiguration;
+    CUtensorMap in_map, grad_map;
+    if (!nhwc_map(&in_map, a.in, a.batch, a.height, a.width, CIN, kTileW, kHaloH) ||
+        !nhwc_map(&grad_map, a.grad_out, a.batch, a.height, a.width, COUT, kTileW, kTileH))
+        return cudaErrorInvalidValue;
+    const int grid = a.n_tiles < sm_count() * per_sm ? a.n_tiles : sm_count() * per_sm;
+    kernel<<<grid, kTmaThreads, G::kSmem, stream>>>(in_map, grad_map, a);
+    return cudaGetLastError();
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 size_t weights_bytes(int in_channels, int out_channels) {
@@ -739,6 +1001,33 @@ int check_shape(int batch, int height, int width) {
     if (tiles > 0x7FFFFFFFll)
         return record_error(SGS_ERROR_INVALID_ARGUMENT, "conv3x3: too many pixels for one call");
     return SGS_OK;
+}
+
+// Buffers of a training step: `saved` (BF16 features, the five hidden activations, the packed weights and
+// biases) from forward to backward, `scratch` (BF16 gradients of the output and of two hidden layers in
+// turn, data-gradient weights, weight-gradient sums) in the backward.
+struct TrainLayout {
+    uint32_t n_px;
+    size_t act_bytes;
+    size_t features, acts, weights, biases, saved;
+    size_t grad16, grad32, dgrad, sums, scratch;
+};
+
+TrainLayout train_layout(int batch, int height, int width) {
+    auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
+    TrainLayout L{};
+    const size_t px = static_cast<size_t>(batch) * height * width;
+    L.n_px = static_cast<uint32_t>(px);
+    L.act_bytes = up(px * SGS_DENOISE_WIDTH * 2);
+    L.acts = up(px * 16);
+    L.weights = L.acts + (kTrainLayers - 1) * L.act_bytes;
+    L.biases = L.weights + up(kPacked * 2);
+    L.saved = L.biases + up(kBiases * 4);
+    L.grad32 = up(px * 32);
+    L.dgrad = L.grad32 + 2 * L.act_bytes;
+    L.sums = L.dgrad + up((kPacked - packed_before(1)) * 2);
+    L.scratch = L.sums + up((kSums + kBiases) * 4);
+    return L;
 }
 
 // Layer shapes of the denoiser: (input channels as the ABI counts them, output channels, epilogue).
@@ -812,9 +1101,9 @@ int sgs_conv3x3_wgrad(const void* input, int32_t in_channels, const void* grad_o
     if (in_channels == 8 && out_channels == 32)
         err = launch_wgrad<16, 32, kInFeatures>(a, stream);
     else if (in_channels == 32 && out_channels == 32)
-        err = launch_wgrad<32, 32, kInBf16>(a, stream);
+        err = launch_wgrad_tma<32, 32>(a, stream);
     else if (in_channels == 32 && out_channels == 16)
-        err = launch_wgrad<32, 16, kInBf16>(a, stream);
+        err = launch_wgrad_tma<32, 16>(a, stream);
     else
         return record_error(SGS_ERROR_INVALID_ARGUMENT, "conv3x3_wgrad: unsupported shape %d -> %d", in_channels,
                             out_channels);
@@ -897,6 +1186,115 @@ int sgs_denoise(const void* features, int32_t batch, int32_t height, int32_t wid
         w += weights_bytes(kLayerIn[l], kLayerOut[l]);
         b += kLayerOut[l];
     }
+    return SGS_OK;
+}
+
+size_t sgs_denoise_train_params(void) { return kParams; }
+
+size_t sgs_denoise_train_saved_size(int32_t batch, int32_t height, int32_t width) {
+    if (batch <= 0 || height <= 0 || width <= 0) return 0;
+    return train_layout(batch, height, width).saved;
+}
+
+size_t sgs_denoise_train_scratch_size(int32_t batch, int32_t height, int32_t width) {
+    if (batch <= 0 || height <= 0 || width <= 0) return 0;
+    return train_layout(batch, height, width).scratch;
+}
+
+int sgs_denoise_train_forward(const void* features, int32_t batch, int32_t height, int32_t width,
+                              const float* const* params, void* saved, size_t saved_bytes, float* output,
+                              void* stream_ptr) {
+    if (int st = check_shape(batch, height, width)) return st;
+    if (features == nullptr || params == nullptr || saved == nullptr || output == nullptr)
+        return record_error(SGS_ERROR_INVALID_ARGUMENT, "denoise train: all arrays are required");
+    const TrainLayout L = train_layout(batch, height, width);
+    if (saved_bytes < L.saved || !aligned16(saved))
+        return record_error(SGS_ERROR_WORKSPACE, "denoise train: the saved buffer needs %zu bytes, 16-byte aligned",
+                            L.saved);
+    if (!aligned16(features)) return record_error(SGS_ERROR_INVALID_ARGUMENT, "denoise train: features not aligned");
+    TrainParams p;
+    for (int l = 0; l < kTrainLayers; ++l) {
+        p.weights[l] = params[2 * l];
+        p.biases[l] = params[2 * l + 1];
+        if (p.weights[l] == nullptr || p.biases[l] == nullptr)
+            return record_error(SGS_ERROR_INVALID_ARGUMENT, "denoise train: null parameter");
+    }
+    unsigned char* const base = static_cast<unsigned char*>(saved);
+    auto* weights = reinterpret_cast<__nv_bfloat16*>(base + L.weights);
+    float* biases = reinterpret_cast<float*>(base + L.biases);
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+    train_pack_kernel<<<kPackBlocks + (L.n_px + 255) / 256, 256, 0, stream>>>(
+        p, weights, biases, static_cast<const uint4*>(features), reinterpret_cast<uint4*>(base + L.features), L.n_px);
+    cudaError_t err = cudaGetLastError();
+    ConvArgs a{};
+    a.batch = batch;
+    a.height = height;
+    a.width = width;
+    a.tiles_x = (width + kTileW - 1) / kTileW;
+    a.tiles_y = (height + kTileH - 1) / kTileH;
+    a.n_tiles = batch * a.tiles_x * a.tiles_y;
+    a.residual = static_cast<const uint4*>(features);
+    for (int l = 0; l < kTrainLayers && err == cudaSuccess; ++l) {
+        a.in = base + (l == 0 ? L.features : L.acts + (l - 1) * L.act_bytes);
+        a.out = l == kTrainLayers - 1 ? static_cast<void*>(output) : base + L.acts + l * L.act_bytes;
+        a.weights = reinterpret_cast<const uint4*>(weights + packed_before(l));
+        a.bias = biases + bias_before(l);
+        // the features' channels 8..15 lie outside the tensor and read zeros
+        err = l == 0                  ? launch_conv_tma<16, 32, kEpiRelu>(a, stream, 8)
+              : l < kTrainLayers - 1 ? launch_conv_tma<32, 32, kEpiRelu>(a, stream)
+                                      : launch_conv_tma<32, 16, kEpiFinal>(a, stream);
+    }
+    if (err != cudaSuccess) return record_error(SGS_ERROR_CUDA, "denoise train forward: %s", cudaGetErrorString(err));
+    return SGS_OK;
+}
+
+int sgs_denoise_train_backward(const float* grad_output, int32_t batch, int32_t height, int32_t width,
+                               const float* const* weights, const void* saved, void* scratch, size_t scratch_bytes,
+                               float* grads, void* stream_ptr) {
+    if (int st = check_shape(batch, height, width)) return st;
+    if (grad_output == nullptr || weights == nullptr || saved == nullptr || scratch == nullptr || grads == nullptr)
+        return record_error(SGS_ERROR_INVALID_ARGUMENT, "denoise train: all arrays are required");
+    const TrainLayout L = train_layout(batch, height, width);
+    if (scratch_bytes < L.scratch || !aligned16(scratch) || !aligned16(saved))
+        return record_error(SGS_ERROR_WORKSPACE, "denoise train: scratch needs %zu bytes, 16-byte aligned", L.scratch);
+    TrainParams p{};
+    for (int l = 0; l < kTrainLayers; ++l) {
+        p.weights[l] = weights[l];
+        if (p.weights[l] == nullptr) return record_error(SGS_ERROR_INVALID_ARGUMENT, "denoise train: null weights");
+    }
+    const unsigned char* const kept = static_cast<const unsigned char*>(saved);
+    unsigned char* const work = static_cast<unsigned char*>(scratch);
+    auto* dgrad = reinterpret_cast<__nv_bfloat16*>(work + L.dgrad);
+    float* sums = reinterpret_cast<float*>(work + L.sums);
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+    cudaError_t err = cudaMemsetAsync(sums, 0, (kSums + kBiases) * sizeof(float), stream);
+    if (err == cudaSuccess) {
+        train_stage_kernel<<<kDgradBlocks + (L.n_px + 255) / 256, 256, 0, stream>>>(
+            p, dgrad, grad_output, reinterpret_cast<uint4*>(work + L.grad16), L.n_px);
+        err = cudaGetLastError();
+    }
+    const int tiles_x = (width + kTileW - 1) / kTileW, tiles_y = (height + kTileH - 1) / kTileH;
+    const void* gz = work + L.grad16;
+    for (int l = kTrainLayers - 1; l >= 0 && err == cudaSuccess; --l) {
+        const unsigned char* in = kept + (l == 0 ? L.features : L.acts + (l - 1) * L.act_bytes);
+        const WgradArgs w{in, static_cast<const uint4*>(gz), sums + sums_before(l), sums + kSums + bias_before(l),
+                          batch, height, width, tiles_x, tiles_y, batch * tiles_x * tiles_y};
+        err = l == 0                  ? launch_wgrad_tma<8, 32>(w, stream)
+              : l < kTrainLayers - 1 ? launch_wgrad_tma<32, 32>(w, stream)
+                                      : launch_wgrad_tma<32, 16>(w, stream);
+        if (l == 0 || err != cudaSuccess) break;
+        void* const out = work + L.grad32 + (l & 1) * L.act_bytes;
+        ConvArgs a{gz, out, reinterpret_cast<const uint4*>(dgrad + packed_before(l) - packed_before(1)), nullptr,
+                   reinterpret_cast<const uint4*>(in), nullptr, batch, height, width, tiles_x, tiles_y, w.n_tiles};
+        err = l < kTrainLayers - 1 ? launch_conv_tma<32, 32, kEpiMask>(a, stream)
+                                    : launch_conv_tma<16, 32, kEpiMask>(a, stream);
+        gz = out;
+    }
+    if (err == cudaSuccess) {
+        train_unpack_kernel<<<(kParams + 255) / 256, 256, 0, stream>>>(sums, grads);
+        err = cudaGetLastError();
+    }
+    if (err != cudaSuccess) return record_error(SGS_ERROR_CUDA, "denoise train backward: %s", cudaGetErrorString(err));
     return SGS_OK;
 }
 
