@@ -195,7 +195,7 @@ __device__ __forceinline__ void store_pixel(const ConvArgs& a, const TileXY& til
     }
 }
 
-template <int CIN, int COUT, int IN, int EPI, bool kPlanar = false>
+template <int CIN, int COUT, int IN, int EPI>
 __global__ void __launch_bounds__(kThreads, 1) conv3x3_kernel(const ConvArgs a) {
     constexpr int KC = CIN / 8;
     constexpr int kWeightVecs = 9 * KC * COUT;
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_kernel(const ConvArgs a) 
         float acc[COUT];
         load_accumulator<COUT>(tmem + (static_cast<uint32_t>(warp * 32) << 16), acc);
 
-        if (ok) store_pixel<COUT, EPI, kPlanar>(a, tile, tid, acc, bias);
+        if (ok) store_pixel<COUT, EPI>(a, tile, tid, acc, bias);
         tc::fence_before_sync();
         if (__syncthreads_or(!ok)) {
             failed = true;
@@ -299,11 +299,11 @@ struct TmaConv {
     static_assert((kChunkPx * 16) % 128 == 0 && (kWeightVecs * 16) % 128 == 0, "128-byte TMA destinations");
 };
 
-// kPlanar: input and BF16 output in the 8-channel-plane layout of store_pixel (the tensor map is then
+// kPlanarIn, kPlanar: input, BF16 output in the 8-channel-plane layout of store_pixel (the input's tensor map is then
 // over [batch][plane][y][x * 8 + channel] and a chunk's halo is one box of 10 x 18 pixels).
 // Held to 4 CTAs per SM (80 registers, no spills): 0.357 against 0.365 ms per 1080p denoiser call at
 // the 3 that 90 registers allow.
-template <int CIN, int COUT, int EPI, bool kPlanar = false>
+template <int CIN, int COUT, int EPI, bool kPlanarIn, bool kPlanar>
 __global__ void __launch_bounds__(kTmaThreads, 4) conv3x3_tma_kernel(const __grid_constant__ CUtensorMap in_map,
                                                                   const ConvArgs a) {
     using S = TmaConv<CIN, COUT>;
@@ -338,6 +338,9 @@ __global__ void __launch_bounds__(kTmaThreads, 4) conv3x3_tma_kernel(const __gri
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    // everything above reads only the weights, which are older than the kernel before
+    tc::wait_dependencies();
+    tc::launch_dependents();
     const uint32_t tmem = *slot;
     const uint32_t halo_a = tc::smem_u32(halo);
     const uint32_t w_a = tc::smem_u32(w_s);
@@ -358,7 +361,7 @@ __global__ void __launch_bounds__(kTmaThreads, 4) conv3x3_tma_kernel(const __gri
 #pragma unroll
                 for (int c = 0; c < S::KC; ++c) {
                     const uint32_t dst = halo_a + (st * S::kHaloVecs + c * S::kChunkPx) * 16;
-                    if constexpr (kPlanar)  // x in elements: 8 per pixel, so always a 16-byte multiple
+                    if constexpr (kPlanarIn)  // x in elements: 8 per pixel, so always a 16-byte multiple
                         tc::tma_load_4d(dst, &in_map, SGS_FULL(st), (tile.x0 - 1) * 8, tile.y0 - 1, c, tile.b);
                     else
                         tc::tma_load_4d(dst, &in_map, SGS_FULL(st), c * 8, tile.x0 - 1, tile.y0 - 1, tile.b);
@@ -704,6 +707,14 @@ __global__ void __launch_bounds__(kTmaThreads) conv3x3_wgrad_tma_kernel(const __
 #undef SGS_EMPTY
 }
 
+// FP16 features as BF16, so that the first layer's halo comes by TMA like the others' (64 to 41 us for both
+// kernels per 1080p frame).
+__global__ void __launch_bounds__(256) features_bf16_kernel(const uint4* __restrict__ features,
+                                                            uint4* __restrict__ out, const uint32_t n_px) {
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i < n_px) out[i] = half8_to_bf16x8(__ldg(features + i));
+}
+
 // ---- training step: packing, staging, unpacking ------------------------------------------------
 
 constexpr int kTrainLayers = SGS_DENOISE_LAYERS;
@@ -884,10 +895,10 @@ int resident_ctas(Kernel kernel, size_t smem, int cap, int threads = kThreads) {
     return blocks < cap ? blocks : cap;
 }
 
-template <int CIN, int COUT, int IN, int EPI, bool kPlanar = false>
+template <int CIN, int COUT, int IN, int EPI>
 cudaError_t launch_conv(const ConvArgs& a, cudaStream_t stream) {
     constexpr size_t smem = static_cast<size_t>(9 * (CIN / 8) * COUT + (CIN / 8) * kHaloPx) * 16 + 16;
-    auto kernel = conv3x3_kernel<CIN, COUT, IN, EPI, kPlanar>;
+    auto kernel = conv3x3_kernel<CIN, COUT, IN, EPI>;
     static const int per_sm = resident_ctas(kernel, smem, 8);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
     const int grid = a.n_tiles < sm_count() * per_sm ? a.n_tiles : sm_count() * per_sm;
@@ -943,20 +954,32 @@ bool planar_halo_map(CUtensorMap* map, const void* base, int batch, int height, 
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// in_channels: the tensor's channels where fewer than CIN (the others read zeros).
-template <int CIN, int COUT, int EPI, bool kPlanar = false>
-cudaError_t launch_conv_tma(const ConvArgs& a, cudaStream_t stream, int in_channels = CIN) {
+// in_channels: the tensor's channels where fewer than CIN (the others read zeros). overlap: the launch
+// before in the stream does not write this one's weights and has waited for all before it, so this one's
+// start (weights, barriers, tensor memory) may overlap its end (programmatic dependent launch: 359 to
+// 345 us per 1080p denoiser call).
+template <int CIN, int COUT, int EPI, bool kPlanarIn = false, bool kPlanar = kPlanarIn>
+cudaError_t launch_conv_tma(const ConvArgs& a, cudaStream_t stream, int in_channels = CIN, bool overlap = false) {
     using S = TmaConv<CIN, COUT>;
-    auto kernel = conv3x3_tma_kernel<CIN, COUT, EPI, kPlanar>;
+    auto kernel = conv3x3_tma_kernel<CIN, COUT, EPI, kPlanarIn, kPlanar>;
     static const int per_sm = resident_ctas(kernel, S::kSmem, 512 / kTmaCols, kTmaThreads);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
     CUtensorMap map;
-    const bool mapped = kPlanar ? planar_halo_map(&map, a.in, a.batch, a.height, a.width, CIN)
+    const bool mapped = kPlanarIn ? planar_halo_map(&map, a.in, a.batch, a.height, a.width, CIN)
                                 : nhwc_map(&map, a.in, a.batch, a.height, a.width, in_channels, kHaloW, kHaloH);
     if (!mapped) return cudaErrorInvalidValue;
     const int grid = a.n_tiles < sm_count() * per_sm ? a.n_tiles : sm_count() * per_sm;
-    kernel<<<grid, kTmaThreads, S::kSmem, stream>>>(map, a);
-    return cudaGetLastError();
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(kTmaThreads);
+    config.dynamicSmemBytes = S::kSmem;
+    config.stream = stream;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, map, a);
 }
 
 template <int CIN, int COUT, int IN>
@@ -1169,19 +1192,25 @@ int sgs_denoise(const void* features, int32_t batch, int32_t height, int32_t wid
     const float* b = biases;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     const int tiles_x = (width + kTileW - 1) / kTileW, tiles_y = (height + kTileH - 1) / kTileH;
+    // the features as BF16 lie in the buffer that the second layer writes
+    const uint32_t n_px = static_cast<uint32_t>(static_cast<size_t>(batch) * height * width);
+    features_bf16_kernel<<<(n_px + 255) / 256, 256, 0, stream>>>(static_cast<const uint4*>(features),
+                                                                 reinterpret_cast<uint4*>(act[1]), n_px);
+    if (const cudaError_t err = cudaGetLastError(); err != cudaSuccess)
+        return record_error(SGS_ERROR_CUDA, "denoise features: %s", cudaGetErrorString(err));
     for (int l = 0; l < kLayers; ++l) {
         const bool last = l == kLayers - 1;
-        ConvArgs a{l == 0 ? features : act[(l + 1) & 1], last ? static_cast<void*>(output) : act[l & 1],
+        ConvArgs a{act[(l + 1) & 1], last ? static_cast<void*>(output) : act[l & 1],
                    reinterpret_cast<const uint4*>(w), b, nullptr,
                    last ? static_cast<const uint4*>(features) : nullptr, batch, height, width, tiles_x, tiles_y, 0};
         a.n_tiles = batch * tiles_x * tiles_y;
         cudaError_t err;
-        if (l == 0)
-            err = launch_conv<16, 32, kInFeatures, kEpiRelu, true>(a, stream);
+        if (l == 0)  // the features' channels 8..15 lie outside the tensor and read zeros
+            err = launch_conv_tma<16, 32, kEpiRelu, false, true>(a, stream, 8, true);
         else if (!last)
-            err = launch_conv_tma<32, 32, kEpiRelu, true>(a, stream);
+            err = launch_conv_tma<32, 32, kEpiRelu, true>(a, stream, 32, true);
         else
-            err = launch_conv_tma<32, 16, kEpiFinal, true>(a, stream);
+            err = launch_conv_tma<32, 16, kEpiFinal, true>(a, stream, 32, true);
         if (err != cudaSuccess) return record_error(SGS_ERROR_CUDA, "denoise layer %d: %s", l + 1, cudaGetErrorString(err));
         w += weights_bytes(kLayerIn[l], kLayerOut[l]);
         b += kLayerOut[l];
@@ -1241,8 +1270,8 @@ int sgs_denoise_train_forward(const void* features, int32_t batch, int32_t heigh
         a.bias = biases + bias_before(l);
         // the features' channels 8..15 lie outside the tensor and read zeros
         err = l == 0                  ? launch_conv_tma<16, 32, kEpiRelu>(a, stream, 8)
-              : l < kTrainLayers - 1 ? launch_conv_tma<32, 32, kEpiRelu>(a, stream)
-                                      : launch_conv_tma<32, 16, kEpiFinal>(a, stream);
+              : l < kTrainLayers - 1 ? launch_conv_tma<32, 32, kEpiRelu>(a, stream, 32, true)
+                                      : launch_conv_tma<32, 16, kEpiFinal>(a, stream, 32, true);
     }
     if (err != cudaSuccess) return record_error(SGS_ERROR_CUDA, "denoise train forward: %s", cudaGetErrorString(err));
     return SGS_OK;

@@ -131,6 +131,12 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tensor_map
       : "memory");
 }
 
+// Programmatic dependent launch: waits until the kernels this launch depends on have completed (returns at
+// once when it was launched without the attribute), and lets the launch that depends on this one begin
+// as CTAs leave.
+__device__ __forceinline__ void wait_dependencies() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Bounded wait for the phase with the given parity to complete; false when the limit ran out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
   for (uint32_t i = 0; i < limit; ++i)
