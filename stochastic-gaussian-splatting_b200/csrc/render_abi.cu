@@ -68,7 +68,25 @@ struct Derived {
     bool st_queue;            // the queue is stochastic transparency's
     uint32_t st_wanted;       // ST entries the queue would hold with room for all
     uint32_t tiles_x, tiles_y;
+    uint32_t n;               // Gaussians
 };
+
+// Whether a scatter pass may run front to back (sgs_front.cuh), and the coverage by all Gaussians above which it
+// does, which the clear pass estimates. The order costs the clear pass some 4 us, and a pass prepared for it that
+// then takes the Gaussians as they lie 1 to 2 % (Gaussian point splatting 5 %, as it has less to do per Gaussian), so
+// that few Gaussians, or few per pixel, are not prepared for it; below some 2.5M most of them are in flight before
+// the first bounds exist. As they lie against front to back, in us, the 6M scene cut to n Gaussians:
+//   one sample: 2.2M 1920x1080 (coverage 49) 264, 287, 1280x720 (55) 200, 196; 3M 1920x1080 (66) 330, 324,
+//     3840x2160 (44) 695, 737, 1280x720 (75) 253, 222; 6M 1920x1080 (133) 577, 415, 3840x2160 (87) 1187, 1000
+//   one sample of point splatting: 4M 1920x1080 (88) 239, 258, 1280x720 (100) 185, 183; 6M 3840x2160 (87) 615, 638,
+//     1920x1080 (133) 323, 305, 1280x720 (150) 255, 223
+//   8 samples: 2.2M 1280x720 738, 666; 6M 1920x1080 2402, 1569; of point splatting 628, 611 and 1860, 1386
+constexpr float kFrontCoverage = 58.0f, kFrontCoverageGps = 110.0f;
+
+bool may_run_front_to_back(const Derived& d, const bool gps, const uint32_t n_samples) {
+    if (n_samples > 1) return d.n >= 1u << 21 && 2ull * d.n >= d.n_fb;
+    return gps ? d.n >= 1u << 22 && 2ull * d.n >= 5ull * d.n_fb : d.n >= 5u << 19 && 2ull * d.n >= d.n_fb;
+}
 
 // Validates the arguments that determine sizes; fills the derived sizes.
 int derive(const sgs_gaussians* g, const sgs_camera* c, const sgs_settings* s, Derived& d) {
@@ -86,6 +104,7 @@ int derive(const sgs_gaussians* g, const sgs_camera* c, const sgs_settings* s, D
     d.max_binned = 0;
     d.st_queue = false;
     d.st_wanted = 0;
+    d.n = g->n_gaussians;
     // tiles per row padded to whole quads
     d.tiles_x = static_cast<uint32_t>((fbw + 4 * kBoundTile - 1) / (4 * kBoundTile)) * 4;
     d.tiles_y = static_cast<uint32_t>((fbh + kBoundTile - 1) / kBoundTile);
@@ -124,7 +143,11 @@ struct FullLayout {
     // lie in a section of their own where it is too small
     size_t tile_bound, histogram, list, st_b;
     uint32_t st_own, st_capacity, st_items;
+    size_t group_order;  // the front-to-back scatter pass's; 0: none
 };
+
+uint32_t scatter_groups(const uint32_t n) { return n / 32u + (n % 32u != 0 ? 1u : 0u); }
+
 
 FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n_samples = 1) {
     FullLayout F{};
@@ -143,11 +166,17 @@ FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n
         // 60 bytes for each of min(N, 2^18) entries in any case; more where the workspace stays within the
         // scratch of the allocation-free render (several samples per call never run there)
         const size_t bounds = align_up((static_cast<size_t>(d.tiles_x) * d.tiles_y + bound_blocks(d)) * sizeof(uint32_t));
-        const size_t fixed = bounds + align_up(2 * kDepthBuckets * sizeof(uint32_t));
+        size_t fixed = bounds + align_up(2 * kDepthBuckets * sizeof(uint32_t));
         constexpr size_t kListBytes = kItemsPerEntry * sizeof(uint32_t);
         const size_t room = d.n_fb * sizeof(float4);
         size_t own = std::max<size_t>(std::min(d.st_wanted, kStQueueCapacity) * size_t(60) / kStEntryBytes, 1);
         const bool borrow = fixed + align_up(own * kListBytes) <= room;
+        // the front-to-back pass's order, where the section has room for it too
+        const size_t groups = align_up(scatter_groups(d.n) * sizeof(uint32_t));
+        if (may_run_front_to_back(d, false, n_samples) && fixed + groups + align_up(own * kListBytes) <= room) {
+            F.group_order = L.samples + fixed;
+            fixed += groups;
+        }
         if (borrow) {
             const size_t listed = (room - fixed) / kListBytes - kAlign / kListBytes;
             const size_t spare =
@@ -176,17 +205,28 @@ FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n
         L.total = off;
         return F;
     }
+    // GPS front to back: tile bounds, depth histogram (cleared with them) and order borrow the samples section.
+    // Where the queue cannot hold all Gaussians, the binned ones are those that come first, as they lie.
+    const bool front = s->use_gps && may_run_front_to_back(d, true, s->hybrid_scheduling ? 1 : n_samples) &&
+                       (!s->hybrid_scheduling || d.max_binned >= d.n);
     // hybrid GPS: tile bounds, depth histogram and item list borrow the samples section; a short queue, or
     // one whose items turn out not to fit the list, is taken as it came
-    if (d.queue_capacity >= kMinOrdered && d.queue_capacity <= kItemEntryMask + 1u) {
+    const bool listed = d.queue_capacity >= kMinOrdered && d.queue_capacity <= kItemEntryMask + 1u;
+    if (front || listed) {
         const size_t bounds = align_up((static_cast<size_t>(d.tiles_x) * d.tiles_y + bound_blocks(d)) * sizeof(uint32_t));
-        const size_t fixed = bounds + align_up(2 * kDepthBuckets * sizeof(uint32_t));
+        size_t fixed = bounds + align_up(2 * kDepthBuckets * sizeof(uint32_t));
         const size_t room = d.n_fb * sizeof(float4);
-        if (fixed + kMinOrdered * sizeof(uint32_t) <= room) {
+        const size_t list = listed ? kMinOrdered * sizeof(uint32_t) : 0;
+        const size_t groups = align_up(scatter_groups(d.n) * sizeof(uint32_t));
+        if (front && fixed + groups + list <= room) {
+            F.group_order = L.samples + fixed;
+            fixed += groups;
+        }
+        if (fixed + list <= room && (listed || F.group_order != 0)) {
             F.tile_bound = L.samples;
             F.histogram = L.samples + bounds;
             F.list = L.samples + fixed;
-            F.st_items = static_cast<uint32_t>(std::min<size_t>((room - fixed) / sizeof(uint32_t), kMaxItems));
+            if (listed) F.st_items = static_cast<uint32_t>(std::min<size_t>((room - fixed) / sizeof(uint32_t), kMaxItems));
         }
     }
     const size_t q = d.queue_capacity;
@@ -353,8 +393,8 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
     w.q.count = reinterpret_cast<uint32_t*>(ws + F.q_count);
     w.q.capacity = d.queue_capacity;
     StQueue stq{};
-    if (F.st_items != 0) {
-        stq.list = reinterpret_cast<uint32_t*>(ws + F.list);
+    if (F.tile_bound != 0) {
+        stq.list = F.st_items != 0 ? reinterpret_cast<uint32_t*>(ws + F.list) : nullptr;
         stq.list_capacity = F.st_items;
         stq.histogram = reinterpret_cast<uint32_t*>(ws + F.histogram);
         stq.tile_bound = reinterpret_cast<uint32_t*>(ws + F.tile_bound);
@@ -382,8 +422,23 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
             stq.log_row_split = 0;
     }
 
+    GroupOrder groups{};
+    if (F.group_order != 0) {
+        groups.order = reinterpret_cast<uint32_t*>(ws + F.group_order);
+        groups.groups = scatter_groups(g->n_gaussians);
+        groups.slices = (groups.groups + kSliceGroups - 1) / kSliceGroups;
+        const uint32_t quads = d.tiles_x / 4 * d.tiles_y;
+        // One block in 24 refreshes, within 8 to 16 sweeps over the framebuffer: more of them drop more (6M at 1080p:
+        // 4 sweeps 455 us, 8 431, 16 434; at 3840x2160 1220, 1183, 1219), but each reads the framebuffer.
+        const uint32_t drawing = groups.groups / kOrderedWarps, sweep = quads / (16 * kOrderedWarps) + 1;
+        const uint32_t sweeps = std::min(std::max(drawing / (24 * sweep), 8u), 16u);
+        groups.refresh_period = 1 + std::max(drawing / (sweeps * sweep), 1u);
+        groups.min_pixels = (s->use_gps && n_samples == 1 ? kFrontCoverageGps : kFrontCoverage) * static_cast<float>(d.n_fb);
+    }
+
     const PassCamera cam = pass_camera(c, s, d.ss);
     AccumulateParams ap{};
+    ap.groups = groups;
     ap.means = g->means;
     ap.scales = g->scales;
     ap.rotations = reinterpret_cast<const float4*>(g->rotations);
@@ -453,7 +508,8 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
 
     // the clear and accumulate passes of one framebuffer (or, with p.n_samples > 1, of all of them)
     auto accumulate = [&](const AccumulateParams& p, const size_t n_clear) -> int {
-        cudaError_t err = d.st_queue ? launch_clear_st(p, n_clear, sms, acc_stream)
+        cudaError_t err = d.st_queue || p.groups.order != nullptr
+                                    ? launch_clear_st(p, n_clear, sms, acc_stream)
                                     : launch_clear(p.framebuffer, n_clear, w.queue, p.stq, sms, acc_stream);
         if (err != cudaSuccess) return fail(SGS_ERROR_CUDA, "clear: %s", cudaGetErrorString(err));
         if (g->n_gaussians == 0) return SGS_OK;
@@ -497,7 +553,9 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
         // Several GPS samples with hybrid scheduling: each frame's points are drawn by its own scatter
         // and queue passes into its own framebuffer (the work queue is reused in stream order), then one
         // resolve pass merges the n framebuffers in frame order.
-        cudaError_t err = launch_clear(w.framebuffer, d.n_fb * n_samples, w.queue, stq, sms, acc_stream);
+        cudaError_t err = ap.groups.order != nullptr
+                              ? launch_clear_st(ap, d.n_fb * n_samples, sms, acc_stream)
+                              : launch_clear(w.framebuffer, d.n_fb * n_samples, w.queue, stq, sms, acc_stream);
         if (err != cudaSuccess) return fail(SGS_ERROR_CUDA, "clear: %s", cudaGetErrorString(err));
         if (t_stage_start != nullptr) cudaEventRecord(t_stage_start, acc_stream);
         for (uint32_t sm = 0; sm < n_samples && g->n_gaussians > 0; ++sm) {

@@ -20,9 +20,11 @@ struct WorkQueue {
     unsigned int st_entries;     // ST: entries and list items reserved by producers
     unsigned int st_items;
     unsigned int st_listed;      // items the order pass has listed (GPS: or kNotListed)
-    alignas(16) float covered[4];  // ST: AABB pixels of the scene, estimated by kSampleBlocks blocks of the clear pass
+    alignas(16) float covered[4];      // AABB pixels of the scene's larger Gaussians, estimated by kSampleBlocks
+                                       // blocks of the clear pass
+    alignas(16) float covered_all[4];  // the same of all its Gaussians
 };
-static_assert(offsetof(WorkQueue, covered) % 16 == 0, "read as one float4");
+static_assert(offsetof(WorkQueue, covered) % 16 == 0 && offsetof(WorkQueue, covered_all) % 16 == 0, "read as float4");
 constexpr unsigned long long kQueueEntryShift = 40;
 constexpr unsigned long long kQueueChunkMask = (1ull << kQueueEntryShift) - 1;
 // Producers queue chunk indices below this, so the consumers' cursor (which overshoots the last chunk
@@ -66,6 +68,24 @@ struct StQueue {
     uint32_t blocks_x, n_blocks;
     uint32_t bound_pitch, tiles_y;  // tiles per row (a multiple of 4) and rows
     uint32_t height;                // framebuffer rows
+};
+
+// Scatter passes in depth order: groups of 32 consecutive Gaussians (neighbours in a Morton-ordered model), sorted
+// by the depth of their middle one. The clear pass sorts every `slices`-th group in one block; as each of these
+// slices is an even sample of the scene, the r-th groups of all of them lie at nearly the same depth, and the
+// order takes these together, so that no sum over the blocks is needed.
+constexpr uint32_t kSliceGroups = 1024;  // groups per slice, at most
+constexpr uint32_t kGroupBuckets = 1024;  // 1/64 octave each over view depths of 2^-4 .. 2^12
+constexpr int kGroupShift = 17;           // depth bits below a bucket's
+// Warps per block of a front-to-back pass: many of its warps end early, and a block keeps its place until its last
+// warp has ended (8 warps a block: 478 us where 2 take 437 on 6M Gaussians at 1080p; fewer make more blocks to start).
+constexpr uint32_t kOrderedWarps = 4;
+struct GroupOrder {
+    uint32_t* order;          // groups front to back; null: the pass takes them as they come
+    uint32_t groups;
+    uint32_t slices;
+    uint32_t refresh_period;  // every refresh_period-th block of the pass lowers tile bounds
+    float min_pixels;         // covered pixels above which the pass runs in depth order
 };
 
 // Depth bucket of a key's high word; depths off the range share the end buckets (the order only
@@ -159,6 +179,7 @@ struct AccumulateParams {
     WorkQueue* queue;
     QueueArrays q;
     StQueue stq;
+    GroupOrder groups;
     uint32_t n_samples;               // samples of one call (frames frame .. frame + n_samples - 1)
     size_t fb_stride;                 // framebuffer elements between consecutive samples' framebuffers
     const float4* pre;                // preactivated layout (2 float4 per Gaussian) or null
