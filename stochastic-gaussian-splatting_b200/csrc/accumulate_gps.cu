@@ -162,6 +162,7 @@ __device__ __forceinline__ void evaluate_parked(const AccumulateParams& a, unsig
 template <bool kHybrid, bool kMulti, bool kFront>
 __device__ __forceinline__ void gps_scatter(const AccumulateParams& a) {
     static_assert(!(kHybrid && kMulti), "several samples per call use scatter scheduling");
+    wait_for_pass_before();
     constexpr uint32_t kWarps = kFront ? kOrderedWarps : kBlock / 32;
     __shared__ uint2 s_state[kWarps][kItemsPerWarp];
     __shared__ uint8_t s_src[kWarps][kItemsPerWarp];
@@ -389,6 +390,7 @@ __device__ __forceinline__ void consume_chunks(const AccumulateParams& a) {
 }
 
 __global__ void __launch_bounds__(kBlock, kChunkBlocksPerSM) gps_chunks_kernel(const AccumulateParams a) {
+    wait_for_pass_before();
     consume_chunks(a);
 }
 
@@ -465,6 +467,7 @@ __device__ __forceinline__ bool occluded(const AccumulateParams& a, const GpsIte
 // reach, for keys only decrease during a pass.
 __global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) gps_queue_kernel(const AccumulateParams a) {
     __shared__ GpsItem s_item[kBlock / 32][kMaxClaim];
+    wait_for_pass_before();
     if (a.queue->st_listed == kNotListed) {
         consume_chunks(a);
         return;
@@ -539,22 +542,26 @@ __global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) gps_queue_kernel(co
 cudaError_t launch_accumulate_gps(const AccumulateParams& p, const int num_sms, cudaStream_t stream) {
     if (p.n == 0) return cudaSuccess;
     const unsigned grid = (p.n + kBlock - 1) / kBlock;
+    constexpr unsigned kFrontThreads = kOrderedWarps * 32u;
+    cudaError_t err;
     if (p.groups.order != nullptr) {  // sgs_front.cuh
         const unsigned blocks = ordered_blocks(p.groups);
-        if (p.hybrid) gps_front_kernel<true, false><<<blocks, kOrderedWarps * 32u, 0, stream>>>(p);
-        else if (p.n_samples > 1) gps_front_kernel<false, true><<<blocks, kOrderedWarps * 32u, 0, stream>>>(p);
-        else gps_front_kernel<false, false><<<blocks, kOrderedWarps * 32u, 0, stream>>>(p);
-    } else if (p.hybrid) gps_scatter_hybrid_kernel<<<grid, kBlock, 0, stream>>>(p);
-    else if (p.n_samples > 1) gps_scatter_kernel<true><<<grid, kBlock, 0, stream>>>(p);
-    else gps_scatter_kernel<false><<<grid, kBlock, 0, stream>>>(p);
-    if (p.hybrid && p.stq.list != nullptr) {
-        const cudaError_t err = launch_order_gps(p, num_sms, stream);
-        if (err != cudaSuccess) return err;
-        gps_queue_kernel<<<static_cast<unsigned>(num_sms) * kQueueBlocksPerSM, kBlock, 0, stream>>>(p);
+        if (p.hybrid) err = launch_pass(gps_front_kernel<true, false>, blocks, kFrontThreads, p, stream);
+        else if (p.n_samples > 1) err = launch_pass(gps_front_kernel<false, true>, blocks, kFrontThreads, p, stream);
+        else err = launch_pass(gps_front_kernel<false, false>, blocks, kFrontThreads, p, stream);
     } else if (p.hybrid) {
-        gps_chunks_kernel<<<static_cast<unsigned>(num_sms) * kChunkBlocksPerSM, kBlock, 0, stream>>>(p);
+        err = launch_pass(gps_scatter_hybrid_kernel, grid, kBlock, p, stream);
+    } else if (p.n_samples > 1) {
+        err = launch_pass(gps_scatter_kernel<true>, grid, kBlock, p, stream);
+    } else {
+        err = launch_pass(gps_scatter_kernel<false>, grid, kBlock, p, stream);
     }
-    return cudaGetLastError();
+    if (err != cudaSuccess || !p.hybrid) return err;
+    if (p.stq.list == nullptr)
+        return launch_pass(gps_chunks_kernel, static_cast<unsigned>(num_sms) * kChunkBlocksPerSM, kBlock, p, stream);
+    err = launch_order_gps(p, num_sms, stream);
+    if (err != cudaSuccess) return err;
+    return launch_pass(gps_queue_kernel, static_cast<unsigned>(num_sms) * kQueueBlocksPerSM, kBlock, p, stream);
 }
 
 }  // namespace sgs

@@ -444,6 +444,7 @@ st_scatter_kernel(const AccumulateParams a) {
     const uint32_t upto_mask = kFullMask >> (31u - lane);
     // kSplit (small scenes): 2^log_row_split warps share 32 Gaussians, each walking every 2^log_row_split-th
     // batch of their rows (all project them; the first one queues the large ones)
+    wait_for_pass_before();
     constexpr bool kSplit = kMode == kSplitRows;
     uint32_t block = blockIdx.x;
     bool ordered = false;
@@ -615,6 +616,7 @@ __global__ void __launch_bounds__(kOrderBlock) order_kernel(const AccumulatePara
     constexpr uint32_t kPerThread = kDepthBuckets / kOrderBlock;
     __shared__ uint32_t s_first[kDepthBuckets], s_count[kDepthBuckets];
     __shared__ uint32_t s_warp[kOrderBlock / 32];
+    wait_for_pass_before();
     if (!kGps && !dense_scene(a)) return;  // the producers have listed the items as they came
     const uint32_t n = kGps ? static_cast<uint32_t>(min(a.queue->packed >> kQueueEntryShift,
                                                         static_cast<unsigned long long>(min(a.max_binned, a.q.capacity))))
@@ -689,6 +691,7 @@ __global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) st_queue_kernel(con
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
     const uint32_t upto_mask = kFullMask >> (31u - lane);
+    wait_for_pass_before();
     const bool dense = dense_scene(a);
     const uint32_t n_items = dense ? a.queue->st_listed : min(a.queue->st_items, a.stq.list_capacity);
     if (n_items == 0) return;
@@ -869,6 +872,12 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
         const uint32_t step = max(a.n / (kSampleBlocks * kBlock), 1u);
         bool active = t < a.n;
         const uint32_t g = active ? t * step : a.n - 1u;
+        // the projection loads the mean first and the rest after it; here their latency is all there is
+        if (a.quant.records == nullptr && a.pre == nullptr) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(a.scales + 3 * g));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(a.rotations + g));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(a.opacities + g));
+        }
         Projected p;
         float pixels = 0.0f, larger = 0.0f;
         if (project_gaussian(active, g, a.means, a.scales, a.rotations, a.opacities, a.w2c, a.cam, p, a.pre, a.quant) &&
@@ -906,28 +915,30 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
 }
 
 template <bool kBlue, bool kHybrid, bool kMulti>
-void launch_st(const AccumulateParams& p, const unsigned grid, const int num_sms, cudaStream_t stream) {
-    if (p.groups.order != nullptr) {
-        st_scatter_kernel<kBlue, kHybrid, kMulti, kFrontToBack>
-            <<<ordered_blocks(p.groups), kOrderedWarps * 32u, 0, stream>>>(p);
-    } else if (p.stq.log_row_split != 0) {
-        st_scatter_kernel<kBlue, kHybrid, kMulti, kSplitRows><<<grid, kBlock, 0, stream>>>(p);
-    } else {
-        st_scatter_kernel<kBlue, kHybrid, kMulti, kPlain><<<grid, kBlock, 0, stream>>>(p);
-    }
-    if (!isinf(p.stq.dense_pixels))
-        order_kernel<false><<<static_cast<unsigned>(num_sms), kOrderBlock, 0, stream>>>(p);
-    st_queue_kernel<kBlue, kHybrid, kMulti>
-        <<<static_cast<unsigned>(num_sms) * kQueueBlocksPerSM, kBlock, 0, stream>>>(p);
+cudaError_t launch_st(const AccumulateParams& p, const unsigned grid, const int num_sms, cudaStream_t stream) {
+    cudaError_t err;
+    if (p.groups.order != nullptr)
+        err = launch_pass(st_scatter_kernel<kBlue, kHybrid, kMulti, kFrontToBack>, ordered_blocks(p.groups),
+                          kOrderedWarps * 32u, p, stream);
+    else if (p.stq.log_row_split != 0)
+        err = launch_pass(st_scatter_kernel<kBlue, kHybrid, kMulti, kSplitRows>, grid, kBlock, p, stream);
+    else
+        err = launch_pass(st_scatter_kernel<kBlue, kHybrid, kMulti, kPlain>, grid, kBlock, p, stream);
+    if (err == cudaSuccess && !isinf(p.stq.dense_pixels))
+        err = launch_pass(order_kernel<false>, static_cast<unsigned>(num_sms), kOrderBlock, p, stream);
+    if (err == cudaSuccess)
+        err = launch_pass(st_queue_kernel<kBlue, kHybrid, kMulti>, static_cast<unsigned>(num_sms) * kQueueBlocksPerSM,
+                          kBlock, p, stream);
+    return err;
 }
 
 template <bool kMulti>
-void launch_st_variant(const AccumulateParams& p, const unsigned grid, const int num_sms, cudaStream_t stream) {
+cudaError_t launch_st_variant(const AccumulateParams& p, const unsigned grid, const int num_sms, cudaStream_t stream) {
     const bool blue = p.blue_noise != nullptr;
-    if (blue && p.hybrid) launch_st<true, true, kMulti>(p, grid, num_sms, stream);
-    else if (blue) launch_st<true, false, kMulti>(p, grid, num_sms, stream);
-    else if (p.hybrid) launch_st<false, true, kMulti>(p, grid, num_sms, stream);
-    else launch_st<false, false, kMulti>(p, grid, num_sms, stream);
+    if (blue && p.hybrid) return launch_st<true, true, kMulti>(p, grid, num_sms, stream);
+    if (blue) return launch_st<true, false, kMulti>(p, grid, num_sms, stream);
+    if (p.hybrid) return launch_st<false, true, kMulti>(p, grid, num_sms, stream);
+    return launch_st<false, false, kMulti>(p, grid, num_sms, stream);
 }
 
 }  // namespace
@@ -948,8 +959,7 @@ cudaError_t launch_clear(unsigned long long* framebuffer, const size_t n_fb, Wor
 }
 
 cudaError_t launch_order_gps(const AccumulateParams& p, const int num_sms, cudaStream_t stream) {
-    order_kernel<true><<<static_cast<unsigned>(num_sms), kOrderBlock, 0, stream>>>(p);
-    return cudaGetLastError();
+    return launch_pass(order_kernel<true>, static_cast<unsigned>(num_sms), kOrderBlock, p, stream);
 }
 
 cudaError_t launch_clear_st(const AccumulateParams& p, const size_t n_fb, const int num_sms, cudaStream_t stream) {
@@ -961,9 +971,8 @@ cudaError_t launch_clear_st(const AccumulateParams& p, const size_t n_fb, const 
 cudaError_t launch_accumulate_st(const AccumulateParams& p, const int num_sms, cudaStream_t stream) {
     if (p.n == 0) return cudaSuccess;
     const unsigned grid = (((p.n + 31u) / 32u << p.stq.log_row_split) + kWarpsPerBlock - 1u) / kWarpsPerBlock;
-    if (p.n_samples > 1) launch_st_variant<true>(p, grid, num_sms, stream);
-    else launch_st_variant<false>(p, grid, num_sms, stream);
-    return cudaGetLastError();
+    return p.n_samples > 1 ? launch_st_variant<true>(p, grid, num_sms, stream)
+                           : launch_st_variant<false>(p, grid, num_sms, stream);
 }
 
 }  // namespace sgs

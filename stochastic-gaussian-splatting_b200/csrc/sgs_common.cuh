@@ -12,6 +12,9 @@
 
 namespace sgs {
 
+// Waits for the kernel before it in the stream, where the launch lets this one begin earlier (no wait otherwise).
+__device__ __forceinline__ void wait_for_pass_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- Gaussian splatting constants (gs_utils.h:13-18) ----
 constexpr float kDilation = 0.3f;
 constexpr float kDilationProperAA = 0.1f;

@@ -209,6 +209,22 @@ __device__ __forceinline__ FrameRng frame_rng(const AccumulateParams& a) {
     return frame_rng_at(a, (a.frame_ptr != nullptr ? *a.frame_ptr : a.frame_idx) + a.frame_offset);
 }
 
+// Launch of a pass whose kernel begins with wait_for_pass_before(): its launch overlaps the end of the pass before
+// it, which it then waits for with all that pass wrote.
+inline cudaError_t launch_pass(void (*kernel)(AccumulateParams), const unsigned blocks, const unsigned threads,
+                               const AccumulateParams& p, cudaStream_t stream) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(blocks);
+    config.blockDim = dim3(threads);
+    config.stream = stream;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, p);
+}
+
 cudaError_t launch_clear(unsigned long long* framebuffer, size_t n_fb, WorkQueue* queue, const StQueue& stq,
                          int num_sms, cudaStream_t stream);
 cudaError_t launch_order_gps(const AccumulateParams& p, int num_sms, cudaStream_t stream);
