@@ -856,6 +856,7 @@ __device__ __forceinline__ void clear_bounds(const StQueue& q, const size_t tid,
 // q.tile_bound null: no tile bounds and no depth histogram.
 __global__ void clear_kernel(unsigned long long* __restrict__ fb, const size_t n_fb, WorkQueue* __restrict__ queue,
                              const StQueue q) {
+    wait_for_pass_before();
     const size_t tid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
     clear_keys(fb, n_fb, queue, tid, stride);
@@ -866,6 +867,7 @@ __global__ void clear_kernel(unsigned long long* __restrict__ fb, const size_t n
 // the first kSampleBlocks blocks, the AABB pixels of one Gaussian per thread evenly over the scene, from
 // which dense_scene tells how often the larger ones cover the framebuffer.
 __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams a, const size_t n_fb) {
+    wait_for_pass_before();
     if (blockIdx.x < kSampleBlocks) {
         __shared__ float2 s_sum[kWarpsPerBlock];
         const uint32_t t = blockIdx.x * kBlock + threadIdx.x;
@@ -954,8 +956,7 @@ unsigned clear_blocks(const size_t n_fb, const int num_sms) {
 cudaError_t launch_clear(unsigned long long* framebuffer, const size_t n_fb, WorkQueue* queue, const StQueue& stq,
                          const int num_sms, cudaStream_t stream) {
     const size_t n = n_fb + static_cast<size_t>(stq.bound_pitch) * stq.tiles_y / 2;
-    clear_kernel<<<clear_blocks(n, num_sms), kBlock, 0, stream>>>(framebuffer, n_fb, queue, stq);
-    return cudaGetLastError();
+    return launch_pass_with(0, clear_kernel, dim3(clear_blocks(n, num_sms)), kBlock, stream, framebuffer, n_fb, queue, stq);
 }
 
 cudaError_t launch_order_gps(const AccumulateParams& p, const int num_sms, cudaStream_t stream) {
@@ -964,8 +965,7 @@ cudaError_t launch_order_gps(const AccumulateParams& p, const int num_sms, cudaS
 
 cudaError_t launch_clear_st(const AccumulateParams& p, const size_t n_fb, const int num_sms, cudaStream_t stream) {
     const unsigned others = kSampleBlocks + (p.groups.order != nullptr ? p.groups.slices : 0u);
-    st_clear_kernel<<<others + clear_blocks(n_fb, num_sms), kBlock, 0, stream>>>(p, n_fb);
-    return cudaGetLastError();
+    return launch_pass_with(0, st_clear_kernel, dim3(others + clear_blocks(n_fb, num_sms)), kBlock, stream, p, n_fb);
 }
 
 cudaError_t launch_accumulate_st(const AccumulateParams& p, const int num_sms, cudaStream_t stream) {

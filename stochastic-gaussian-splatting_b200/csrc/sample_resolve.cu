@@ -101,6 +101,7 @@ __device__ __forceinline__ float4 warp_sample(const ResolveParams& a, const unsi
 // loaded only when they are used: the entry occludes this sample, or the insertion of a new
 // primitive shifts it. The pass is bound by the k-buffer traffic.
 __global__ void __launch_bounds__(kBlock) reuse_sample_kernel(const ResolveParams a) {
+    wait_for_pass_before();
     const uint32_t idx = blockIdx.x * kBlock + threadIdx.x;
     const bool active = idx < a.n_fb;
     const uint32_t pixel = active ? idx : a.n_fb - 1;
@@ -184,6 +185,7 @@ __global__ void __launch_bounds__(kBlock) reuse_sample_kernel(const ResolveParam
 // that read them from memory: Reproject without spatial reuse at supersampling factors whose tile
 // does not fit in shared memory.
 __global__ void __launch_bounds__(kBlock) plain_sample_kernel(const ResolveParams a) {
+    wait_for_pass_before();
     const uint32_t idx = blockIdx.x * kBlock + threadIdx.x;
     const bool active = idx < a.n_fb;
     const uint32_t pixel = active ? idx : a.n_fb - 1;
@@ -257,6 +259,7 @@ TileLayout tile_layout(const uint32_t ss, const bool reuse, const bool reproject
 // every read goes to global memory, for tiles too large to stage).
 template <bool kReuse, bool kFused, bool kReproject, bool kStaged>
 __global__ void __launch_bounds__(kBlock) tile_resolve_kernel(const ResolveParams a, const TileLayout L) {
+    wait_for_pass_before();
     extern __shared__ __align__(16) unsigned char smem[];
     float4* s_samples = reinterpret_cast<float4*>(smem + L.samples);
     float4* s_weights = reinterpret_cast<float4*>(smem + L.weights);
@@ -588,6 +591,7 @@ __global__ void __launch_bounds__(kBlock) tile_resolve_kernel(const ResolveParam
 // still written for inspection. The pass waits on its dependent gathers (key, then the winner's SH),
 // so it is held to 40 registers for 6 resident blocks per SM.
 __global__ void __launch_bounds__(kBlock, 6) sample_resolve_fused_kernel(const ResolveParams a) {
+    wait_for_pass_before();
     advance_frame(a);
     const uint32_t idx = blockIdx.x * kBlock + threadIdx.x;
     const bool active = idx < a.n_pixels;
@@ -652,6 +656,7 @@ __global__ void __launch_bounds__(kBlock, 6) sample_resolve_fused_kernel(const R
 // sample_resolve_fused_kernel once per sample, the history carried in registers between samples, so
 // the outputs equal those of one call per sample bit for bit.
 __global__ void __launch_bounds__(kBlock) samples_resolve_kernel(const ResolveParams a) {
+    wait_for_pass_before();
     if (a.frame_counter != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *a.frame_counter += a.n_samples;
     const uint32_t idx = blockIdx.x * kBlock + threadIdx.x;
     const bool active = idx < a.n_pixels;
@@ -734,28 +739,24 @@ cudaError_t launch_tile(const ResolveParams& p, const TileLayout& L, cudaStream_
         if (err != cudaSuccess) return err;
     }
     const dim3 grid((p.width + kTileW - 1) / kTileW, (p.height + kTileH - 1) / kTileH);
-    kernel<<<grid, kBlock, bytes, stream>>>(p, L);
-    return cudaGetLastError();
+    return launch_pass_with(bytes, kernel, grid, kBlock, stream, p, L);
 }
 
 }  // namespace
 
 cudaError_t launch_sample_resolve(const ResolveParams& p, cudaStream_t stream) {
     if (p.n_samples > 1) {
-        samples_resolve_kernel<<<(p.n_pixels + kBlock - 1) / kBlock, kBlock, 0, stream>>>(p);
-        return cudaGetLastError();
+        return launch_pass(samples_resolve_kernel, (p.n_pixels + kBlock - 1) / kBlock, kBlock, p, stream);
     }
     const bool reproject = p.temporal_mode == 2;
     if (!p.spatial_reuse && !reproject) {
-        sample_resolve_fused_kernel<<<(p.n_pixels + kBlock - 1) / kBlock, kBlock, 0, stream>>>(p);
-        return cudaGetLastError();
+        return launch_pass(sample_resolve_fused_kernel, (p.n_pixels + kBlock - 1) / kBlock, kBlock, p, stream);
     }
     const TileLayout L = tile_layout(p.ss, p.spatial_reuse, reproject);
     const bool staged = L.bytes <= kMaxTileBytes;
     const unsigned grid_sample = (p.n_fb + kBlock - 1) / kBlock;
     if (p.spatial_reuse) {
-        reuse_sample_kernel<<<grid_sample, kBlock, 0, stream>>>(p);
-        const cudaError_t err = cudaGetLastError();
+        const cudaError_t err = launch_pass(reuse_sample_kernel, grid_sample, kBlock, p, stream);
         if (err != cudaSuccess) return err;
         if (reproject) return staged ? launch_tile<true, false, true, true>(p, L, stream)
                                      : launch_tile<true, false, true, false>(p, L, stream);
@@ -764,8 +765,7 @@ cudaError_t launch_sample_resolve(const ResolveParams& p, cudaStream_t stream) {
     }
     // Reproject without spatial reuse: the winners' colours evaluated by the resolve tiles themselves
     if (staged) return launch_tile<false, true, true, true>(p, L, stream);
-    plain_sample_kernel<<<grid_sample, kBlock, 0, stream>>>(p);
-    const cudaError_t err = cudaGetLastError();
+    const cudaError_t err = launch_pass(plain_sample_kernel, grid_sample, kBlock, p, stream);
     if (err != cudaSuccess) return err;
     return launch_tile<false, false, true, false>(p, L, stream);
 }

@@ -211,18 +211,25 @@ __device__ __forceinline__ FrameRng frame_rng(const AccumulateParams& a) {
 
 // Launch of a pass whose kernel begins with wait_for_pass_before(): its launch overlaps the end of the pass before
 // it, which it then waits for with all that pass wrote.
-inline cudaError_t launch_pass(void (*kernel)(AccumulateParams), const unsigned blocks, const unsigned threads,
-                               const AccumulateParams& p, cudaStream_t stream) {
+template <typename... Params, typename... Args>
+cudaError_t launch_pass_with(const size_t shared_bytes, void (*kernel)(Params...), const dim3 blocks,
+                             const unsigned threads, cudaStream_t stream, const Args&... args) {
     cudaLaunchConfig_t config{};
-    config.gridDim = dim3(blocks);
+    config.gridDim = blocks;
     config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = shared_bytes;
     config.stream = stream;
     cudaLaunchAttribute attribute{};
     attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attribute.val.programmaticStreamSerializationAllowed = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, kernel, p);
+    return cudaLaunchKernelEx(&config, kernel, args...);
+}
+template <typename P>
+cudaError_t launch_pass(void (*kernel)(P), const unsigned blocks, const unsigned threads, const P& p,
+                        cudaStream_t stream) {
+    return launch_pass_with(0, kernel, dim3(blocks), threads, stream, p);
 }
 
 cudaError_t launch_clear(unsigned long long* framebuffer, size_t n_fb, WorkQueue* queue, const StQueue& stq,
