@@ -615,6 +615,10 @@ __global__ void __launch_bounds__(kTmaThreads) conv3x3_wgrad_tma_kernel(const __
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    // everything above touches nothing but shared memory and TMEM; the layer's data gradient, launched behind this
+    // kernel, may load its weights and set up from here on
+    tc::wait_dependencies();
+    tc::launch_dependents();
     const uint32_t tmem = *slot;
     const uint32_t smem0 = tc::smem_u32(base);
     bool failed = false;
@@ -711,6 +715,7 @@ __global__ void __launch_bounds__(kTmaThreads) conv3x3_wgrad_tma_kernel(const __
 // kernels per 1080p frame).
 __global__ void __launch_bounds__(256) features_bf16_kernel(const uint4* __restrict__ features,
                                                             uint4* __restrict__ out, const uint32_t n_px) {
+    tc::wait_dependencies();
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
     if (i < n_px) out[i] = half8_to_bf16x8(__ldg(features + i));
 }
@@ -754,6 +759,7 @@ constexpr int kPackBlocks = (kPacked + kBiases + 255) / 256;
 __global__ void __launch_bounds__(256) train_pack_kernel(const TrainParams p, __nv_bfloat16* __restrict__ weights,
                                                          float* __restrict__ biases, const uint4* __restrict__ features,
                                                          uint4* __restrict__ features_bf16, const uint32_t n_px) {
+    tc::wait_dependencies();
     if (blockIdx.x >= kPackBlocks) {
         const uint32_t i = (blockIdx.x - kPackBlocks) * 256u + threadIdx.x;
         if (i < n_px) features_bf16[i] = half8_to_bf16x8(__ldg(features + i));
@@ -779,6 +785,7 @@ constexpr int kDgradBlocks = (kPacked - packed_before(1) + 255) / 256;
 __global__ void __launch_bounds__(256) train_stage_kernel(const TrainParams p, __nv_bfloat16* __restrict__ weights,
                                                           const float* __restrict__ grad, uint4* __restrict__ staged,
                                                           const uint32_t n_px) {
+    tc::wait_dependencies();
     if (blockIdx.x >= kDgradBlocks) {
         const uint32_t i = (blockIdx.x - kDgradBlocks) * 256u + threadIdx.x;
         if (i >= n_px) return;
@@ -800,6 +807,7 @@ __global__ void __launch_bounds__(256) train_stage_kernel(const TrainParams p, _
 
 // Parameter gradients W1[co][ci][3][3], b1, ..., back to back from the sums [tap][co][ci] and bias sums.
 __global__ void __launch_bounds__(256) train_unpack_kernel(const float* __restrict__ sums, float* __restrict__ grads) {
+    tc::wait_dependencies();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= kParams) return;
     int l = 0;
@@ -1005,8 +1013,8 @@ cudaError_t launch_wgrad_tma(const WgradArgs& a, cudaStream_t stream) {
         !nhwc_map(&grad_map, a.grad_out, a.batch, a.height, a.width, COUT, kTileW, kTileH))
         return cudaErrorInvalidValue;
     const int grid = a.n_tiles < sm_count() * per_sm ? a.n_tiles : sm_count() * per_sm;
-    kernel<<<grid, kTmaThreads, G::kSmem, stream>>>(in_map, grad_map, a);
-    return cudaGetLastError();
+    // its set-up overlaps the end of the kernel before, which it waits for (and with it for all before that one)
+    return launch_pass_with(G::kSmem, kernel, dim3(grid), kTmaThreads, stream, in_map, grad_map, a);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -1194,9 +1202,10 @@ int sgs_denoise(const void* features, int32_t batch, int32_t height, int32_t wid
     const int tiles_x = (width + kTileW - 1) / kTileW, tiles_y = (height + kTileH - 1) / kTileH;
     // the features as BF16 lie in the buffer that the second layer writes
     const uint32_t n_px = static_cast<uint32_t>(static_cast<size_t>(batch) * height * width);
-    features_bf16_kernel<<<(n_px + 255) / 256, 256, 0, stream>>>(static_cast<const uint4*>(features),
-                                                                 reinterpret_cast<uint4*>(act[1]), n_px);
-    if (const cudaError_t err = cudaGetLastError(); err != cudaSuccess)
+    if (const cudaError_t err = launch_pass_with(0, features_bf16_kernel, dim3((n_px + 255) / 256), 256, stream,
+                                                 static_cast<const uint4*>(features), reinterpret_cast<uint4*>(act[1]),
+                                                 n_px);
+        err != cudaSuccess)
         return record_error(SGS_ERROR_CUDA, "denoise features: %s", cudaGetErrorString(err));
     for (int l = 0; l < kLayers; ++l) {
         const bool last = l == kLayers - 1;
@@ -1252,9 +1261,9 @@ int sgs_denoise_train_forward(const void* features, int32_t batch, int32_t heigh
     auto* weights = reinterpret_cast<__nv_bfloat16*>(base + L.weights);
     float* biases = reinterpret_cast<float*>(base + L.biases);
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-    train_pack_kernel<<<kPackBlocks + (L.n_px + 255) / 256, 256, 0, stream>>>(
-        p, weights, biases, static_cast<const uint4*>(features), reinterpret_cast<uint4*>(base + L.features), L.n_px);
-    cudaError_t err = cudaGetLastError();
+    cudaError_t err = launch_pass_with(0, train_pack_kernel, dim3(kPackBlocks + (L.n_px + 255) / 256), 256, stream, p,
+                                       weights, biases, static_cast<const uint4*>(features),
+                                       reinterpret_cast<uint4*>(base + L.features), L.n_px);
     ConvArgs a{};
     a.batch = batch;
     a.height = height;
@@ -1298,9 +1307,8 @@ int sgs_denoise_train_backward(const float* grad_output, int32_t batch, int32_t 
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     cudaError_t err = cudaMemsetAsync(sums, 0, (kSums + kBiases) * sizeof(float), stream);
     if (err == cudaSuccess) {
-        train_stage_kernel<<<kDgradBlocks + (L.n_px + 255) / 256, 256, 0, stream>>>(
-            p, dgrad, grad_output, reinterpret_cast<uint4*>(work + L.grad16), L.n_px);
-        err = cudaGetLastError();
+        err = launch_pass_with(0, train_stage_kernel, dim3(kDgradBlocks + (L.n_px + 255) / 256), 256, stream, p, dgrad,
+                               grad_output, reinterpret_cast<uint4*>(work + L.grad16), L.n_px);
     }
     const int tiles_x = (width + kTileW - 1) / kTileW, tiles_y = (height + kTileH - 1) / kTileH;
     const void* gz = work + L.grad16;
@@ -1315,13 +1323,13 @@ int sgs_denoise_train_backward(const float* grad_output, int32_t batch, int32_t 
         void* const out = work + L.grad32 + (l & 1) * L.act_bytes;
         ConvArgs a{gz, out, reinterpret_cast<const uint4*>(dgrad + packed_before(l) - packed_before(1)), nullptr,
                    reinterpret_cast<const uint4*>(in), nullptr, batch, height, width, tiles_x, tiles_y, w.n_tiles};
-        err = l < kTrainLayers - 1 ? launch_conv_tma<32, 32, kEpiMask>(a, stream)
-                                    : launch_conv_tma<16, 32, kEpiMask>(a, stream);
+        err = l < kTrainLayers - 1 ? launch_conv_tma<32, 32, kEpiMask>(a, stream, 32, true)
+                                    : launch_conv_tma<16, 32, kEpiMask>(a, stream, 16, true);
         gz = out;
     }
     if (err == cudaSuccess) {
-        train_unpack_kernel<<<(kParams + 255) / 256, 256, 0, stream>>>(sums, grads);
-        err = cudaGetLastError();
+        err = launch_pass_with(0, train_unpack_kernel, dim3((kParams + 255) / 256), 256, stream,
+                               static_cast<const float*>(sums), grads);
     }
     if (err != cudaSuccess) return record_error(SGS_ERROR_CUDA, "denoise train backward: %s", cudaGetErrorString(err));
     return SGS_OK;
