@@ -55,14 +55,14 @@ WORKLOADS = {
 }
 DEFAULT_WORKLOAD = "batch_6m_1080_st"
 
-# One `ncu --set full` capture of st_scatter_kernel on the default workload: DRAM bytes (read + write)
+# An `ncu` capture of st_scatter_kernel on the default workload: DRAM bytes (read + write)
 # and warp instructions of one launch, with the digest of the kernel sources the capture ran. When
 # those sources change, the figures no longer describe the kernel: bench then reports them as null
 # ("stale") until a new capture replaces them.
-SCATTER_SOURCES = ("accumulate_st.cu", "sgs_rows.cuh", "sgs_project.cuh", "sgs_common.cuh", "sgs_internal.h")
+SCATTER_SOURCES = ("accumulate_st.cu", "sgs_front.cuh", "sgs_rows.cuh", "sgs_project.cuh", "sgs_common.cuh", "sgs_internal.h")
 NCU_CAPTURE = {
-    "batch_6m_1080_st": {"sources_digest": "181952a8e319cca7", "dram_bytes": 278.77e6 + 15.54e6,
-                         "warp_instructions": 469.53e6},
+    "batch_6m_1080_st": {"sources_digest": "5dabccd2bb09a3e1", "dram_bytes": 211.38e6 + 10.70e6,
+                         "warp_instructions": 281.64e6},
 }
 CSRC = ROOT / "stochastic-gaussian-splatting_b200" / "csrc"
 
@@ -339,7 +339,8 @@ def run_ours(args, world, rank, local) -> dict | None:
     winners = fb[fb != -1]
     unique = int(torch.unique(winners & 0xFFFFFFFF).numel())
     alg = algorithmic_bytes(n, n_fb, n_px, unique)
-    launches_per_step = 2 + (2 if not fl["gps"] else (2 if fl["hybrid"] else 1))
+    # clear, scatter and resolve; the queue and its order pass (scenes of 8192 Gaussians and more)
+    launches_per_step = 3 + (2 if not fl["gps"] or fl["hybrid"] else 0)
 
     # end to end through the public API: each step copies the camera in from pinned host memory,
     # renders, and reads the image back into pinned host memory; the read-back runs on a second
@@ -515,7 +516,8 @@ def run_ours(args, world, rank, local) -> dict | None:
             "fragments_per_s": round(counts["fragments"] / acc_s, 0),
             "issued_per_s": round(counts["accepted"] / acc_s, 0),
             "frac_of_probe_rows": round(counts["accepted"] / acc_s / probe["rows_per_s"], 4),
-            "counts_source": f"CPU restatement, mean of {args.cpu_frames} frames; rates over the accumulate stage",
+            "counts_source": f"CPU restatement, mean of {args.cpu_frames} frames: what a pass without culling evaluates "
+                             "and issues; rates over the accumulate stage",
         })
     return line
 
