@@ -129,7 +129,7 @@ __device__ __forceinline__ Reach reach_of(const AccumulateParams& a, const uint3
     const float4 r1 = a.w2c[0], r2 = a.w2c[1], r3 = a.w2c[2];
     const PassCamera& cam = a.cam;
     const float z = dot_plus(r3, m);
-    if (z < 0.9999f * cam.near_plane) return kReachesNothing;
+    if (z < cam.near_plane - 1.0e-4f * fabsf(cam.near_plane)) return kReachesNothing;
     if (!(z > 0.0f)) return kReachUnknown;
     const float z_rcp = 1.0f / z;
     const float x = dot_plus(r1, m) * z_rcp, y = dot_plus(r2, m) * z_rcp;
