@@ -116,6 +116,11 @@ __device__ __forceinline__ bool behind_bounds(const StQueue& q, const uint32_t x
 // scale times the squared length of the axis' row of the Jacobian, the opacity at most 1, and one per cent and a
 // pixel cover the rounding. Points of Gaussian point splatting (accumulate_gps.cu) stay within the same extents
 // where the ellipse is not too thin, which the dilation grants below 900 times its variance.
+// The preactivated layout holds the covariance, whose quadratic form is the variance itself. For Gaussians that are
+// stretched along their ray it cancels, down to rounding residue that the projection, which evaluates it in
+// another order, does not share. Either evaluation is off by less than 20 roundings (2^-24) of the squared length of
+// the axis times the covariance's norm, which the sum of its entries' magnitudes bounds: kFormError of it covers both.
+constexpr float kFormError = 4.0e-6f;
 enum Reach { kReachesNothing, kReachesRect, kReachUnknown };
 struct ReachRect {
     uint32_t x0, x1, y0, y1, key_hi;
@@ -147,8 +152,10 @@ __device__ __forceinline__ Reach reach_of(const AccumulateParams& a, const uint3
             return d.x * (v0.x * d.x + 2.0f * (v0.y * d.y + v0.z * d.z)) + d.y * (v0.w * d.y + 2.0f * v1.x * d.z) +
                    v1.y * d.z * d.z;
         };
-        vx = fmaxf(along(ax), 0.0f);
-        vy = fmaxf(along(ay), 0.0f);
+        const float error = kFormError * (fabsf(v0.x) + fabsf(v0.w) + fabsf(v1.y) +
+                                          2.0f * (fabsf(v0.y) + fabsf(v0.z) + fabsf(v1.x)));
+        vx = fmaxf(along(ax), 0.0f) + error * (ax.x * ax.x + ax.y * ax.y + ax.z * ax.z);
+        vy = fmaxf(along(ay), 0.0f) + error * (ay.x * ay.x + ay.y * ay.y + ay.z * ay.z);
     } else {
         float widest;
         if (a.quant.records != nullptr)
