@@ -121,6 +121,10 @@ __device__ __forceinline__ bool behind_bounds(const StQueue& q, const uint32_t x
 // another order, does not share. Either evaluation is off by less than 20 roundings (2^-24) of the squared length of
 // the axis times the covariance's norm, which the sum of its entries' magnitudes bounds: kFormError of it covers both.
 constexpr float kFormError = 4.0e-6f;
+// A NaN among the parameters, or a quaternion whose norm overflows, gives a NaN covariance, which the projection
+// bounds by the whole framebuffer: no extents are known then (maxima would drop the NaN). The rotation is read for
+// this alone.
+constexpr float kMaxNormSq = 1.0e37f;
 enum Reach { kReachesNothing, kReachesRect, kReachUnknown };
 struct ReachRect {
     uint32_t x0, x1, y0, y1, key_hi;
@@ -131,6 +135,12 @@ __device__ __forceinline__ Reach reach_of(const AccumulateParams& a, const uint3
     const float3 m = a.quant.records != nullptr
                          ? quant_position(a.quant, g, rec.x)
                          : make_float3(a.means[3 * g], a.means[3 * g + 1], a.means[3 * g + 2]);
+    // Loaded with the mean: after the depth test the rotations cost one sample of 6M Gaussians at 1080p 1.4 %, here
+    // nothing.
+    const bool plain = a.quant.records == nullptr && a.pre == nullptr;
+    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
+    float4 q = make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+    if (plain) s0 = a.scales[3 * g], s1 = a.scales[3 * g + 1], s2 = a.scales[3 * g + 2], q = a.rotations[g];
     const float4 r1 = a.w2c[0], r2 = a.w2c[1], r3 = a.w2c[2];
     const PassCamera& cam = a.cam;
     const float z = dot_plus(r3, m);
@@ -157,11 +167,10 @@ __device__ __forceinline__ Reach reach_of(const AccumulateParams& a, const uint3
         vx = fmaxf(along(ax), 0.0f) + error * (ax.x * ax.x + ax.y * ax.y + ax.z * ax.z);
         vy = fmaxf(along(ay), 0.0f) + error * (ay.x * ay.x + ay.y * ay.y + ay.z * ay.z);
     } else {
-        float widest;
-        if (a.quant.records != nullptr)
-            widest = fmaxf(fmaxf(quant_half(rec.z), quant_half(rec.z >> 16)), quant_half(rec.w));
-        else
-            widest = fmaxf(fmaxf(a.scales[3 * g], a.scales[3 * g + 1]), a.scales[3 * g + 2]);
+        if (a.quant.records != nullptr) s0 = quant_half(rec.z), s1 = quant_half(rec.z >> 16), s2 = quant_half(rec.w);
+        const float norm_sq = q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+        const float widest = fmaxf(fmaxf(s0, s1), s2);
+        if (!(s0 <= widest && s1 <= widest && s2 <= widest && norm_sq <= kMaxNormSq)) return kReachUnknown;
         const float variance = expf(2.0f * widest);
         vx = variance * (ax.x * ax.x + ax.y * ax.y + ax.z * ax.z);
         vy = variance * (ay.x * ay.x + ay.y * ay.y + ay.z * ay.z);

@@ -2,7 +2,7 @@
 
 A curtain closes the left of the image; Gaussians behind it are dropped in groups when the tiles within their
 extents are closed (csrc/sgs_front.cuh). Here their projections reach past the curtain's edge although rough
-extents would not. With 2^21 to 5 * 2^19 Gaussians several samples per call run front to back and single
+extents would not, by cancellation or by parameters that are not finite. With 2^21 to 5 * 2^19 Gaussians several samples per call run front to back and single
 calls draw the Gaussians as they lie: both must give the same framebuffers bit for bit.
 """
 import math
@@ -96,4 +96,32 @@ def test_needles_along_their_rays_in_the_preactivated_layout(gps, cuda_device):
     together, single = framebuffers(with_curtain(g, *copies), "pre", gps, cuda_device)
     won = (single != -1) & ((single & 0xFFFFFFFF) >= N_CURTAIN)
     assert won.sum() > 100, "the needles reach past the curtain"
+    assert_bitwise("framebuffers", together, single)
+
+
+POISON = {  # (log-scale of one axis, factor on the quaternion)
+    "nan_scale": (float("nan"), 1.0),
+    "inf_scale": (float("inf"), 1.0),
+    "nan_quaternion": (-6.4, float("nan")),
+    "huge_quaternion": (-6.4, 1.0e25),
+}
+
+
+@pytest.mark.parametrize("layout,poison", [("float", "nan_scale"), ("float", "inf_scale"), ("float", "nan_quaternion"),
+                                           ("float", "huge_quaternion"), ("pre", "nan_scale"),
+                                           ("pre", "huge_quaternion"), ("quant", "nan_scale")])
+def test_parameters_that_are_not_finite(layout, poison, cuda_device):
+    """One such Gaussian among the 32 of a group: its projection is bounded by the whole image."""
+    g = torch.Generator().manual_seed(2)
+    n = 32 * 32
+    x, y = uniform(g, 32, 100.0, 300.0), uniform(g, 32, 100.0, 400.0)  # groups some ten pixels wide
+    means = at_pixel(x.repeat_interleave(32) + uniform(g, n, -8.0, 8.0),
+                     y.repeat_interleave(32) + uniform(g, n, -8.0, 8.0), torch.full((n,), 1.5))
+    scales, q = torch.full((n, 3), -6.4), torch.tensor([1.0, 0.5, -0.25, 0.125]).repeat(n, 1)
+    scales[5::32, 1], factor = POISON[poison]
+    q[5::32] *= factor
+    together, single = framebuffers(with_curtain(g, means, scales, q, torch.zeros(n)), layout, False, cuda_device)
+    if poison == "nan_scale":
+        won = (single != -1) & ((single & 0xFFFFFFFF) >= N_CURTAIN)
+        assert won.sum() > 1000, "the Gaussian is drawn beside the curtain"
     assert_bitwise("framebuffers", together, single)
