@@ -34,7 +34,6 @@ namespace {
 constexpr uint32_t kBlock = 256;
 constexpr uint32_t kFullMask = 0xffffffffu;
 constexpr uint32_t kBinningPointThreshold = 512;  // accumulate_hybrid_gps.cu:21
-constexpr uint32_t kChunkPoints = 256;             // accumulate_hybrid_gps.cu:19
 constexpr uint32_t kChunkBlocksPerSM = 8;
 constexpr uint32_t kQueueBlocksPerSM = 4;
 constexpr uint32_t kItemsPerWarp = 128;  // parked cooperative points per warp (multiple of 32)
@@ -223,7 +222,7 @@ __device__ __forceinline__ void gps_scatter(const AccumulateParams& a) {
             const bool want = act && count > kBinningPointThreshold;
             const uint32_t ballot = __ballot_sync(kFullMask, want);
             if (ballot != 0) {
-                const uint32_t chunks = want ? (count + kChunkPoints - 1) / kChunkPoints : 0u;
+                const uint32_t chunks = want ? gps_chunks(count) : 0u;
                 uint32_t incl = chunks;
 #pragma unroll
                 for (uint32_t o = 1; o < 32; o <<= 1) {
@@ -345,7 +344,7 @@ __device__ __forceinline__ void consume_chunks(const AccumulateParams& a) {
     // every chunk, so the search below never lands on one
     uint32_t last = n_entries - 1;
     if (a.q.meta[last].w == kUnusedQueueEntry) last = queue_entry_of_chunk(a.q.meta, n_entries, kUnusedQueueEntry - 1u, lane);
-    const uint32_t n_chunks = a.q.meta[last].w + (a.q.count[last] + kChunkPoints - 1) / kChunkPoints;
+    const uint32_t n_chunks = a.q.meta[last].w + gps_chunks(a.q.count[last]);
     const uint32_t frame = frame_rng(a).frame;
     for (;;) {
         uint32_t c0 = 0;
@@ -374,7 +373,7 @@ __device__ __forceinline__ void consume_chunks(const AccumulateParams& a) {
                 s.conic = make_float3(__uint_as_float(m.x), __uint_as_float(m.y), __uint_as_float(m.z));
                 n_points = a.q.count[lo];
                 entry_first = m.w;
-                entry_end = m.w + (n_points + kChunkPoints - 1) / kChunkPoints;
+                entry_end = m.w + gps_chunks(n_points);
                 base_seed = gps_seed(static_cast<uint32_t>(s.key), frame);
             }
             const uint32_t first_point = (c - entry_first) * kChunkPoints;
@@ -399,7 +398,7 @@ struct GpsItem {
     float4 geom, geom2;  // as in the queue arrays
     uint4 meta;
     unsigned long long key;
-    uint32_t first, end;  // points of the item
+    GpsItemPoints points;
 };
 
 // Whether every pixel the Gaussian can reach is nearer than it. Its points register only in pixels whose
@@ -493,9 +492,7 @@ __global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) gps_queue_kernel(co
             G.geom2 = a.q.geom2[e];
             G.meta = a.q.meta[e];
             G.key = a.q.key[e];
-            const uint32_t points = gps_parts(count).points;
-            G.first = (item >> kItemEntryBits) * points;
-            G.end = min(G.first + points, count);
+            G.points = gps_item_points(count, item >> kItemEntryBits);
             s_item[warp][lane] = G;
         }
         __syncwarp();
@@ -512,14 +509,14 @@ __global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) gps_queue_kernel(co
             s.conic = make_float3(__uint_as_float(G.meta.x), __uint_as_float(G.meta.y), __uint_as_float(G.meta.z));
             const uint2 base_seed = gps_seed(static_cast<uint32_t>(s.key), frame);
             // a group's pixels first, then their keys, read together, then the atomics the keys leave
-            for (uint32_t point = G.first + lane; point < G.end; point += 32u * kFilterGroup) {
+            for (uint32_t point = lane; point < G.points.n; point += 32u * kFilterGroup) {
                 unsigned long long* pixel[kFilterGroup];
                 unsigned long long current[kFilterGroup];
 #pragma unroll
                 for (uint32_t k = 0; k < kFilterGroup; ++k) {
                     uint2 seed = base_seed;
-                    seed.x ^= (point + 32u * k) * 0x9E3779B9u;
-                    pixel[k] = point + 32u * k < G.end ? gps_point_pixel(a, a.framebuffer, pcg2d_uniform(seed), s) : nullptr;
+                    seed.x ^= (G.points.first + point + 32u * k) * 0x9E3779B9u;
+                    pixel[k] = point + 32u * k < G.points.n ? gps_point_pixel(a, a.framebuffer, pcg2d_uniform(seed), s) : nullptr;
                 }
 #pragma unroll
                 for (uint32_t k = 0; k < kFilterGroup; ++k) {

@@ -4,6 +4,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
+#include "sgs_gps_parts.h"
 #include "sgs_project.cuh"
 
 namespace sgs {
@@ -105,21 +106,8 @@ __device__ __forceinline__ void count_at_depth(uint32_t* __restrict__ histogram,
     if (sum != 0 && lane == __ffs(peers) - 1u) atomicAdd(histogram + bucket, sum);
 }
 
-// Items of a binned GPS Gaussian of `count` points: kGpsItemPoints points each (more where it would have
-// more than kMaxGpsParts items, so that the items of 2^20 entries stay below 2^31); an unused entry has none.
-constexpr uint32_t kGpsItemPoints = 2048;
-constexpr uint32_t kMaxGpsParts = 1024;
+// The items of the binned GPS Gaussians: sgs_gps_parts.h.
 constexpr uint32_t kNotListed = 0xffffffffu;  // WorkQueue::st_listed: the items do not fit the list
-struct GpsParts {
-    uint32_t parts, points;
-};
-__device__ __forceinline__ GpsParts gps_parts(const uint32_t count) {
-    GpsParts p;
-    const uint32_t items = (count + kGpsItemPoints - 1u) / kGpsItemPoints;
-    p.points = (items + kMaxGpsParts - 1u) / kMaxGpsParts * kGpsItemPoints;
-    p.parts = count != 0 ? (count + p.points - 1u) / p.points : 0u;
-    return p;
-}
 
 // Per-entry arrays of the GPS large-Gaussian queue (structure of arrays, 16-byte aligned).
 struct QueueArrays {
