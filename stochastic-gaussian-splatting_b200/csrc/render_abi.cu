@@ -139,15 +139,13 @@ struct FullLayout {
     sgs_workspace_layout pub;
     size_t q_key, q_geom, q_geom2, q_meta, q_count;
     // stochastic transparency: the queue's own entries at q_key; tile bounds, depth histogram, list and
-    // further entries (st_b) borrow the samples section, which the accumulate passes leave unused, or
-    // lie in a section of their own where it is too small
+    // further entries (st_b) borrow the samples section, which the accumulate passes leave unused
     size_t tile_bound, histogram, list, st_b;
     uint32_t st_own, st_capacity, st_items;
     size_t group_order;  // the front-to-back scatter pass's; 0: none
 };
 
 uint32_t scatter_groups(const uint32_t n) { return n / 32u + (n % 32u != 0 ? 1u : 0u); }
-
 
 FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n_samples = 1) {
     FullLayout F{};
@@ -158,51 +156,48 @@ FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n
     L.framebuffer = off;  // n_samples framebuffers of n_fb keys, back to back
     off = align_up(off + d.n_fb * n_samples * sizeof(unsigned long long));
     L.samples = off;
-    off = align_up(off + d.n_fb * sizeof(float4));
+    const size_t bounds = align_up((static_cast<size_t>(d.tiles_x) * d.tiles_y + bound_blocks(d)) * sizeof(uint32_t));
+    const size_t groups = align_up(scatter_groups(d.n) * sizeof(uint32_t));
+    size_t fixed = bounds + align_up(2 * kDepthBuckets * sizeof(uint32_t));
+    // stochastic transparency: 60 bytes for each of min(N, 2^18) entries of the queue in any case; the samples
+    // section grows where it cannot hold their list
+    constexpr size_t kListBytes = kItemsPerEntry * sizeof(uint32_t);
+    const size_t least = std::max<size_t>(std::min(d.st_wanted, kStQueueCapacity) * size_t(60) / kStEntryBytes, 1);
+    size_t room = d.n_fb * sizeof(float4);
+    if (d.st_queue) room = std::max(room, fixed + align_up(least * kListBytes));
+    off = align_up(off + room);
     L.reuse_weights = off;
     if (s->spatial_reuse) off = align_up(off + d.n_fb * sizeof(float4));
     F.q_key = off;
     if (d.st_queue) {
-        // 60 bytes for each of min(N, 2^18) entries in any case; more where the workspace stays within the
-        // scratch of the allocation-free render (several samples per call never run there)
-        const size_t bounds = align_up((static_cast<size_t>(d.tiles_x) * d.tiles_y + bound_blocks(d)) * sizeof(uint32_t));
-        size_t fixed = bounds + align_up(2 * kDepthBuckets * sizeof(uint32_t));
-        constexpr size_t kListBytes = kItemsPerEntry * sizeof(uint32_t);
-        const size_t room = d.n_fb * sizeof(float4);
-        size_t own = std::max<size_t>(std::min(d.st_wanted, kStQueueCapacity) * size_t(60) / kStEntryBytes, 1);
-        const bool borrow = fixed + align_up(own * kListBytes) <= room;
         // the front-to-back pass's order, where the section has room for it too
-        const size_t groups = align_up(scatter_groups(d.n) * sizeof(uint32_t));
-        if (may_run_front_to_back(d, false, n_samples) && fixed + groups + align_up(own * kListBytes) <= room) {
+        if (may_run_front_to_back(d, false, n_samples) && fixed + groups + align_up(least * kListBytes) <= room) {
             F.group_order = L.samples + fixed;
             fixed += groups;
         }
-        if (borrow) {
-            const size_t listed = (room - fixed) / kListBytes - kAlign / kListBytes;
-            const size_t spare =
-                n_samples > 1 ? d.st_wanted : (kNoAllocScratchBytes - std::min(off, kNoAllocScratchBytes)) / kStEntryBytes;
-            own = std::max(own, std::min({static_cast<size_t>(d.st_wanted), spare, listed}));
-        }
+        // more entries where the workspace stays within the scratch of the allocation-free render (several samples
+        // per call never run there)
+        const size_t spare =
+            n_samples > 1 ? d.st_wanted : (kNoAllocScratchBytes - std::min(off, kNoAllocScratchBytes)) / kStEntryBytes;
+        const size_t more_wanted = std::min<size_t>(d.st_wanted, spare);
+        const size_t own = std::max(least, std::min(more_wanted, (room - fixed) / kListBytes - kAlign / kListBytes));
         F.st_own = static_cast<uint32_t>(own);
-        off = align_up(off + own * kStEntryBytes);
-        F.tile_bound = borrow ? L.samples : off;
-        F.histogram = F.tile_bound + bounds;
-        F.list = F.tile_bound + fixed;
+        F.tile_bound = L.samples;
+        F.histogram = L.samples + bounds;
+        F.list = L.samples + fixed;
         // the list: kItemsPerEntry places for each entry, or half of the borrowed section (two items per
         // framebuffer pixel, more than a scene that covers it 10,000 times needs); further entries behind it
+        const size_t left = room - fixed - kAlign;
+        const size_t items = std::max(own * kItemsPerEntry, std::min<size_t>(left / 2 / sizeof(uint32_t), kMaxItems));
+        const size_t used = align_up(items * sizeof(uint32_t));
+        const size_t more = left > used ? (left - used) / kStEntryBytes : 0;
         F.st_capacity = F.st_own;
-        size_t items = own * kItemsPerEntry;
-        if (borrow) {
-            const size_t left = room - fixed - kAlign;
-            items = std::max(items, std::min<size_t>(left / 2 / sizeof(uint32_t), kMaxItems));
-            const size_t used = align_up(items * sizeof(uint32_t));
-            const size_t more = left > used ? (left - used) / kStEntryBytes : 0;
-            if (d.st_wanted > own) F.st_capacity += static_cast<uint32_t>(std::min<size_t>(d.st_wanted - own, more));
-        }
+        if (d.st_wanted > own) F.st_capacity += static_cast<uint32_t>(std::min<size_t>(d.st_wanted - own, more));
         F.st_items = static_cast<uint32_t>(items);
-        F.st_b = F.list + align_up(items * sizeof(uint32_t));
-        if (!borrow) off = F.st_b;
-        L.total = off;
+        F.st_b = F.list + used;
+        // The size is that of as many entries as there would be without bounds, histogram and order, which take
+        // more of the section in larger scenes: a workspace serves every smaller scene and image.
+        L.total = align_up(off + std::max(least, std::min(more_wanted, room / kListBytes)) * kStEntryBytes);
         return F;
     }
     // GPS front to back: tile bounds, depth histogram (cleared with them) and order borrow the samples section.
@@ -213,11 +208,7 @@ FullLayout make_layout(const Derived& d, const sgs_settings* s, const uint32_t n
     // one whose items turn out not to fit the list, is taken as it came
     const bool listed = d.queue_capacity >= kMinOrdered && d.queue_capacity <= kItemEntryMask + 1u;
     if (front || listed) {
-        const size_t bounds = align_up((static_cast<size_t>(d.tiles_x) * d.tiles_y + bound_blocks(d)) * sizeof(uint32_t));
-        size_t fixed = bounds + align_up(2 * kDepthBuckets * sizeof(uint32_t));
-        const size_t room = d.n_fb * sizeof(float4);
         const size_t list = listed ? kMinOrdered * sizeof(uint32_t) : 0;
-        const size_t groups = align_up(scatter_groups(d.n) * sizeof(uint32_t));
         if (front && fixed + groups + list <= room) {
             F.group_order = L.samples + fixed;
             fixed += groups;
