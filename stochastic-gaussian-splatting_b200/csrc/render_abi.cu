@@ -71,8 +71,8 @@ struct Derived {
     uint32_t n;               // Gaussians
 };
 
-// Whether a scatter pass may run front to back (sgs_front.cuh), and the coverage by all Gaussians above which it
-// does, which the clear pass estimates. The order costs the clear pass some 4 us, and a pass prepared for it that
+// Whether a scatter pass of n_samples samples may run front to back (sgs_front.cuh), and the coverage by all
+// Gaussians above which it does, which the clear pass estimates. The order costs the clear pass some 4 us, and a pass prepared for it that
 // then takes the Gaussians as they lie 1 to 2 % (Gaussian point splatting 5 %, as it has less to do per Gaussian), so
 // that few Gaussians, or few per pixel, are not prepared for it; below some 2.5M most of them are in flight before
 // the first bounds exist. As they lie against front to back, in us, the 6M scene cut to n Gaussians:
@@ -413,8 +413,15 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
             stq.log_row_split = 0;
     }
 
+    // Point splatting whose passes draw one sample each (for the k-buffer, the Reproject history, the queue) goes by the
+    // rule of one sample: 2 samples of 2.2M Gaussians at 1280x720 with Reproject 316 us by the call's number, 271 by
+    // the pass's, of 4M at 1920x1080 586 and 549. (Stochastic transparency: 417 and 425, of 2.2M at 1920x1080 592 and
+    // 593.) The layout has room for the order by the call's number, which asks for fewer Gaussians.
+    const bool sample_by_sample = s->use_gps && (s->spatial_reuse || s->temporal_mode == SGS_TEMPORAL_REPROJECT ||
+                                                 s->hybrid_scheduling);
+    const uint32_t pass_samples = sample_by_sample ? 1u : n_samples;
     GroupOrder groups{};
-    if (F.group_order != 0) {
+    if (F.group_order != 0 && may_run_front_to_back(d, s->use_gps != 0, pass_samples)) {
         groups.order = reinterpret_cast<uint32_t*>(ws + F.group_order);
         groups.groups = scatter_groups(g->n_gaussians);
         groups.slices = (groups.groups + kSliceGroups - 1) / kSliceGroups;
@@ -424,8 +431,10 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
         const uint32_t drawing = groups.groups / kOrderedWarps, sweep = quads / (16 * kOrderedWarps) + 1;
         const uint32_t sweeps = std::min(std::max(drawing / (24 * sweep), 8u), 16u);
         groups.refresh_period = 1 + std::max(drawing / (sweeps * sweep), 1u);
-        groups.min_pixels = (s->use_gps && n_samples == 1 ? kFrontCoverageGps : kFrontCoverage) * static_cast<float>(d.n_fb);
+        groups.min_pixels = (s->use_gps && pass_samples == 1 ? kFrontCoverageGps : kFrontCoverage) * static_cast<float>(d.n_fb);
     }
+
+    if (s->use_gps && groups.order == nullptr && stq.list == nullptr) stq = StQueue{};  // nothing reads the bounds
 
     const PassCamera cam = pass_camera(c, s, d.ss);
     AccumulateParams ap{};
