@@ -421,7 +421,12 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
                                                  s->hybrid_scheduling);
     const uint32_t pass_samples = sample_by_sample ? 1u : n_samples;
     GroupOrder groups{};
-    if (F.group_order != 0 && may_run_front_to_back(d, s->use_gps != 0, pass_samples)) {
+    // Hybrid stochastic transparency evaluates the first max_binned large Gaussians in the gather's form. A bin that a
+    // caller sets smaller than the reference's may fill, and depth order, which leaves hidden groups out of the count,
+    // would choose others by the view; past the reference's 2^20 the order of arrival is left to chance as ever.
+    const bool small_bin =
+        !s->use_gps && s->hybrid_scheduling && d.max_binned < std::min(g->n_gaussians, kDefaultMaxBinned);
+    if (F.group_order != 0 && !small_bin && may_run_front_to_back(d, s->use_gps != 0, pass_samples)) {
         groups.order = reinterpret_cast<uint32_t*>(ws + F.group_order);
         groups.groups = scatter_groups(g->n_gaussians);
         groups.slices = (groups.groups + kSliceGroups - 1) / kSliceGroups;

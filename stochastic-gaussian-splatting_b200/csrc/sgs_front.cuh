@@ -4,7 +4,9 @@
 // reaches a pixel before the pixel's last winner. Warps take groups of 32 consecutive Gaussians in depth order
 // (GroupOrder), blocks among them lower an upper bound of the keys' depths per 8 x 8 pixel tile, and Gaussians
 // behind the bounds of all tiles that they touch are dropped, most of them before their projection. Keys only
-// decrease during a pass and a bound is never below its tile's keys, so the winners do not depend on any of it.
+// decrease during a pass and a bound is never below its tile's keys, so the winners do not depend on any of it. (With
+// more than 2^20 Gaussians above 512 pixels under hybrid scheduling, which of them the bin holds, and with that the
+// last bit of an alpha, depends on the order of arrival, here as in passes that take them as they lie.)
 #pragma once
 
 #include <cstdint>

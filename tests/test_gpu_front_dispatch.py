@@ -56,3 +56,20 @@ def test_passes_of_one_sample_keep_the_rule_of_one_sample(more, cuda_device):
     assert covered_all(together) > 58 * WIDTH * HEIGHT
     _, _, apart = render(scene, cuda_device, samples=2, **more)
     assert covered_all(apart) == 0
+
+
+def binned(header):
+    return int(header[20:24].view(torch.int32))  # WorkQueue::binned
+
+
+def test_a_small_bin_of_stochastic_transparency_fills_as_the_gaussians_lie(cuda_device):
+    """Hybrid scheduling evaluates the first max_binned Gaussians above 512 pixels in another form; depth order, and
+    groups left out of the count, would change which these are."""
+    scene = deep_scene((1 << 21) + 45, -4.2).to(cuda_device).tensors()
+    _, _, alone = render(scene, cuda_device, gps=False, hybrid=True, max_binned=64)
+    assert binned(alone) > 1000
+    _, _, small = render(scene, cuda_device, gps=False, hybrid=True, max_binned=64, samples=2)
+    assert binned(small) == binned(alone)
+    # a bin that cannot fill does not hinder the order, which leaves most of them out
+    _, _, full = render(scene, cuda_device, gps=False, hybrid=True, samples=2)
+    assert binned(full) < binned(alone)
