@@ -107,7 +107,7 @@ __device__ __forceinline__ void count_at_depth(uint32_t* __restrict__ histogram,
 }
 
 // The items of the binned GPS Gaussians: sgs_gps_parts.h.
-constexpr uint32_t kNotListed = 0xffffffffu;  // WorkQueue::st_listed: the items do not fit the list
+constexpr uint32_t kNotListed = 0xffffffffu;  // WorkQueue::st_listed: the chunks are taken as they came
 
 // Per-entry arrays of the GPS large-Gaussian queue (structure of arrays, 16-byte aligned).
 struct QueueArrays {
