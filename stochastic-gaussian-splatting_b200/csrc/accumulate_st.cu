@@ -49,10 +49,8 @@ constexpr uint32_t kBlock = 256;
 constexpr uint32_t kWarpsPerBlock = kBlock / 32;
 constexpr uint32_t kFullMask = 0xffffffffu;
 constexpr uint32_t kQueueBlocksPerSM = 4;
-// AABBs with more pixels are queued: kDenseMinPixels where the Gaussians above that size cover the
-// framebuffer many times over, kMinPixels elsewhere (dense_scene).
-constexpr uint32_t kMinPixels = 2048;
-constexpr uint32_t kDenseMinPixels = 256;
+// AABBs with more pixels are queued where the scene is not dense (queued_above).
+constexpr uint32_t kMinPixels = kDenseMinPixels << kQueueSteps;
 constexpr uint32_t kChunkPixels = 2048;   // pixels per chunk of rows of a queued Gaussian in a sparse scene
 constexpr float kSampleMaxCover = 32.0f;  // a sampled Gaussian counts for at most this many framebuffers
 constexpr uint32_t kOrderBlock = 512;
@@ -426,6 +424,22 @@ __device__ __forceinline__ bool dense_scene(const AccumulateParams& a) {
     return c.x + c.y + c.z + c.w > a.stq.dense_pixels;
 }
 
+// AABBs above this many pixels are queued: in a dense scene all above kDenseMinPixels if the queue holds them, else
+// those of the next larger size that it holds. A warp draws what finds the queue full by itself, which takes long where
+// that are Gaussians of many thousand pixels (2M Gaussians and 24,000 large ones at 1920x1080, room for 0.53 of 1.30
+// million above 256: 2631 us a sample; of the larger ones that it holds 1367; with a queue for 2048 and more 1731). A
+// few per cent past the room cost less than the next size (1M Gaussians at 1280x720, room for all: 455 and 539 us).
+__device__ __forceinline__ uint32_t queued_above(const AccumulateParams& a, const bool dense) {
+    const float room = 1.05f * static_cast<float>(a.stq.capacity);
+    uint32_t step = kQueueSteps;
+#pragma unroll
+    for (uint32_t i = kQueueSteps; i-- > 0;) {
+        const float4 n = *reinterpret_cast<const float4*>(a.queue->larger[i]);
+        if (n.x + n.y + n.z + n.w <= room) step = i;
+    }
+    return dense ? kDenseMinPixels << step : kMinPixels;
+}
+
 // How a scatter pass takes its Gaussians: a warp 32 of them, several warps the same 32 (small scenes), or a warp
 // 32 of them front to back, dropping those behind their tiles' bounds.
 enum ScatterMode { kPlain, kSplitRows, kFrontToBack };
@@ -466,10 +480,21 @@ st_scatter_kernel(const AccumulateParams a) {
 
     if (kMode == kFrontToBack && ordered && group_hidden(a, active, g, lane)) return;
 
+    // Loaded while the projection waits for its own loads: after it, the scatter pass over 400k large Gaussians took 73 us
+    // instead of 68. Deep scenes are seldom dense and load the sizes only then, after the projection.
+    bool dense = false;
+    uint32_t queue_above = kMinPixels;
+    if (kMode != kFrontToBack) {
+        dense = dense_scene(a);
+        queue_above = queued_above(a, dense);
+    }
     Projected p;
     if (!project_gaussian(active, g, a.means, a.scales, a.rotations, a.opacities, a.w2c, a.cam, p, a.pre, a.quant)) return;
     const FrameRng rng = frame_rng(a);
-    const bool dense = dense_scene(a);
+    if (kMode == kFrontToBack) {
+        dense = dense_scene(a);
+        if (dense) queue_above = queued_above(a, true);
+    }
 
     const PixelRect rect = pixel_rect(p.bounds, a.cam);
     uint32_t count = active ? rect.width * rect.height : 0u;
@@ -517,7 +542,7 @@ st_scatter_kernel(const AccumulateParams a) {
     // larger footprints: an entry in the work queue (or kept here when it is full); one atomic per warp
     bool keep_big = false;
     bool has_rows = count > 0;
-    const bool large = count > (dense ? kDenseMinPixels : kMinPixels);
+    const bool large = count > queue_above;
     const bool want = large && sub == 0;
     if (large) has_rows = false;
     const uint32_t big = __ballot_sync(kFullMask, want);
@@ -878,6 +903,7 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
     wait_for_pass_before();
     if (blockIdx.x < kSampleBlocks) {
         __shared__ float2 s_sum[kWarpsPerBlock];
+        __shared__ uint32_t s_larger[kQueueSteps][kWarpsPerBlock];
         const uint32_t t = blockIdx.x * kBlock + threadIdx.x;
         const uint32_t step = max(a.n / (kSampleBlocks * kBlock), 1u);
         bool active = t < a.n;
@@ -889,11 +915,11 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
             asm volatile("prefetch.global.L2 [%0];" ::"l"(a.opacities + g));
         }
         Projected p;
-        float pixels = 0.0f, larger = 0.0f;
+        float pixels = 0.0f, larger = 0.0f, own = 0.0f;
         if (project_gaussian(active, g, a.means, a.scales, a.rotations, a.opacities, a.w2c, a.cam, p, a.pre, a.quant) &&
             active) {
             const PixelRect rect = pixel_rect(p.bounds, a.cam);
-            const float own = static_cast<float>(rect.width) * static_cast<float>(rect.height);
+            own = static_cast<float>(rect.width) * static_cast<float>(rect.height);
             pixels = fminf(own * static_cast<float>(step), kSampleMaxCover * a.cam.width * a.cam.height);
             larger = own > static_cast<float>(kDenseMinPixels) ? pixels : 0.0f;
         }
@@ -902,11 +928,20 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
             larger += __shfl_xor_sync(kFullMask, larger, o);
         }
         if ((threadIdx.x & 31u) == 0) s_sum[threadIdx.x >> 5] = make_float2(larger, pixels);
+        for (uint32_t i = 0; i < kQueueSteps; ++i) {
+            const uint32_t above = __ballot_sync(kFullMask, own > static_cast<float>(kDenseMinPixels << i));
+            if ((threadIdx.x & 31u) == 0) s_larger[i][threadIdx.x >> 5] = __popc(above);
+        }
         __syncthreads();
         if (threadIdx.x == 0) {
             for (uint32_t w = 1; w < kWarpsPerBlock; ++w) larger += s_sum[w].x, pixels += s_sum[w].y;
             a.queue->covered[blockIdx.x] = larger;
             a.queue->covered_all[blockIdx.x] = pixels;
+            for (uint32_t i = 0; i < kQueueSteps; ++i) {
+                uint32_t sum = 0;
+                for (uint32_t w = 0; w < kWarpsPerBlock; ++w) sum += s_larger[i][w];
+                a.queue->larger[i][blockIdx.x] = static_cast<float>(sum) * static_cast<float>(step);
+            }
         }
         return;
     }

@@ -9,6 +9,11 @@
 
 namespace sgs {
 
+// Stochastic transparency queues AABBs above kDenseMinPixels << step pixels in dense scenes, by the first step whose
+// Gaussians the queue holds, and above kDenseMinPixels << kQueueSteps elsewhere.
+constexpr uint32_t kDenseMinPixels = 256;
+constexpr uint32_t kQueueSteps = 3;
+
 // Large-Gaussian work queue shared by the ST and GPS accumulate passes. Entries are appended
 // with one 64-bit atomicAdd on `packed` = (entry count << 40) | chunk count, so every entry's
 // first chunk index is known at insertion and increases with the entry index.
@@ -24,8 +29,10 @@ struct WorkQueue {
     alignas(16) float covered[4];      // AABB pixels of the scene's larger Gaussians, estimated by kSampleBlocks
                                        // blocks of the clear pass
     alignas(16) float covered_all[4];  // the same of all its Gaussians
+    alignas(16) float larger[kQueueSteps][4];  // Gaussians with AABBs above kDenseMinPixels << step, estimated likewise
 };
-static_assert(offsetof(WorkQueue, covered) % 16 == 0 && offsetof(WorkQueue, covered_all) % 16 == 0, "read as float4");
+static_assert(offsetof(WorkQueue, covered) % 16 == 0 && offsetof(WorkQueue, covered_all) % 16 == 0 &&
+              offsetof(WorkQueue, larger) % 16 == 0, "read as float4");
 constexpr unsigned long long kQueueEntryShift = 40;
 constexpr unsigned long long kQueueChunkMask = (1ull << kQueueEntryShift) - 1;
 // Producers queue chunk indices below this, so the consumers' cursor (which overshoots the last chunk
