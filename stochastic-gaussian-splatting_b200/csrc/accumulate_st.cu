@@ -914,6 +914,8 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
             asm volatile("prefetch.global.L2 [%0];" ::"l"(a.rotations + g));
             asm volatile("prefetch.global.L2 [%0];" ::"l"(a.opacities + g));
         }
+        const bool points = a.stq.capacity == 0;  // of point splatting, which has no such queue
+        const bool compact = !points || in_compact_group(a, g);
         Projected p;
         float pixels = 0.0f, larger = 0.0f, own = 0.0f;
         if (project_gaussian(active, g, a.means, a.scales, a.rotations, a.opacities, a.w2c, a.cam, p, a.pre, a.quant) &&
@@ -922,6 +924,7 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
             own = static_cast<float>(rect.width) * static_cast<float>(rect.height);
             pixels = fminf(own * static_cast<float>(step), kSampleMaxCover * a.cam.width * a.cam.height);
             larger = own > static_cast<float>(kDenseMinPixels) ? pixels : 0.0f;
+            if (!compact) pixels = 0.0f;
         }
         for (uint32_t o = 16; o > 0; o >>= 1) {
             pixels += __shfl_xor_sync(kFullMask, pixels, o);

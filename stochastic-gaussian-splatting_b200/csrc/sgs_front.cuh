@@ -43,6 +43,20 @@ __device__ __forceinline__ float dot_plus(const float4 r, const float3 m) {
     return r.x * m.x + r.y * m.y + r.z * m.z + r.w;
 }
 
+// Whether Gaussian g lies near one of the other half of its group, on the screen (group_hidden tests rectangles of up to
+// 256 pixels) and in depth. In a model that is not in Morton order hardly one does: there the groups' order and tests are
+// for nothing, and point splatting, which drops only whole groups, is slower (6M Gaussians at random at 1080p: 457 us
+// front to back, 396 as they lie; 8 samples 2289 and 2193 us). Stochastic transparency drops single Gaussians all the
+// same (642 and 631 us, 8 samples 2480 and 2690).
+__device__ __forceinline__ bool in_compact_group(const AccumulateParams& a, const uint32_t g) {
+    const float3 m = gaussian_position(a, g), o = gaussian_position(a, min(g ^ 16u, a.n - 1u));
+    const float4 r1 = a.w2c[0], r2 = a.w2c[1], r3 = a.w2c[2];
+    const float z = dot_plus(r3, m), zo = dot_plus(r3, o);
+    const float dx = (dot_plus(r1, m) / z - dot_plus(r1, o) / zo) * a.cam.focal_x;
+    const float dy = (dot_plus(r2, m) / z - dot_plus(r2, o) / zo) * a.cam.focal_y;
+    return fabsf(z - zo) <= 0.25f * fabsf(z) && fabsf(dx) <= 128.0f && fabsf(dy) <= 128.0f;
+}
+
 // Sorts the groups slice, slice + a.groups.slices, ... by depth (GroupOrder).
 template <uint32_t kBlock>
 __device__ __forceinline__ void sort_slice(const AccumulateParams& a, const uint32_t slice) {

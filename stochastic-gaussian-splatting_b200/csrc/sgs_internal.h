@@ -28,7 +28,7 @@ struct WorkQueue {
     unsigned int st_listed;      // items the order pass has listed (GPS: or kNotListed)
     alignas(16) float covered[4];      // AABB pixels of the scene's larger Gaussians, estimated by kSampleBlocks
                                        // blocks of the clear pass
-    alignas(16) float covered_all[4];  // the same of all its Gaussians
+    alignas(16) float covered_all[4];  // the same of all its Gaussians (GPS: of those in compact groups)
     alignas(16) float larger[kQueueSteps][4];  // Gaussians with AABBs above kDenseMinPixels << step, estimated likewise
 };
 static_assert(offsetof(WorkQueue, covered) % 16 == 0 && offsetof(WorkQueue, covered_all) % 16 == 0 &&

@@ -73,3 +73,15 @@ def test_a_small_bin_of_stochastic_transparency_fills_as_the_gaussians_lie(cuda_
     # a bin that cannot fill does not hinder the order, which leaves most of them out
     _, _, full = render(scene, cuda_device, gps=False, hybrid=True, samples=2)
     assert binned(full) < binned(alone)
+
+
+@pytest.mark.parametrize("layout", ["float", "pre", "quant"])
+def test_points_of_models_in_no_order_are_drawn_as_they_lie(layout, cuda_device):
+    """Groups of Gaussians from all over the scene are not compact: their coverage does not count."""
+    scene = deep_scene((1 << 21) + 45, -5.0)
+    ordered = render(scene.to(cuda_device).tensors(), cuda_device, samples=2, mode=1, layout=layout)[2]
+    perm = torch.randperm(scene.means.shape[0], generator=torch.Generator().manual_seed(3))
+    shuffled = [t[perm].contiguous().to(cuda_device) for t in scene.tensors()]
+    at_random = render(shuffled, cuda_device, samples=2, mode=1, layout=layout)[2]
+    n_fb = WIDTH * HEIGHT
+    assert covered_all(ordered) > 110 * n_fb and 0 < covered_all(at_random) < 58 * n_fb
