@@ -436,6 +436,7 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
         const uint32_t drawing = groups.groups / kOrderedWarps, sweep = quads / (16 * kOrderedWarps) + 1;
         const uint32_t sweeps = std::min(std::max(drawing / (24 * sweep), 8u), 16u);
         groups.refresh_period = 1 + std::max(drawing / (sweeps * sweep), 1u);
+        groups.refresh_rcp = 1.0 / static_cast<double>(groups.refresh_period);
         groups.min_pixels = (s->use_gps && pass_samples == 1 ? kFrontCoverageGps : kFrontCoverage) * static_cast<float>(d.n_fb);
     }
 

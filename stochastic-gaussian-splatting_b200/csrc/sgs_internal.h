@@ -93,6 +93,7 @@ struct GroupOrder {
     uint32_t groups;
     uint32_t slices;
     uint32_t refresh_period;  // every refresh_period-th block of the pass lowers tile bounds
+    double refresh_rcp;       // 1 / refresh_period
     float min_pixels;         // covered pixels above which the pass runs in depth order
 };
 
