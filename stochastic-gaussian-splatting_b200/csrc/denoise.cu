@@ -2,16 +2,17 @@
 //
 // The reference has no learned resolve; plain progressive averaging (resolve.cu, Static mode) is the
 // fallback and the yardstick of its error. This file holds every kernel of the denoiser:
-//   conv3x3_kernel        implicit-GEMM 3x3 convolution, zero padding 1, stride 1. Forward layers
-//                         (bias + ReLU, or bias + residual for the last layer) and data gradients
-//                         (flipped, transposed weights; the ReLU mask of the layer below fused).
-//   conv3x3_wgrad_kernel  weight and bias gradients of one layer, summed over all pixels.
-//   conv3x3_wgrad_tma_kernel the same for BF16 inputs, loaded by TMA.
+//   conv3x3_tma_kernel    implicit-GEMM 3x3 convolution, zero padding 1, stride 1, of BF16 inputs loaded
+//                         by TMA. Forward layers (bias + ReLU, or bias + residual for the last layer) and
+//                         data gradients (flipped, transposed weights; the ReLU mask of the layer below fused).
+//   conv3x3_kernel        the first layer on FP16 features (sgs_conv3x3 alone; whole calls convert them first).
+//   conv3x3_wgrad_tma_kernel weight and bias gradients of one layer with BF16 input, summed over all pixels.
+//   conv3x3_wgrad_kernel  those of the first layer on FP16 features (sgs_conv3x3_wgrad alone).
 //   train_*               one training step's weight packing, gradient staging and unpacking.
 //   features_*            the 8-channel FP16 input built from the per-sample renders.
 //
-// Activations are NHWC BF16 [batch][height][width][channels], channels 16 or 32. One CTA of 128
-// threads computes an 8 x 16 pixel tile (M = 128) at a time: it stages the 10 x 18 input halo in
+// Activations are NHWC BF16 [batch][height][width][channels], channels 16 or 32. A CTA
+// computes an 8 x 16 pixel tile (M = 128) at a time: it stages the 10 x 18 input halo in
 // shared memory as [8-channel chunk][halo pixel][8 channels], so that for every tap (dy, dx) the A
 // operand is a K-major no-swizzle view of the halo starting (dy * 10 + dx) * 16 bytes in: the 8
 // pixels of a tile row are 16 bytes apart (one core matrix), tile rows 160 bytes apart (SBO), the
@@ -23,7 +24,7 @@
 // halo loads overlap another's MMAs and epilogue.
 //
 // The weight gradient is a GEMM over pixels: dW[tap][co][ci] = sum_p dZ[p][co] * X[p + tap][ci].
-// Per tile the kernel builds an im2col block in shared memory, [group][pixel][8], group =
+// Per tile conv3x3_wgrad_kernel builds an im2col block in shared memory, [group][pixel][8], group =
 // (tap, 8-channel chunk) plus one group whose first channel is 1 (its row of the product is the
 // bias gradient), and multiplies it as an MN-major A (M = 128 rows of (tap, channel)) with the
 // tile's output gradient as an MN-major B (N = COUT). Accumulators stay in TMEM across all the
@@ -56,7 +57,6 @@ constexpr int kTilePx = kTileW * kTileH;  // 128 = MMA M
 constexpr int kThreads = 128;
 constexpr uint32_t kWaitLimit = 1u << 20;
 
-enum InKind { kInBf16 = 0, kInFeatures = 1 };
 enum Epilogue { kEpiRelu = SGS_CONV_RELU, kEpiFinal = SGS_CONV_FINAL, kEpiMask = SGS_CONV_MASK };
 
 __device__ unsigned int g_error;
@@ -107,30 +107,17 @@ __device__ __forceinline__ TileXY tile_xy(int t, int tiles_x, int tiles_y) {
 }
 
 // Stages the 10 x 18 halo of the tile at (x0, y0) as [chunk][halo pixel][8] BF16, zero outside the
-// image. kInFeatures: 8 FP16 channels per pixel, converted to BF16, channels 8..15 zero.
-template <int CIN, int IN>
+// image, from 8 FP16 channels per pixel; channels 8..15 are zero.
+constexpr int kFeatureChannels = 16;  // as staged
 __device__ __forceinline__ void load_halo(const void* in, uint4* halo, const TileXY& t, int height, int width) {
     const uint4* src = static_cast<const uint4*>(in);
-    if constexpr (IN == kInFeatures) {
-        static_assert(CIN == 16, "features stage as 16 channels");
-        for (int p = threadIdx.x; p < kHaloPx; p += kThreads) {
-            const int gx = t.x0 - 1 + p % kHaloW, gy = t.y0 - 1 + p / kHaloW;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (gx >= 0 && gx < width && gy >= 0 && gy < height)
-                v = half8_to_bf16x8(__ldg(src + (static_cast<size_t>(t.b) * height + gy) * width + gx));
-            halo[p] = v;
-            halo[kHaloPx + p] = make_uint4(0u, 0u, 0u, 0u);
-        }
-    } else {
-        constexpr int KC = CIN / 8;
-        for (int i = threadIdx.x; i < kHaloPx * KC; i += kThreads) {
-            const int p = i / KC, c = i % KC;
-            const int gx = t.x0 - 1 + p % kHaloW, gy = t.y0 - 1 + p / kHaloW;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (gx >= 0 && gx < width && gy >= 0 && gy < height)
-                v = __ldg(src + ((static_cast<size_t>(t.b) * height + gy) * width + gx) * KC + c);
-            halo[c * kHaloPx + p] = v;
-        }
+    for (int p = threadIdx.x; p < kHaloPx; p += kThreads) {
+        const int gx = t.x0 - 1 + p % kHaloW, gy = t.y0 - 1 + p / kHaloW;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (gx >= 0 && gx < width && gy >= 0 && gy < height)
+            v = half8_to_bf16x8(__ldg(src + (static_cast<size_t>(t.b) * height + gy) * width + gx));
+        halo[p] = v;
+        halo[kHaloPx + p] = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
@@ -195,13 +182,12 @@ __device__ __forceinline__ void store_pixel(const ConvArgs& a, const TileXY& til
     }
 }
 
-template <int CIN, int COUT, int IN, int EPI>
 __global__ void __launch_bounds__(kThreads, 1) conv3x3_kernel(const ConvArgs a) {
-    constexpr int KC = CIN / 8;
+    constexpr int COUT = 32;
+    constexpr int KC = kFeatureChannels / 8;
     constexpr int kWeightVecs = 9 * KC * COUT;
     constexpr int kHaloVecs = KC * kHaloPx;
     constexpr uint32_t kIdesc = tc::instr_desc_bf16(kTilePx, COUT, false, false);
-    static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "tile shapes");
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     uint4* w_s = reinterpret_cast<uint4*>(smem_raw);
@@ -223,13 +209,13 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_kernel(const ConvArgs a) 
 
     float bias[COUT];
 #pragma unroll
-    for (int n = 0; n < COUT; ++n) bias[n] = (EPI == kEpiMask) ? 0.0f : __ldg(a.bias + n);
+    for (int n = 0; n < COUT; ++n) bias[n] = __ldg(a.bias + n);
 
     uint32_t phase = 0;
     bool failed = false;
     for (int t = blockIdx.x; t < a.n_tiles; t += gridDim.x) {
         const TileXY tile = tile_xy(t, a.tiles_x, a.tiles_y);
-        load_halo<CIN, IN>(a.in, halo, tile, a.height, a.width);
+        load_halo(a.in, halo, tile, a.height, a.width);
         tc::fence_async_smem();
         tc::fence_before_sync();
         __syncthreads();
@@ -255,7 +241,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_kernel(const ConvArgs a) 
         float acc[COUT];
         load_accumulator<COUT>(tmem + (static_cast<uint32_t>(warp * 32) << 16), acc);
 
-        if (ok) store_pixel<COUT, EPI>(a, tile, tid, acc, bias);
+        if (ok) store_pixel<COUT, kEpiRelu>(a, tile, tid, acc, bias);
         tc::fence_before_sync();
         if (__syncthreads_or(!ok)) {
             failed = true;
@@ -339,7 +325,7 @@ __global__ void __launch_bounds__(kTmaThreads, 4) conv3x3_tma_kernel(const __gri
     __syncthreads();
     tc::fence_after_sync();
     // everything above reads only the weights, which are older than the kernel before
-    tc::wait_dependencies();
+    wait_for_pass_before();
     tc::launch_dependents();
     const uint32_t tmem = *slot;
     const uint32_t halo_a = tc::smem_u32(halo);
@@ -437,31 +423,32 @@ __global__ void __launch_bounds__(kTmaThreads, 4) conv3x3_tma_kernel(const __gri
 #undef SGS_ACC_EMPTY
 }
 
-// Weight-gradient geometry: im2col groups of 8 rows, (tap, chunk) for tap-major order, then the
-// bias group, then zero groups up to the allocation. M-tile m reads groups start(m) .. start(m)+15
-// and owns (adds to the gradient) groups [own(m), own(m+1)).
-template <int CIN, int COUT>
+// Weight-gradient geometry of the FP16 features: im2col groups of 8 rows, (tap, chunk) for tap-major order,
+// then the bias group, then a zero group. M-tile m reads groups start(m) .. start(m) + 15 and owns (adds to
+// the gradient) groups [own(m), own(m + 1)).
 struct Wgrad {
-    static constexpr int KC = CIN / 8;
+    static constexpr int COUT = 32;
+    static constexpr int KC = kFeatureChannels / 8;
     static constexpr int KCO = COUT / 8;
     static constexpr int kConvGroups = 9 * KC;
     static constexpr int kBiasGroup = kConvGroups;
-    static constexpr int kMTiles = CIN == 32 ? 3 : 2;
-    static constexpr int kGroups = CIN == 32 ? 40 : 20;
-    static constexpr int kCols = kMTiles * COUT <= 32 ? 32 : kMTiles * COUT <= 64 ? 64 : 128;
+    static constexpr int kMTiles = 2;
+    static constexpr int kGroups = 20;
+    static constexpr int kCols = kMTiles * COUT;
     static constexpr int kHaloVecs = KC * kHaloPx;
     static constexpr int kGradVecs = KCO * kTilePx;
     static constexpr int kColVecs = kGroups * kTilePx;
     static constexpr size_t kSmem = static_cast<size_t>(kHaloVecs + kGradVecs + kColVecs) * 16 + 16;
-    __host__ __device__ static constexpr int start(int m) { return CIN == 32 ? (m == 0 ? 0 : m == 1 ? 16 : 24) : (m == 0 ? 0 : 4); }
+    static constexpr int kSecond = kGroups - 16;
+    __host__ __device__ static constexpr int start(int m) { return m * kSecond; }
     __host__ __device__ static constexpr int own(int m) { return m == 0 ? 0 : m == kMTiles ? kGroups : 16 * m; }
-    static_assert(start(kMTiles - 1) + 16 == kGroups, "last M tile ends at the allocation");
     static_assert(kBiasGroup < kGroups, "bias group allocated");
+    static_assert(kCols == 64, "a power of two of TMEM columns");
 };
 
-template <int CIN, int COUT, int IN>
 __global__ void __launch_bounds__(kThreads) conv3x3_wgrad_kernel(const WgradArgs a) {
-    using G = Wgrad<CIN, COUT>;
+    using G = Wgrad;
+    constexpr int CIN = kFeatureChannels, COUT = G::COUT;
     constexpr uint32_t kIdesc = tc::instr_desc_bf16(kTilePx, COUT, true, true);
     constexpr uint32_t kGroupBytes = kTilePx * 16;  // 2048
 
@@ -491,7 +478,7 @@ __global__ void __launch_bounds__(kThreads) conv3x3_wgrad_kernel(const WgradArgs
     bool first = true;
     for (int t = blockIdx.x; t < a.n_tiles; t += gridDim.x) {
         const TileXY tile = tile_xy(t, a.tiles_x, a.tiles_y);
-        load_halo<CIN, IN>(a.in, halo, tile, a.height, a.width);
+        load_halo(a.in, halo, tile, a.height, a.width);
         for (int i = tid; i < G::kGradVecs; i += kThreads) {
             const int k = i / G::KCO, c = i % G::KCO;
             const int x = tile.x0 + (k & 7), y = tile.y0 + (k >> 3);
@@ -617,7 +604,7 @@ __global__ void __launch_bounds__(kTmaThreads) conv3x3_wgrad_tma_kernel(const __
     tc::fence_after_sync();
     // everything above touches nothing but shared memory and TMEM; the layer's data gradient, launched behind this
     // kernel, may load its weights and set up from here on
-    tc::wait_dependencies();
+    wait_for_pass_before();
     tc::launch_dependents();
     const uint32_t tmem = *slot;
     const uint32_t smem0 = tc::smem_u32(base);
@@ -715,7 +702,7 @@ __global__ void __launch_bounds__(kTmaThreads) conv3x3_wgrad_tma_kernel(const __
 // kernels per 1080p frame).
 __global__ void __launch_bounds__(256) features_bf16_kernel(const uint4* __restrict__ features,
                                                             uint4* __restrict__ out, const uint32_t n_px) {
-    tc::wait_dependencies();
+    wait_for_pass_before();
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
     if (i < n_px) out[i] = half8_to_bf16x8(__ldg(features + i));
 }
@@ -759,7 +746,7 @@ constexpr int kPackBlocks = (kPacked + kBiases + 255) / 256;
 __global__ void __launch_bounds__(256) train_pack_kernel(const TrainParams p, __nv_bfloat16* __restrict__ weights,
                                                          float* __restrict__ biases, const uint4* __restrict__ features,
                                                          uint4* __restrict__ features_bf16, const uint32_t n_px) {
-    tc::wait_dependencies();
+    wait_for_pass_before();
     if (blockIdx.x >= kPackBlocks) {
         const uint32_t i = (blockIdx.x - kPackBlocks) * 256u + threadIdx.x;
         if (i < n_px) features_bf16[i] = half8_to_bf16x8(__ldg(features + i));
@@ -785,7 +772,7 @@ constexpr int kDgradBlocks = (kPacked - packed_before(1) + 255) / 256;
 __global__ void __launch_bounds__(256) train_stage_kernel(const TrainParams p, __nv_bfloat16* __restrict__ weights,
                                                           const float* __restrict__ grad, uint4* __restrict__ staged,
                                                           const uint32_t n_px) {
-    tc::wait_dependencies();
+    wait_for_pass_before();
     if (blockIdx.x >= kDgradBlocks) {
         const uint32_t i = (blockIdx.x - kDgradBlocks) * 256u + threadIdx.x;
         if (i >= n_px) return;
@@ -807,7 +794,7 @@ __global__ void __launch_bounds__(256) train_stage_kernel(const TrainParams p, _
 
 // Parameter gradients W1[co][ci][3][3], b1, ..., back to back from the sums [tap][co][ci] and bias sums.
 __global__ void __launch_bounds__(256) train_unpack_kernel(const float* __restrict__ sums, float* __restrict__ grads) {
-    tc::wait_dependencies();
+    wait_for_pass_before();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= kParams) return;
     int l = 0;
@@ -903,14 +890,13 @@ int resident_ctas(Kernel kernel, size_t smem, int cap, int threads = kThreads) {
     return blocks < cap ? blocks : cap;
 }
 
-template <int CIN, int COUT, int IN, int EPI>
 cudaError_t launch_conv(const ConvArgs& a, cudaStream_t stream) {
-    constexpr size_t smem = static_cast<size_t>(9 * (CIN / 8) * COUT + (CIN / 8) * kHaloPx) * 16 + 16;
-    auto kernel = conv3x3_kernel<CIN, COUT, IN, EPI>;
-    static const int per_sm = resident_ctas(kernel, smem, 8);
+    constexpr int kChunks = kFeatureChannels / 8;
+    constexpr size_t smem = static_cast<size_t>(9 * kChunks * 32 + kChunks * kHaloPx) * 16 + 16;
+    static const int per_sm = resident_ctas(conv3x3_kernel, smem, 8);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
     const int grid = a.n_tiles < sm_count() * per_sm ? a.n_tiles : sm_count() * per_sm;
-    kernel<<<grid, kThreads, smem, stream>>>(a);
+    conv3x3_kernel<<<grid, kThreads, smem, stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -990,15 +976,13 @@ cudaError_t launch_conv_tma(const ConvArgs& a, cudaStream_t stream, int in_chann
     return cudaLaunchKernelEx(&config, kernel, map, a);
 }
 
-template <int CIN, int COUT, int IN>
 cudaError_t launch_wgrad(const WgradArgs& a, cudaStream_t stream) {
-    using G = Wgrad<CIN, COUT>;
-    auto kernel = conv3x3_wgrad_kernel<CIN, COUT, IN>;
+    using G = Wgrad;
     // TMEM columns bound the CTAs per SM: 512 / kCols
-    static const int per_sm = resident_ctas(kernel, G::kSmem, 512 / G::kCols);
+    static const int per_sm = resident_ctas(conv3x3_wgrad_kernel, G::kSmem, 512 / G::kCols);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
     const int grid = a.n_tiles < sm_count() * per_sm ? a.n_tiles : sm_count() * per_sm;
-    kernel<<<grid, kThreads, G::kSmem, stream>>>(a);
+    conv3x3_wgrad_kernel<<<grid, kThreads, G::kSmem, stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -1100,7 +1084,7 @@ int sgs_conv3x3(const sgs_conv3x3_args* p, void* stream_ptr) {
     const int ci = p->in_channels, co = p->out_channels, epi = p->epilogue;
     cudaError_t err;
     if (ci == 8 && co == 32 && epi == SGS_CONV_RELU)
-        err = launch_conv<16, 32, kInFeatures, kEpiRelu>(a, stream);
+        err = launch_conv(a, stream);
     else if (ci == 32 && co == 32 && epi == SGS_CONV_RELU)
         err = launch_conv_tma<32, 32, kEpiRelu>(a, stream);
     else if (ci == 32 && co == 16 && epi == SGS_CONV_FINAL)
@@ -1130,7 +1114,7 @@ int sgs_conv3x3_wgrad(const void* input, int32_t in_channels, const void* grad_o
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     cudaError_t err;
     if (in_channels == 8 && out_channels == 32)
-        err = launch_wgrad<16, 32, kInFeatures>(a, stream);
+        err = launch_wgrad(a, stream);
     else if (in_channels == 32 && out_channels == 32)
         err = launch_wgrad_tma<32, 32>(a, stream);
     else if (in_channels == 32 && out_channels == 16)

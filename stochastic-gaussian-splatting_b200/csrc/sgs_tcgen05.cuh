@@ -131,10 +131,8 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tensor_map
       : "memory");
 }
 
-// Programmatic dependent launch: waits until the kernels this launch depends on have completed (returns at
-// once when it was launched without the attribute), and lets the launch that depends on this one begin
-// as CTAs leave.
-__device__ __forceinline__ void wait_dependencies() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Programmatic dependent launch: lets the launch that depends on this one begin as CTAs leave (it waits with
+// wait_for_pass_before).
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Bounded wait for the phase with the given parity to complete; false when the limit ran out.
