@@ -92,26 +92,28 @@ cudaError_t launch_walk(const BackwardSetup& S, cudaStream_t stream) {
                  : launch_backward_fragments_samples(S.p, stream);
 }
 
-// Entries of the large-Gaussian queue of the fused walk (at most 2^18).
+// Entries of each of the fused walk's two queues (at most 2^18), and of both.
 uint32_t queue_capacity(const uint32_t n) { return n < (1u << 18) ? n : (1u << 18); }
+uint32_t queue_slots(const uint32_t n) { return n < (1u << 19) ? n : (1u << 19); }
 constexpr size_t kWalkGaussianBytes = 128;  // walk constants (96) and GPS constants (32)
 
 // Backward workspace: colours (3 per Gaussian, padded to 4), accumulators (10 per Gaussian), then
-// the fused walk's queue (header, entries, meta, indices), each section 256-byte aligned.
+// the fused walk's queues (two headers, the entries of both, meta of one after the other, the entries' indices), each
+// section 256-byte aligned.
 struct BackwardLayout {
     size_t colors, accum, queue, entries, meta, index, total;
 };
 
 BackwardLayout backward_layout(const uint32_t n) {
     BackwardLayout L{};
-    const size_t cap = queue_capacity(n);
+    const size_t cap = queue_capacity(n), slots = queue_slots(n);
     L.colors = 0;
     L.accum = align256(sizeof(float) * ((3 * static_cast<size_t>(n) + 3) & ~size_t(3)));
     L.queue = L.accum + align256(sizeof(double) * kAccumSums * n);
-    L.entries = L.queue + align256(sizeof(WorkQueue));
-    L.meta = L.entries + align256(kWalkGaussianBytes * cap);
-    L.index = L.meta + align256(sizeof(uint4) * cap);
-    L.total = L.index + align256(sizeof(uint32_t) * cap);
+    L.entries = L.queue + align256(2 * sizeof(WorkQueue));
+    L.meta = L.entries + align256(kWalkGaussianBytes * slots);
+    L.index = L.meta + align256(2 * sizeof(uint4) * cap);
+    L.total = L.index + align256(sizeof(uint32_t) * slots);
     return L;
 }
 
@@ -125,6 +127,7 @@ void set_backward_buffers(BackwardParams& p, void* backward_workspace) {
     p.bw_meta = reinterpret_cast<uint4*>(base + L.meta);
     p.bw_index = reinterpret_cast<uint32_t*>(base + L.index);
     p.bw_capacity = queue_capacity(p.n);
+    p.bw_slots = queue_slots(p.n);
 }
 
 }  // namespace
@@ -241,7 +244,7 @@ int sgs_backward_accumulate_samples(const sgs_gaussians* gaussians, const sgs_ca
         err = cudaMemsetAsync(p.accum, 0, kAccumSums * p.n * sizeof(double), stream);
         if (err == cudaSuccess) err = launch_backward_colors(p, stream);
     }
-    if (err == cudaSuccess) err = cudaMemsetAsync(p.bw_queue, 0, sizeof(WorkQueue), stream);
+    if (err == cudaSuccess) err = cudaMemsetAsync(p.bw_queue, 0, 2 * sizeof(WorkQueue), stream);
     if (err == cudaSuccess) {
         int device = 0;
         err = cudaGetDevice(&device);
@@ -280,7 +283,7 @@ int sgs_backward_accumulate_framebuffers(const sgs_gaussians* gaussians, const s
     if (first) err = cudaMemsetAsync(p.accum, 0, kAccumSums * p.n * sizeof(double), stream);
     if (err == cudaSuccess) err = launch_backward_colors(p, stream);
     if (err == cudaSuccess) err = launch_backward_framebuffer_terms(p, stream);
-    if (err == cudaSuccess) err = cudaMemsetAsync(p.bw_queue, 0, sizeof(WorkQueue), stream);
+    if (err == cudaSuccess) err = cudaMemsetAsync(p.bw_queue, 0, 2 * sizeof(WorkQueue), stream);
     if (err == cudaSuccess) {
         int device = 0;
         err = cudaGetDevice(&device);

@@ -29,7 +29,8 @@ constexpr uint32_t kWarpsPerBlock = kBlock / 32;
 constexpr uint32_t kProjectionBlock = 128;
 constexpr uint32_t kFullMask = 0xffffffffu;
 constexpr uint32_t kCoopFragments = 64;  // larger AABBs are processed by the whole warp
-constexpr uint32_t kBigFragments = 256;   // fused walk: larger AABBs go to the row-chunk queue
+constexpr uint32_t kBigFragments = 256;   // fused walk: larger AABBs go to a row-chunk queue,
+constexpr uint32_t kHugeFragments = 2048;  // those above this one to a queue of their own
 constexpr uint32_t kMaxLaneTiles = 16;    // AABBs of at most this many tiles are tested by their lane
 constexpr uint32_t kChunkPixels = 2048;   // pixels per stolen chunk (whole rows, at most 32)
 constexpr uint32_t kQueueBlocksPerSM = 8;
@@ -499,6 +500,12 @@ struct WalkEntry {
 };
 static_assert(sizeof(WalkEntry) == 128, "the backward workspace reserves 128 bytes per queue entry");
 
+// Place of entry e of queue k (0: huge, 1: large footprints): the two queues grow from the ends of one array. They hold
+// min(N, 2^18) entries each, together at most N, and the array min(N, 2^19).
+__device__ __forceinline__ uint32_t walk_slot(const BackwardParams& b, const uint32_t k, const uint32_t e) {
+    return k == 0 ? e : b.bw_slots - 1u - e;
+}
+
 // Lane walks the span of row y of Gaussian q (when valid), one pixel per step, and adds the S
 // samples' fragment gradients to acc. kGps: the fragment probability is the GPS hit probability
 // (constants gc) instead of alpha.
@@ -655,21 +662,32 @@ __global__ void __launch_bounds__(walk_block(kGps)) fragments_samples_kernel(con
         }
         if (lane == src && !front) has_rows = false;
     }
-    // large footprints go to the queue (walked in row chunks across all SMs) unless it is full; one atomic per warp
-    const bool large = has_rows && rect.width * rect.height > kBigFragments;
+    // large footprints go to a queue (walked in row chunks across all SMs) unless it is full; one atomic per warp and
+    // queue. The huge ones have their own: where they found one queue full of smaller ones, their warps walked many
+    // thousand pixels alone (2M faint Gaussians at 1080p, 2000 of them huge, backward of 8 samples: 31.3 ms with one
+    // queue for all above 256 pixels, 11.9 for those above 2048, 11.1 with both; 1M without: 13.8, 8.8 and 8.1 ms).
+    const uint32_t pixels = has_rows ? rect.width * rect.height : 0u;
+    const bool huge = pixels > kHugeFragments;
     const uint32_t log_rpc = log_chunk_rows(rect.width);
-    const uint32_t chunks = large ? (rect.height + (1u << log_rpc) - 1u) >> log_rpc : 0u;
-    const uint32_t larges = __ballot_sync(kFullMask, large);
     uint32_t entry_at = 0xffffffffu;
+    uint32_t chunks = 0;
     unsigned long long first_chunk = 0;
-    if (larges != 0) {
-        const uint32_t incl = warp_inclusive_sum(chunks, lane);
+#pragma unroll
+    for (uint32_t k = 0; k < 2; ++k) {
+        const bool mine = pixels > kBigFragments && huge == (k == 0);
+        const uint32_t all = __ballot_sync(kFullMask, mine);
+        if (all == 0) continue;
+        const uint32_t own = mine ? (rect.height + (1u << log_rpc) - 1u) >> log_rpc : 0u;
+        const uint32_t incl = warp_inclusive_sum(own, lane);
         unsigned long long old = 0;
         if (lane == 31)
-            old = atomicAdd(&b.bw_queue->packed, (static_cast<unsigned long long>(__popc(larges)) << kQueueEntryShift) | incl);
+            old = atomicAdd(&b.bw_queue[k].packed, (static_cast<unsigned long long>(__popc(all)) << kQueueEntryShift) | incl);
         old = __shfl_sync(kFullMask, old, 31);
-        if (large) entry_at = static_cast<uint32_t>(old >> kQueueEntryShift) + __popc(larges & lt_mask);
-        first_chunk = (old & kQueueChunkMask) + (incl - chunks);
+        if (mine) {
+            entry_at = static_cast<uint32_t>(old >> kQueueEntryShift) + __popc(all & lt_mask);
+            chunks = own;
+            first_chunk = (old & kQueueChunkMask) + (incl - own);
+        }
     }
     WalkGaussian q;
     GpsConstants c{};
@@ -698,16 +716,18 @@ __global__ void __launch_bounds__(walk_block(kGps)) fragments_samples_kernel(con
         q.w = rect.width;
         q.row_first = 0;
         if (entry_at < b.bw_capacity) {
+            uint4* const meta = b.bw_meta + (huge ? 0u : b.bw_capacity) + entry_at;
             if (first_chunk + chunks <= kMaxQueueChunks) {
-                WalkEntry* entry = static_cast<WalkEntry*>(b.bw_entries) + entry_at;
+                const uint32_t at = walk_slot(b, huge ? 0u : 1u, entry_at);
+                WalkEntry* entry = static_cast<WalkEntry*>(b.bw_entries) + at;
                 entry->g = q;
                 if (kGps) entry->c = c;
-                b.bw_meta[entry_at] = make_uint4(rect.y_min, rect.height, log_rpc, static_cast<uint32_t>(first_chunk));
-                b.bw_index[entry_at] = g;
+                *meta = make_uint4(rect.y_min, rect.height, log_rpc, static_cast<uint32_t>(first_chunk));
+                b.bw_index[at] = g;
                 has_rows = false;
             } else {
                 // past 32-bit chunk indices: marked unused (the marked entries are the last ones), walked here
-                b.bw_meta[entry_at] = make_uint4(0u, 0u, 0u, kUnusedQueueEntry);
+                *meta = make_uint4(0u, 0u, 0u, kUnusedQueueEntry);
             }
         }
     }
@@ -752,37 +772,49 @@ __global__ void __launch_bounds__(walk_block(kGps)) fragments_samples_kernel(con
     }
 }
 
-// Persistent consumer of the fused walk's large-Gaussian queue: each warp steals one chunk of rows
+// Persistent consumer of the fused walk's queues, the huge footprints first: each warp steals one chunk of rows
 // (R rows, each split into 32 / R lane segments), sums the lanes' gradients and adds them to the
 // Gaussian's accumulators.
 template <bool kGps>
 __global__ void __launch_bounds__(kBlock) fragments_samples_queue_kernel(const BackwardParams b,
                                                                          const float2* __restrict__ law) {
     const uint32_t lane = threadIdx.x & 31u;
-    const unsigned long long packed = b.bw_queue->packed;
-    const uint32_t n_entries =
-        static_cast<uint32_t>(min(packed >> kQueueEntryShift, static_cast<unsigned long long>(b.bw_capacity)));
-    if (n_entries == 0) return;
-    uint32_t last_entry = n_entries - 1;  // the last used entry; entry 0 starts at chunk 0 and always is
-    if (b.bw_meta[last_entry].w == kUnusedQueueEntry)
-        last_entry = queue_entry_of_chunk(b.bw_meta, n_entries, kUnusedQueueEntry - 1u, lane);
-    const uint4 last = b.bw_meta[last_entry];
-    const uint32_t n_chunks = last.w + ((last.y + (1u << last.z) - 1u) >> last.z);
     const WalkEntry* entries = static_cast<const WalkEntry*>(b.bw_entries);
+    uint32_t k = 0, n_entries = 0, n_chunks = 0;
+    // the used entries and the chunks of queue k
+    auto open_queue = [&] {
+        const uint4* const meta = b.bw_meta + k * b.bw_capacity;
+        n_entries = static_cast<uint32_t>(
+            min(b.bw_queue[k].packed >> kQueueEntryShift, static_cast<unsigned long long>(b.bw_capacity)));
+        n_chunks = 0;
+        if (n_entries == 0) return;
+        uint32_t last_entry = n_entries - 1;  // the last used entry; entry 0 starts at chunk 0 and always is
+        if (meta[last_entry].w == kUnusedQueueEntry)
+            last_entry = queue_entry_of_chunk(meta, n_entries, kUnusedQueueEntry - 1u, lane);
+        const uint4 last = meta[last_entry];
+        n_chunks = last.w + ((last.y + (1u << last.z) - 1u) >> last.z);
+    };
+    open_queue();
     for (;;) {
         uint32_t c = 0;
-        if (lane == 0) c = atomicAdd(&b.bw_queue->next_chunk, 1u);
+        if (lane == 0 && n_chunks != 0) c = atomicAdd(&b.bw_queue[k].next_chunk, 1u);
         c = __shfl_sync(kFullMask, c, 0);
-        if (c >= n_chunks) break;
-        const uint32_t lo = queue_entry_of_chunk(b.bw_meta, n_entries, c, lane);
-        const uint4 m = b.bw_meta[lo];
+        if (c >= n_chunks) {
+            if (++k == 2u) break;
+            open_queue();
+            continue;
+        }
+        const uint4* const meta = b.bw_meta + k * b.bw_capacity;
+        const uint32_t lo = queue_entry_of_chunk(meta, n_entries, c, lane);
+        const uint4 m = meta[lo];
+        const uint32_t at = walk_slot(b, k, lo);
         const uint32_t log_rows = m.z;
         const uint32_t r0 = (c - m.w) << log_rows;
         if (r0 >= m.y || log_rows > 5u) {
-            if (lane == 0) atomicOr(&b.bw_queue->error, 1u);
+            if (lane == 0) atomicOr(&b.bw_queue[k].error, 1u);
             continue;
         }
-        const WalkGaussian q = entries[lo].g;
+        const WalkGaussian q = entries[at].g;
         // the chunk's tiles, one per lane: behind the winners of all of them nothing is added
         const uint32_t rows = min(1u << log_rows, m.y - r0);
         const uint32_t tx0 = q.x_min / kBoundTile, tw = (q.x_min + q.w - 1u) / kBoundTile - tx0 + 1u;
@@ -793,13 +825,13 @@ __global__ void __launch_bounds__(kBlock) fragments_samples_queue_kernel(const B
             front = __ldg(b.tile_far + (ty0 + ty) * b.tiles_x + tx0 + (t - ty * tw)) >= q.key_hi;
         }
         if (!__any_sync(kFullMask, front)) continue;
-        const GpsConstants gc = kGps ? entries[lo].c : GpsConstants{};
+        const GpsConstants gc = kGps ? entries[at].c : GpsConstants{};
         const uint32_t r = r0 + (lane & ((1u << log_rows) - 1u));
         FragAccum acc;
 #pragma unroll
         for (int i = 0; i < kAccum; ++i) acc.v[i] = 0.0;
         walk_row_gradients<kGps>(b, q, gc, law, r < m.y, q.y_min + r, acc, lane >> log_rows, 5u - log_rows);
-        double* out = b.accum + static_cast<size_t>(b.bw_index[lo]) * kAccum;
+        double* out = b.accum + static_cast<size_t>(b.bw_index[at]) * kAccum;
 #pragma unroll
         for (int i = 0; i < kAccum; ++i) {
             double v = acc.v[i];

@@ -318,12 +318,12 @@ struct BackwardParams {
     uint32_t* pix_far;                       // per pixel, the largest depth bits of the samples' winners
     uint32_t* tile_far;                      // per 8 x 8 tile, the largest of those
     uint32_t tiles_x, tiles_y;
-    // queue of Gaussians with large footprints, walked in row chunks by a persistent kernel
-    WorkQueue* bw_queue;
-    void* bw_entries;                        // WalkGaussian per entry (backward_st.cu)
-    uint4* bw_meta;                          // y_min, height, log2 rows per chunk, first chunk
-    uint32_t* bw_index;                      // Gaussian index per entry
-    uint32_t bw_capacity;
+    // queues of Gaussians with huge and with large footprints, walked in row chunks by a persistent kernel
+    WorkQueue* bw_queue;                     // two
+    void* bw_entries;                        // WalkEntry per place (backward_st.cu), bw_slots in all
+    uint4* bw_meta;                          // per queue bw_capacity: y_min, height, log2 rows per chunk, first chunk
+    uint32_t* bw_index;                      // Gaussian index per place
+    uint32_t bw_capacity, bw_slots;
     int num_sms;
     uint32_t n_samples;                      // S
     uint32_t sample;                         // the sample whose terms sample_terms writes
