@@ -332,7 +332,8 @@ int sgs_denoise(const void* features, int32_t batch, int32_t height, int32_t wid
  * (FP16 [batch][height][width][8]) give `output` (FP32 [batch][height][width][3]), and `saved` keeps what the
  * backward needs. Backward: `weights` holds the 6 device pointers of the weights; `grads` receives
  * sgs_denoise_train_params() floats, the gradients of W1, b1, ..., W6, b6 back to back. Buffers are
- * 16-byte aligned; the same bits as the layers through sgs_conv3x3. */
+ * 16-byte aligned. The output has the same bits as the layers through sgs_conv3x3; the gradients are sums over
+ * thread blocks in any order, equal to rounding from one call to the next. */
 size_t sgs_denoise_train_params(void);
 size_t sgs_denoise_train_saved_size(int32_t batch, int32_t height, int32_t width);
 size_t sgs_denoise_train_scratch_size(int32_t batch, int32_t height, int32_t width);
@@ -353,9 +354,9 @@ int sgs_denoise_status(void* stream);
 void sgs_set_stage_events(void* accumulate_start, void* accumulate_end);
 
 /* Diagnostics (no counterpart in the reference): caps the stochastic-transparency large-Gaussian
- * work queue at `max_entries` entries (0 restores the default, min(N, 2^18)) for the workspace
- * sizes and renders that follow, process-wide. Gaussians that find the queue full are rendered in
- * place by their warp (same framebuffer); tests use a small cap to exercise that path. */
+ * work queue at `max_entries` entries (0 restores the default: what the workspace's sections hold, at
+ * least 15/16 of min(N, 2^18), at most min(N, 2^20 - 1)) for the workspace sizes and renders that
+ * follow, process-wide. Gaussians that find the queue full are rendered in place by their warp (same framebuffer); tests use a small cap to exercise that path. */
 void sgs_set_queue_limit(uint32_t max_entries);
 
 /* Preactivated layout (README.md:139-142 of the reference lists it as a possible improvement): writes,

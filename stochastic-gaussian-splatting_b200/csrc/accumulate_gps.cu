@@ -16,7 +16,7 @@
 //
 // Deep scenes of millions of Gaussians run front to back and skip whole groups of 32 that lie behind their
 // tiles' bounds (sgs_front.cuh; single Gaussians could not be left out, as the lanes' streams run through
-// them). 6M Gaussians at 1080p: 323 to 302 us a sample, 1860 to 1386 us for 8; the groups left are bound by
+// them). 6M Gaussians at 1080p: 323 to 293 us a sample, 1860 to 1372 us for 8; the groups left are bound by
 // instruction issue like the pass as a whole.
 //
 // Hybrid scheduling bins the Gaussians with more than 512 points (up to max_binned of them) into
@@ -389,6 +389,7 @@ __device__ __forceinline__ void consume_chunks(const AccumulateParams& a) {
     }
 }
 
+// (8 blocks per SM spill 8 bytes: 3200 us per sample of the progressive benchmark, as with 6 and none.)
 __global__ void __launch_bounds__(kBlock, kChunkBlocksPerSM) gps_chunks_kernel(const AccumulateParams a) {
     wait_for_pass_before();
     if (a.stq.list != nullptr && a.queue->st_listed != kNotListed) return;  // gps_queue_kernel takes the items

@@ -23,7 +23,7 @@
 //    off the ellipse, and the warp walks the rest, two pixels per lane, lowering the bounds with the
 //    keys it reads. Keys only decrease during a pass, so a dropped fragment could not have won;
 //  * deep scenes of millions of Gaussians run front to back (sgs_front.cuh): the pass drops the groups and
-//    the Gaussians that lie behind their tiles' bounds (6M at 1080p: 580 us a sample to 415, 275 million
+//    the Gaussians that lie behind their tiles' bounds (6M at 1080p: 577 us a sample to 399, 283 million
 //    warp instructions instead of 469; half of the rows are left, and their walk is what bounds it);
 //  * u64 atomicMin (fire-and-forget RED) on the L2-resident framebuffer.
 //
@@ -445,6 +445,10 @@ __device__ __forceinline__ uint32_t queued_above(const AccumulateParams& a, cons
 enum ScatterMode { kPlain, kSplitRows, kFrontToBack };
 
 // One thread per Gaussian (accumulate_scatter.cu:19-77 for the projection and the AABB).
+// Held to as many blocks as leave 64 registers (front to back and one sample: 56), at the price of some spills; with
+// the registers that need none fewer warps hide the latencies. Per call with spills and without: split rows and 8
+// samples, 30k Gaussians at 640x480, 671 and 693 us, hybrid with blue noise, 100k, 1103 and 1114; front to back, 6M at
+// 1920x1080, 398 and 409 us (8 bytes), hybrid 404 and 422 (32), blue noise 433 and 441 (24), both 436 and 449 (68).
 template <bool kBlue, bool kHybrid, bool kMulti, ScatterMode kMode>
 __global__ void __launch_bounds__(kMode == kFrontToBack ? kOrderedWarps * 32u : kBlock,
                                   kMode == kFrontToBack ? (kMulti ? 32u : 36u) / kOrderedWarps : 4u)
@@ -716,6 +720,9 @@ __global__ void __launch_bounds__(kOrderBlock) order_kernel(const AccumulatePara
 // end to end and compares 32 quads of tile bounds at a time, one 16-byte load per lane; the tiles in
 // front of their bounds are tested against the ellipse, one per lane, and those that remain are
 // walked, the next tile's keys read ahead. Short queues are dealt out in pieces of items.
+// Four blocks per SM spill up to 32 bytes where three would not: 500k training Gaussians, 800x800, 8 samples, 1142 us
+// per call with four, 1161 with three; hybrid 400k heavy-tailed ones at 1279x719, one sample 436 and 466, 4 samples 1015
+// and 970.
 template <bool kBlue, bool kHybrid, bool kMulti>
 __global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) st_queue_kernel(const AccumulateParams a) {
     __shared__ RowGaussian s_gauss[kWarpsPerBlock][32];

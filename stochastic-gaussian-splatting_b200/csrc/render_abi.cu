@@ -76,11 +76,11 @@ struct Derived {
 // then takes the Gaussians as they lie 1 to 2 % (Gaussian point splatting 5 %, as it has less to do per Gaussian), so
 // that few Gaussians, or few per pixel, are not prepared for it; below some 2.5M most of them are in flight before
 // the first bounds exist. As they lie against front to back, in us, the 6M scene cut to n Gaussians:
-//   one sample: 2.2M 1920x1080 (coverage 49) 264, 287, 1280x720 (55) 200, 196; 3M 1920x1080 (66) 330, 324,
-//     3840x2160 (44) 695, 737, 1280x720 (75) 253, 222; 6M 1920x1080 (133) 577, 415, 3840x2160 (87) 1187, 1000
+//   one sample: 2.2M 1920x1080 (coverage 49) 264, 287, 1280x720 (55) 200, 196; 3M 1920x1080 (66) 330, 310,
+//     3840x2160 (44) 695, 737, 1280x720 (75) 253, 208; 6M 1920x1080 (133) 577, 399, 3840x2160 (87) 1187, 978
 //   one sample of point splatting: 4M 1920x1080 (88) 239, 258, 1280x720 (100) 185, 183; 6M 3840x2160 (87) 615, 638,
-//     1920x1080 (133) 323, 305, 1280x720 (150) 255, 223
-//   8 samples: 2.2M 1280x720 738, 666; 6M 1920x1080 2402, 1569; of point splatting 628, 611 and 1860, 1386
+//     1920x1080 (133) 323, 293, 1280x720 (150) 255, 209
+//   8 samples: 2.2M 1280x720 738, 650; 6M 1920x1080 2402, 1533; of point splatting 628, 600 and 1860, 1372
 constexpr float kFrontCoverage = 58.0f, kFrontCoverageGps = 110.0f;
 
 bool may_run_front_to_back(const Derived& d, const bool gps, const uint32_t n_samples) {

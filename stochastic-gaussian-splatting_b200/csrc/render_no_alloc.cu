@@ -24,8 +24,8 @@
 //    streams or threads without ordering) race on the array and must be serialised by the caller;
 //  * requests whose scratch exceeds kScratchBytes are rejected with SGS_ERROR_WORKSPACE before any
 //    launch. Stochastic transparency at 1920x1080 without supersampling or spatial reuse fits for
-//    any scene size: at most 66.6 MB (framebuffer 16.6 MB, samples 33.2 MB, a work queue whose own
-//    entries fill the rest, at least min(N, 2^18) of 64 bytes, 16.8 MB). Hybrid GPS sizes its work queue by max_binned
+//    any scene size: at most these 67.1 MB (framebuffer 16.6 MB, samples 33.2 MB, a work queue whose own
+//    entries of 64 bytes fill the rest, at least 15/16 of min(N, 2^18), 15.7 MB). Hybrid GPS sizes its work queue by max_binned
 //    instead (by default min(N, 2^20) entries of 60 bytes): at 1920x1080 it fits up to about
 //    289,000 entries, so scenes with more Gaussians need settings->max_binned at or below that.
 // No cudaMalloc, cudaFree or allocating library routine is called.

@@ -43,7 +43,7 @@ constexpr unsigned long long kMaxQueueChunks = 0xffffffffull - (1ull << 24);
 constexpr uint32_t kUnusedQueueEntry = 0xffffffffu;
 
 // Scratch of the allocation-free render (render_no_alloc.cu). The stochastic-transparency queue takes
-// more than its 2^18 entries only while a one-sample workspace stays within it.
+// more than 15/16 of 2^18 entries only while a one-sample workspace stays within it.
 constexpr size_t kNoAllocScratchBytes = size_t(64) << 20;
 
 // ---- queues in depth order, depth bounds per tile (stochastic transparency; binned GPS Gaussians) ----
@@ -86,7 +86,8 @@ constexpr uint32_t kSliceGroups = 1024;  // groups per slice, at most
 constexpr uint32_t kGroupBuckets = 1024;  // 1/64 octave each over view depths of 2^-4 .. 2^12
 constexpr int kGroupShift = 17;           // depth bits below a bucket's
 // Warps per block of a front-to-back pass: many of its warps end early, and a block keeps its place until its last
-// warp has ended (8 warps a block: 478 us where 2 take 437 on 6M Gaussians at 1080p; fewer make more blocks to start).
+// warp has ended (6M Gaussians at 1080p: 426 us with 8 warps a block, 399 with 4, 399 with 2; point splatting 305, 293
+// and 294).
 constexpr uint32_t kOrderedWarps = 4;
 struct GroupOrder {
     uint32_t* order;          // groups front to back; null: the pass takes them as they come
