@@ -929,7 +929,10 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
             active) {
             const PixelRect rect = pixel_rect(p.bounds, a.cam);
             own = static_cast<float>(rect.width) * static_cast<float>(rect.height);
-            pixels = fminf(own * static_cast<float>(step), kSampleMaxCover * a.cam.width * a.cam.height);
+            // a faint Gaussian hides little of what lies behind it; the weight is 1 in the mean over scenes whose opacity
+            // logits are N(0, 2^2)
+            pixels = fminf(2.5f * p.opacity, 1.25f) *
+                     fminf(own * static_cast<float>(step), kSampleMaxCover * a.cam.width * a.cam.height);
             larger = own > static_cast<float>(kDenseMinPixels) ? pixels : 0.0f;
             if (!compact) pixels = 0.0f;
         }

@@ -32,12 +32,14 @@ std::atomic<uint32_t> g_queue_limit{0};
 constexpr size_t kAlign = 256;
 constexpr uint32_t kDefaultMaxBinned = 1u << 20;     // accumulate_hybrid_gps.cu:22
 constexpr uint32_t kStQueueCapacity = 1u << 18;       // ST queue entries with space of their own
-// Coverage by larger Gaussians (AABB pixels over framebuffer pixels) above which a scene counts as dense
+// Coverage by larger Gaussians (AABB pixels, weighted by opacity, over framebuffer pixels) above which a scene counts as dense
 // (accumulate_st.cu). Sparse against dense, in us: the training scene at 800x800 with 60k Gaussians
 // (coverage 255) 197, 223, with 120k (514) 339, 252; the 100k scene at 640x480 (64) 82, 129, with 400k (259)
 // 193, 213, with 800k (484) 312, 287; heavy-tailed at 1279x719 with 20k (277) 257, 292, with 40k (550) 415,
-// 364; the 6M scene at 1280x720 (6) 455, 481.
-constexpr float kDenseCoverage = 420.0f;
+// 364; the 6M scene at 1280x720 (6) 455, 481. Fainter ones, logits -2, -3, -4 on average: 500k training Gaussians at
+// 800x800, 8 samples (375) 2740, 2061, (173) 2134, 2647; 400k heavy-tailed at 1279x719 (755) 838, 515, (430) 644, 615,
+// (202) 465, 673; 750k at 1817x1616 (415) 3081, 2169, (180) 2104, 2471.
+constexpr float kDenseCoverage = 350.0f;
 constexpr uint32_t kMinOrdered = 8192;                // Gaussians of a scene whose queue may be ordered
 constexpr uint32_t kMaxSamplesPerCall = 1024;         // sgs_render_samples
 constexpr int kMaxDevices = 64;
@@ -80,6 +82,7 @@ struct Derived {
 //     3840x2160 (44) 695, 737, 1280x720 (75) 253, 208; 6M 1920x1080 (133) 577, 399, 3840x2160 (87) 1187, 978
 //   one sample of point splatting: 4M 1920x1080 (88) 239, 258, 1280x720 (100) 185, 183; 6M 3840x2160 (87) 615, 638,
 //     1920x1080 (133) 323, 293, 1280x720 (150) 255, 209
+//   faint ones, logits -2 and -3 on average, 6M 1920x1080 (48) 471, 533, (18) 416, 506; 8 samples 1862, 1931, 1540, 1632
 //   8 samples: 2.2M 1280x720 738, 650; 6M 1920x1080 2402, 1533; of point splatting 628, 600 and 1860, 1372
 constexpr float kFrontCoverage = 58.0f, kFrontCoverageGps = 110.0f;
 

@@ -26,8 +26,8 @@ struct WorkQueue {
     unsigned int st_entries;     // ST: entries and list items reserved by producers
     unsigned int st_items;
     unsigned int st_listed;      // items the order pass has listed (GPS: or kNotListed)
-    alignas(16) float covered[4];      // AABB pixels of the scene's larger Gaussians, estimated by kSampleBlocks
-                                       // blocks of the clear pass
+    alignas(16) float covered[4];      // AABB pixels of the scene's larger Gaussians, weighted by opacity, estimated by
+                                       // kSampleBlocks blocks of the clear pass
     alignas(16) float covered_all[4];  // the same of all its Gaussians (GPS: of those in compact groups)
     alignas(16) float larger[kQueueSteps][4];  // Gaussians with AABBs above kDenseMinPixels << step, estimated likewise
 };

@@ -1,0 +1,39 @@
+"""What the coverage estimate of the clear pass leaves to the passes in depth order (WorkQueue::covered, covered_all).
+
+Faint Gaussians hide little, however much they cover: their scenes are drawn as they lie, whatever the footprints.
+"""
+import numpy as np
+import pytest
+
+import sgs_scenes
+from oracle import cpu
+from test_gpu_front_dispatch import HEIGHT, WIDTH, covered_all, render
+from test_gpu_front_to_back import deep_scene
+from test_gpu_schedule import KEYS, cam_dict
+from test_gpu_st_queue import dense_scene
+from test_gpu_st_queue_sizes import call
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shift,ordered", [(0.0, True), (-5.0, False)])
+def test_queues_of_faint_scenes_are_not_ordered(shift, ordered, cuda_device):
+    scene = dense_scene(20_000, -2.0)
+    scene.opacities += shift
+    cam = sgs_scenes.front_camera(321, 181)
+    fb, entries, items, listed, _ = call(scene.to(cuda_device), cam)
+    assert items > 1000 and (listed > 0) == ordered
+    want = cpu.accumulate({k: t.numpy() for k, t in zip(KEYS, scene.tensors())}, cam_dict(cam),
+                          dict(aa=False, ss=1, gps=False, hybrid=False), 40)
+    assert float((fb == want).mean()) >= 0.9999
+    assert np.unique(fb).size > 1
+
+
+@pytest.mark.parametrize("gps", [False, True])
+def test_deep_faint_scenes_are_drawn_as_they_lie(gps, cuda_device):
+    estimates = []
+    for shift in (0.0, -5.0):
+        scene = deep_scene((1 << 21) + 45, -5.0)
+        scene.opacities += shift
+        estimates.append(covered_all(render(scene.to(cuda_device).tensors(), cuda_device, samples=2, mode=1, gps=gps)[2]))
+    assert estimates[0] > 58 * WIDTH * HEIGHT > estimates[1] > 0
