@@ -40,6 +40,10 @@ constexpr uint32_t kStQueueCapacity = 1u << 18;       // ST queue entries with s
 // 800x800, 8 samples (375) 2740, 2061, (173) 2134, 2647; 400k heavy-tailed at 1279x719 (755) 838, 515, (430) 644, 615,
 // (202) 465, 673; 750k at 1817x1616 (415) 3081, 2169, (180) 2104, 2471.
 constexpr float kDenseCoverage = 350.0f;
+// and covered pixels below which it does not in any case: the order and its passes' latency take some 30 us, and tiles of
+// a small image are few. 160x120, 30k (16 million) 52, 113, 100k (56) 91, 154, 400k (199) 291, 321; 96x72, 400k (52)
+// 150, 209; 240x180, 1.5M (20) 193, 245, 100k (129) 161, 159; 480x360, 30k (142) 167, 117, 100k (500) 490, 173.
+constexpr float kDensePixels = 137.0e6f;
 constexpr uint32_t kMinOrdered = 8192;                // Gaussians of a scene whose queue may be ordered
 constexpr uint32_t kMaxSamplesPerCall = 1024;         // sgs_render_samples
 constexpr int kMaxDevices = 64;
@@ -405,8 +409,9 @@ int render_on_streams(const sgs_gaussians* g, const sgs_camera* c, const sgs_set
         stq.entries_a = F.st_own;
         stq.capacity = F.st_capacity;
         // a queue of a few thousand entries is not worth the order pass's launch
-        stq.dense_pixels = g->n_gaussians < kMinOrdered ? std::numeric_limits<float>::infinity()
-                                                        : kDenseCoverage * static_cast<float>(d.n_fb);
+        stq.dense_pixels = g->n_gaussians < kMinOrdered
+                               ? std::numeric_limits<float>::infinity()
+                               : std::max(kDenseCoverage * static_cast<float>(d.n_fb), kDensePixels);
         // Few Gaussians leave the chip idle while single warps walk the rows of 32 large ones: 2^split
         // warps share them (640x480, 100k: 117 to 93 us; 640x480 training scene of 30k, 8 samples: 1012 to
         // 785 us). From 256k up the repeated projections cost more than that gains. Hybrid scheduling

@@ -1,6 +1,7 @@
 """What the coverage estimate of the clear pass leaves to the passes in depth order (WorkQueue::covered, covered_all).
 
-Faint Gaussians hide little, however much they cover: their scenes are drawn as they lie, whatever the footprints.
+Faint Gaussians hide little, however much they cover: their scenes are drawn as they lie, whatever the footprints. So are
+scenes of few covered pixels, for which the order takes longer than it saves: in small images however dense.
 """
 import numpy as np
 import pytest
@@ -16,11 +17,13 @@ from test_gpu_st_queue_sizes import call
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("shift,ordered", [(0.0, True), (-5.0, False)])
-def test_queues_of_faint_scenes_are_not_ordered(shift, ordered, cuda_device):
-    scene = dense_scene(20_000, -2.0)
+@pytest.mark.parametrize("n,shift,width,height,ordered", [
+    (60_000, 0.0, 321, 181, True), (60_000, -5.0, 321, 181, False), (9_000, 0.0, 321, 181, False), (120_000, 0.0, 81, 46, False),
+    (100_000, 0.0, 500, 280, True)])
+def test_queues_of_faint_and_small_scenes_are_not_ordered(n, shift, width, height, ordered, cuda_device):
+    scene = dense_scene(n, -2.0)
     scene.opacities += shift
-    cam = sgs_scenes.front_camera(321, 181)
+    cam = sgs_scenes.front_camera(width, height)
     fb, entries, items, listed, _ = call(scene.to(cuda_device), cam)
     assert items > 1000 and (listed > 0) == ordered
     want = cpu.accumulate({k: t.numpy() for k, t in zip(KEYS, scene.tensors())}, cam_dict(cam),

@@ -3,7 +3,7 @@
 The clear pass estimates how many AABBs lie above 256, 512 and 1024 pixels (WorkQueue::larger), and the scatter pass
 queues those above the first of these sizes that fit, else those above 2048. The framebuffers must be the same
 bit for bit, also at image sizes below a tile, a quad and a claim's worth of items. (Scenes of fewer than 8192
-Gaussians are never dense.)
+Gaussians, or of fewer than 137 million covered pixels, are never dense.)
 """
 import numpy as np
 import pytest
@@ -41,8 +41,8 @@ def call(scene, cam, samples=1, **flags):
 def test_every_size_gives_the_same(samples, cuda_device):
     from StochasticGSCudaBackend import _C
 
-    scene = dense_scene(40_000, -2.5).to(cuda_device)
-    cam = sgs_scenes.front_camera(321, 181)
+    scene = dense_scene(150_000, -2.6).to(cuda_device)
+    cam = sgs_scenes.front_camera(450, 253)
     fb, entries, items, listed, larger = call(scene, cam, samples)
     assert larger[0] > larger[1] > larger[2] > 1000 and listed > 0
     queued = [entries]
@@ -58,12 +58,14 @@ def test_every_size_gives_the_same(samples, cuda_device):
     assert queued == sorted(queued, reverse=True) and len(set(queued)) == 4
 
 
-@pytest.mark.parametrize("width,height,hybrid", [(7, 5, False), (8, 8, False), (31, 9, True), (33, 65, False), (257, 131, True)])
-def test_dense_scenes_at_the_edges_of_tiles(width, height, hybrid, cuda_device):
-    """The depth-ordered queue: at least 8192 Gaussians, all of them large, and its items listed."""
-    scene = sgs_scenes.make_scene(sgs_scenes.SceneSpec(n=9000, log_scale_mean=1.0, log_scale_std=0.8), seed=11)
-    if width > 100:
-        scene = dense_scene(9000, -1.5)
+@pytest.mark.parametrize("width,height,hybrid,n", [(7, 5, False, 9000), (8, 8, False, 9000), (127, 57, True, 100_000),
+                                                   (33, 257, False, 100_000), (257, 131, True, 60_000)])
+def test_dense_scenes_at_the_edges_of_tiles(width, height, hybrid, n, cuda_device):
+    """The depth-ordered queue: most Gaussians are large, and its items listed."""
+    scene = sgs_scenes.make_scene(sgs_scenes.SceneSpec(n=n, log_scale_mean=1.0, log_scale_std=0.8), seed=11)
+    if width > 200:
+        scene = dense_scene(n, -1.5)
+    scene.scales[::5] = -9.0  # (the queue has room for 15 of 16)
     cam = sgs_scenes.front_camera(width, height)
     fb, entries, items, listed, _ = call(scene.to(cuda_device), cam, hybrid=hybrid)
     if width * height > 256:
