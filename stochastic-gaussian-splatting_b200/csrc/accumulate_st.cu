@@ -97,8 +97,9 @@ __device__ __forceinline__ QuadRect quad_rect(const uint32_t x_min, const uint32
     t.h = (y_min + h - 1u) / kBoundTile - t.y0 + 1u;
     return t;
 }
-__device__ __forceinline__ uint32_t part_count(const QuadRect& t) {
-    return min((t.w * t.h + kPartQuads - 1u) / kPartQuads, kMaxParts);
+// scale: log2 of the quads per part over kPartQuads (part_scale).
+__device__ __forceinline__ uint32_t part_count(const QuadRect& t, const uint32_t scale) {
+    return min((t.w * t.h + (kPartQuads << scale) - 1u) / kPartQuads >> scale, kMaxParts);
 }
 
 // Packed FP32x2 arithmetic (sm_100a): two independent round-to-nearest operations per instruction,
@@ -296,7 +297,7 @@ __device__ __forceinline__ bool tile_on_ellipse(const RowGaussian& G, const uint
 
 // Sparse scenes: rows per chunk of a queued Gaussian of AABB width w (about kChunkPixels pixels, a power
 // of two between 1 and 32; each row is walked in 32 / rows segments, so wide footprints keep every lane
-// walking) and chunks per item (one, but for AABBs of more than kMaxParts chunks).
+// walking) and chunks per item (1 << scale, but for AABBs of more than kMaxParts times that).
 __device__ __forceinline__ uint32_t log_chunk_rows(const uint32_t w) {
     const uint32_t rows = max(1u, min(32u, kChunkPixels / max(w, 1u)));
     return 31u - __clz(rows);
@@ -304,11 +305,11 @@ __device__ __forceinline__ uint32_t log_chunk_rows(const uint32_t w) {
 struct RowParts {
     uint32_t log_rows, chunks, per_part, parts;
 };
-__device__ __forceinline__ RowParts row_parts(const uint32_t w, const uint32_t h) {
+__device__ __forceinline__ RowParts row_parts(const uint32_t w, const uint32_t h, const uint32_t scale) {
     RowParts r;
     r.log_rows = log_chunk_rows(w);
     r.chunks = (h + (1u << r.log_rows) - 1u) >> r.log_rows;
-    r.per_part = (r.chunks + kMaxParts - 1u) / kMaxParts;
+    r.per_part = max((r.chunks + kMaxParts - 1u) / kMaxParts, 1u << scale);
     r.parts = (r.chunks + r.per_part - 1u) / r.per_part;
     return r;
 }
@@ -440,6 +441,23 @@ __device__ __forceinline__ uint32_t queued_above(const AccumulateParams& a, cons
     return dense ? kDenseMinPixels << step : kMinPixels;
 }
 
+// How much larger than usual (log2) the parts of queued Gaussians are, so that the list has room for all that the clear pass
+// expects. Gaussians whose parts found the list full were drawn by their own warps (53,000 of up to 3.7 million pixels at
+// 2560x1448, 21,700 of them without a place: 134 ms a sample, 1.9 ms with larger parts).
+__device__ __forceinline__ uint32_t part_scale(const AccumulateParams& a, const bool dense) {
+    auto sum_of = [](const float* const v) {  // (the same in every kernel)
+        const float4 n = *reinterpret_cast<const float4*>(v);
+        return __fadd_rn(__fadd_rn(n.x, n.y), __fadd_rn(n.z, n.w));
+    };
+    const float parts = sum_of(a.queue->parts[dense ? 0 : 1]);
+    const float list = static_cast<float>(a.stq.list_capacity);
+    if (parts <= 0.9f * list) return 0u;
+    const float entries = fminf(sum_of(a.queue->larger[dense ? 0u : kQueueSteps - 1u]), static_cast<float>(a.stq.capacity));
+    // at most 2^12, where no Gaussian has more than four parts
+    const float scale = __fdiv_rn(parts, 0.9f * fmaxf(__fsub_rn(list, entries), 0.25f * list));
+    return 32u - __clz(static_cast<uint32_t>(fminf(scale, 4095.0f)));
+}
+
 // How a scatter pass takes its Gaussians: a warp 32 of them, several warps the same 32 (small scenes), or a warp
 // 32 of them front to back, dropping those behind their tiles' bounds.
 enum ScatterMode { kPlain, kSplitRows, kFrontToBack };
@@ -487,10 +505,11 @@ st_scatter_kernel(const AccumulateParams a) {
     // Loaded while the projection waits for its own loads: after it, the scatter pass over 400k large Gaussians took 73 us
     // instead of 68. Deep scenes are seldom dense and load the sizes only then, after the projection.
     bool dense = false;
-    uint32_t queue_above = kMinPixels;
+    uint32_t queue_above = kMinPixels, scale = 0;
     if (kMode != kFrontToBack) {
         dense = dense_scene(a);
         queue_above = queued_above(a, dense);
+        scale = part_scale(a, dense);
     }
     Projected p;
     if (!project_gaussian(active, g, a.means, a.scales, a.rotations, a.opacities, a.w2c, a.cam, p, a.pre, a.quant)) return;
@@ -556,10 +575,11 @@ st_scatter_kernel(const AccumulateParams a) {
         if (lane == leader) e = atomicAdd(&a.queue->st_entries, static_cast<uint32_t>(__popc(big)));
         e = __shfl_sync(kFullMask, e, leader) + __popc(big & lt_mask);
         const bool fits = want && e < a.stq.capacity;
+        if (kMode == kFrontToBack) scale = part_scale(a, dense);
         const uint32_t parts =
             !fits   ? 0u
-            : dense ? part_count(quad_rect(rect.x_min, rect.width, rect.y_min, rect.height))
-                    : row_parts(rect.width, rect.height).parts;
+            : dense ? part_count(quad_rect(rect.x_min, rect.width, rect.y_min, rect.height), scale)
+                    : row_parts(rect.width, rect.height, scale).parts;
         const uint32_t incl = warp_inclusive_sum(parts, lane);
         uint32_t item = 0;
         if (lane == 31 && incl != 0) item = atomicAdd(&a.queue->st_items, incl);
@@ -685,6 +705,7 @@ __global__ void __launch_bounds__(kOrderBlock) order_kernel(const AccumulatePara
     const bool fits = s_total <= a.stq.list_capacity;  // ST: always
     if (blockIdx.x == 0 && threadIdx.x == 0) a.queue->st_listed = fits ? s_total : kNotListed;
     if (!fits) return;
+    const uint32_t scale = kGps ? 0u : part_scale(a, true);
     auto parts_of = [&](const uint32_t e, uint32_t& bucket) {
         if (kGps) {
             bucket = depth_bucket(static_cast<uint32_t>(a.q.key[e] >> 32));
@@ -693,7 +714,7 @@ __global__ void __launch_bounds__(kOrderBlock) order_kernel(const AccumulatePara
         const RowGaussian* const G = queue_entry(a.stq, e);
         const uint32_t h = G->row_first;
         bucket = depth_bucket(G->key_hi);
-        return h != 0 ? part_count(quad_rect(G->x_min, G->w, G->y_min, h)) : 0u;
+        return h != 0 ? part_count(quad_rect(G->x_min, G->w, G->y_min, h), scale) : 0u;
     };
     for (uint32_t e = begin + threadIdx.x; e < end; e += kOrderBlock) {
         uint32_t bucket;
@@ -737,6 +758,9 @@ __global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) st_queue_kernel(con
     if (n_items == 0) return;
     const FrameRng rng = frame_rng(a);
     const uint32_t n_warps = kWarpsPerBlock * gridDim.x;
+    __shared__ uint32_t s_scale;  // not a register for all of the loop
+    if (threadIdx.x == 0) s_scale = part_scale(a, dense);
+    __syncthreads();
     if (!dense) {
         // row chunks as they came, each lane a segment of a row, without a look at the keys
         uint32_t c = blockIdx.x + wib * gridDim.x;
@@ -746,7 +770,7 @@ __global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) st_queue_kernel(con
             const uint32_t item = a.stq.list[c];
             if (item != kNoItem) {
                 const RowGaussian G = *queue_entry(a.stq, item & kItemEntryMask);
-                const RowParts r = row_parts(G.w, G.row_first);
+                const RowParts r = row_parts(G.w, G.row_first, s_scale);
                 const uint32_t chunk = (item >> kItemEntryBits) * r.per_part;
                 const uint32_t end = min(chunk + r.per_part, r.chunks);
                 for (uint32_t k = chunk; k < end; ++k) {
@@ -776,7 +800,7 @@ __global__ void __launch_bounds__(kBlock, kQueueBlocksPerSM) st_queue_kernel(con
         if (item != kNoItem) {
             G = *queue_entry(a.stq, item & kItemEntryMask);
             const QuadRect r = quad_rect(G.x_min, G.w, G.y_min, G.row_first);
-            const uint32_t all = r.w * r.h, parts = part_count(r);
+            const uint32_t all = r.w * r.h, parts = part_count(r, s_scale);
             const uint32_t size = (all + parts - 1u) / parts;
             first = min((item >> kItemEntryBits) * size, all);
             quads = min(size, all - first);
@@ -909,7 +933,7 @@ __global__ void clear_kernel(unsigned long long* __restrict__ fb, const size_t n
 __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams a, const size_t n_fb) {
     wait_for_pass_before();
     if (blockIdx.x < kSampleBlocks) {
-        __shared__ float2 s_sum[kWarpsPerBlock];
+        __shared__ float4 s_sum[kWarpsPerBlock];
         __shared__ uint32_t s_larger[kQueueSteps][kWarpsPerBlock];
         const uint32_t t = blockIdx.x * kBlock + threadIdx.x;
         const uint32_t step = max(a.n / (kSampleBlocks * kBlock), 1u);
@@ -924,7 +948,7 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
         const bool points = a.stq.capacity == 0;  // of point splatting, which has no such queue
         const bool compact = !points || in_compact_group(a, g);
         Projected p;
-        float pixels = 0.0f, larger = 0.0f, own = 0.0f;
+        float pixels = 0.0f, larger = 0.0f, own = 0.0f, parts = 0.0f, chunks = 0.0f;
         if (project_gaussian(active, g, a.means, a.scales, a.rotations, a.opacities, a.w2c, a.cam, p, a.pre, a.quant) &&
             active) {
             const PixelRect rect = pixel_rect(p.bounds, a.cam);
@@ -935,19 +959,33 @@ __global__ void __launch_bounds__(kBlock) st_clear_kernel(const AccumulateParams
                      fminf(own * static_cast<float>(step), kSampleMaxCover * a.cam.width * a.cam.height);
             larger = own > static_cast<float>(kDenseMinPixels) ? pixels : 0.0f;
             if (!compact) pixels = 0.0f;
+            // a sampled Gaussian counts for at most 1/32 of the list
+            const float most = static_cast<float>(a.stq.list_capacity) * 0.03125f;
+            if (own > static_cast<float>(kDenseMinPixels))
+                parts = fminf(static_cast<float>(part_count(quad_rect(rect.x_min, rect.width, rect.y_min, rect.height), 0u)) *
+                                  static_cast<float>(step), most);
+            if (own > static_cast<float>(kMinPixels))
+                chunks = fminf(static_cast<float>(row_parts(rect.width, rect.height, 0u).parts) * static_cast<float>(step), most);
         }
         for (uint32_t o = 16; o > 0; o >>= 1) {
             pixels += __shfl_xor_sync(kFullMask, pixels, o);
             larger += __shfl_xor_sync(kFullMask, larger, o);
+            parts += __shfl_xor_sync(kFullMask, parts, o);
+            chunks += __shfl_xor_sync(kFullMask, chunks, o);
         }
-        if ((threadIdx.x & 31u) == 0) s_sum[threadIdx.x >> 5] = make_float2(larger, pixels);
+        if ((threadIdx.x & 31u) == 0) s_sum[threadIdx.x >> 5] = make_float4(larger, pixels, parts, chunks);
         for (uint32_t i = 0; i < kQueueSteps; ++i) {
             const uint32_t above = __ballot_sync(kFullMask, own > static_cast<float>(kDenseMinPixels << i));
             if ((threadIdx.x & 31u) == 0) s_larger[i][threadIdx.x >> 5] = __popc(above);
         }
         __syncthreads();
         if (threadIdx.x == 0) {
-            for (uint32_t w = 1; w < kWarpsPerBlock; ++w) larger += s_sum[w].x, pixels += s_sum[w].y;
+            for (uint32_t w = 1; w < kWarpsPerBlock; ++w) {
+                larger += s_sum[w].x, pixels += s_sum[w].y;
+                parts += s_sum[w].z, chunks += s_sum[w].w;
+            }
+            a.queue->parts[0][blockIdx.x] = parts;
+            a.queue->parts[1][blockIdx.x] = chunks;
             a.queue->covered[blockIdx.x] = larger;
             a.queue->covered_all[blockIdx.x] = pixels;
             for (uint32_t i = 0; i < kQueueSteps; ++i) {

@@ -30,9 +30,10 @@ struct WorkQueue {
                                        // kSampleBlocks blocks of the clear pass
     alignas(16) float covered_all[4];  // the same of all its Gaussians (GPS: of those in compact groups)
     alignas(16) float larger[kQueueSteps][4];  // Gaussians with AABBs above kDenseMinPixels << step, estimated likewise
+    alignas(16) float parts[2][4];             // parts of the queued ones in a dense and in a sparse scene, likewise
 };
 static_assert(offsetof(WorkQueue, covered) % 16 == 0 && offsetof(WorkQueue, covered_all) % 16 == 0 &&
-              offsetof(WorkQueue, larger) % 16 == 0, "read as float4");
+              offsetof(WorkQueue, larger) % 16 == 0 && offsetof(WorkQueue, parts) % 16 == 0, "read as float4");
 constexpr unsigned long long kQueueEntryShift = 40;
 constexpr unsigned long long kQueueChunkMask = (1ull << kQueueEntryShift) - 1;
 // Producers queue chunk indices below this, so the consumers' cursor (which overshoots the last chunk

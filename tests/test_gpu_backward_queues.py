@@ -80,8 +80,8 @@ def test_full_queues(n, huge, full, cuda_device):
         return (v + 255) & ~255
 
     at = up(4 * ((3 * n + 3) & ~3)) + up(8 * 10 * n)
-    headers = bw[at:at + 256].view(torch.int64).cpu().numpy()  # 128 bytes each: entries << 40 | chunks, ...
-    entries = [int(headers[0]) >> 40, int(headers[16]) >> 40]
+    headers = bw[at:at + 512].view(torch.int64).cpu().numpy()  # 160 bytes each: entries << 40 | chunks, ...
+    entries = [int(headers[0]) >> 40, int(headers[20]) >> 40]
     assert [v > FULL for v in entries] == list(full) and min(entries) > 1000, entries
     for name, a, b in zip(("means", "scales", "rotations", "opacities", "sh"), want, got):
         scale = np.abs(a).max()
