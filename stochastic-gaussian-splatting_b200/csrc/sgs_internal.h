@@ -28,7 +28,8 @@ struct WorkQueue {
     unsigned int st_listed;      // items the order pass has listed (GPS: or kNotListed)
     alignas(16) float covered[4];      // AABB pixels of the scene's larger Gaussians, weighted by opacity, estimated by
                                        // kSampleBlocks blocks of the clear pass
-    alignas(16) float covered_all[4];  // the same of all its Gaussians (GPS: of those in compact groups)
+    alignas(16) float covered_all[4];  // the same of all its Gaussians of at most kDenseMinPixels << kQueueSteps pixels (GPS:
+                                       // of those in compact groups)
     alignas(16) float larger[kQueueSteps][4];  // Gaussians with AABBs above kDenseMinPixels << step, estimated likewise
     alignas(16) float parts[2][4];             // parts of the queued ones in a dense and in a sparse scene, likewise
 };

@@ -5,6 +5,7 @@ scenes of few covered pixels, for which the order takes longer than it saves: in
 """
 import numpy as np
 import pytest
+import torch
 
 import sgs_scenes
 from oracle import cpu
@@ -40,3 +41,11 @@ def test_deep_faint_scenes_are_drawn_as_they_lie(gps, cuda_device):
         scene.opacities += shift
         estimates.append(covered_all(render(scene.to(cuda_device).tensors(), cuda_device, samples=2, mode=1, gps=gps)[2]))
     assert estimates[0] > 58 * WIDTH * HEIGHT > estimates[1] > 0
+
+
+def test_footprints_too_large_for_the_tests_do_not_count(cuda_device):
+    """Passes in depth order test Gaussians of few tiles only."""
+    n_fb = WIDTH * HEIGHT
+    header = render(deep_scene((1 << 21) + 45, -1.0).to(cuda_device).tensors(), cuda_device, samples=2, mode=1, gps=False)[2]
+    larger = float(header[48:64].view(torch.float32).sum())
+    assert larger > 10_000 * n_fb and covered_all(header) < 0.1 * larger
