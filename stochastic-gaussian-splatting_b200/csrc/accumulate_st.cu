@@ -23,7 +23,7 @@
 //    off the ellipse, and the warp walks the rest, two pixels per lane, lowering the bounds with the
 //    keys it reads. Keys only decrease during a pass, so a dropped fragment could not have won;
 //  * deep scenes of millions of Gaussians run front to back (sgs_front.cuh): the pass drops the groups and
-//    the Gaussians that lie behind their tiles' bounds (6M at 1080p: 577 us a sample to 399, 283 million
+//    the Gaussians that lie behind their tiles' bounds (6M at 1080p: 577 us a sample to 395, 283 million
 //    warp instructions instead of 469; half of the rows are left, and their walk is what bounds it);
 //  * u64 atomicMin (fire-and-forget RED) on the L2-resident framebuffer.
 //
@@ -429,9 +429,15 @@ __device__ __forceinline__ bool dense_scene(const AccumulateParams& a) {
 // those of the next larger size that it holds. A warp draws what finds the queue full by itself, which takes long where
 // that are Gaussians of many thousand pixels (2M Gaussians and 24,000 large ones at 1920x1080, room for 0.53 of 1.30
 // million above 256: 2631 us a sample; of the larger ones that it holds 1367; with a queue for 2048 and more 1731). A
-// few per cent past the room cost less than the next size (1M Gaussians at 1280x720, room for all: 455 and 539 us).
-__device__ __forceinline__ uint32_t queued_above(const AccumulateParams& a, const bool dense) {
-    const float room = 1.05f * static_cast<float>(a.stq.capacity);
+// few per cent past the room cost less than the next size (1M Gaussians at 1280x720, room for all: 455 and 539 us), but
+// not front to back (kFrontRoom).
+constexpr float kRoom = 1.05f;
+// Front to back, what finds the queue full comes last and together: single warps with 32 Gaussians of thousands of pixels
+// each. Such passes leave some room, and scenes whose large Gaussians may not fit are drawn as they lie (5M Gaussians
+// around the camera, 1600x900: 6382 us a sample front to back, 1738; 2.7M: 2090, 608; 5M faint ones 4720, 1561).
+constexpr float kFrontRoom = 0.95f;
+__device__ __forceinline__ uint32_t queued_above(const AccumulateParams& a, const bool dense, const float share = kRoom) {
+    const float room = share * static_cast<float>(a.stq.capacity);
     uint32_t step = kQueueSteps;
 #pragma unroll
     for (uint32_t i = kQueueSteps; i-- > 0;) {
@@ -484,9 +490,18 @@ st_scatter_kernel(const AccumulateParams a) {
     wait_for_pass_before();
     constexpr bool kSplit = kMode == kSplitRows;
     uint32_t block = blockIdx.x;
-    bool ordered = false;
+    bool ordered = false, dense = false;
+    uint32_t queue_above = kMinPixels, scale = 0;
     if (kMode == kFrontToBack) {
         ordered = front_to_back(a);
+        dense = dense_scene(a);
+        if (dense) {
+            queue_above = queued_above(a, true, ordered ? kFrontRoom : kRoom);
+            if (ordered && queue_above == kMinPixels) {  // none of the sizes is sure to fit
+                ordered = false;
+                queue_above = queued_above(a, true);
+            }
+        }
         if (!draws<kWarps>(a, block, ordered, wib, lane)) return;
     }
     uint32_t gwarp = block * kWarps + wib;
@@ -503,9 +518,7 @@ st_scatter_kernel(const AccumulateParams a) {
     if (kMode == kFrontToBack && ordered && group_hidden(a, active, g, lane)) return;
 
     // Loaded while the projection waits for its own loads: after it, the scatter pass over 400k large Gaussians took 73 us
-    // instead of 68. Deep scenes are seldom dense and load the sizes only then, after the projection.
-    bool dense = false;
-    uint32_t queue_above = kMinPixels, scale = 0;
+    // instead of 68. Deep scenes are seldom dense and load the sizes only then.
     if (kMode != kFrontToBack) {
         dense = dense_scene(a);
         queue_above = queued_above(a, dense);
@@ -514,10 +527,6 @@ st_scatter_kernel(const AccumulateParams a) {
     Projected p;
     if (!project_gaussian(active, g, a.means, a.scales, a.rotations, a.opacities, a.w2c, a.cam, p, a.pre, a.quant)) return;
     const FrameRng rng = frame_rng(a);
-    if (kMode == kFrontToBack) {
-        dense = dense_scene(a);
-        if (dense) queue_above = queued_above(a, true);
-    }
 
     const PixelRect rect = pixel_rect(p.bounds, a.cam);
     uint32_t count = active ? rect.width * rect.height : 0u;

@@ -83,7 +83,7 @@ struct Derived {
 // that few Gaussians, or few per pixel, are not prepared for it; below some 2.5M most of them are in flight before
 // the first bounds exist. As they lie against front to back, in us, the 6M scene cut to n Gaussians:
 //   one sample: 2.2M 1920x1080 (coverage 49) 264, 287, 1280x720 (55) 200, 196; 3M 1920x1080 (66) 330, 310,
-//     3840x2160 (44) 695, 737, 1280x720 (75) 253, 208; 6M 1920x1080 (133) 577, 399, 3840x2160 (87) 1187, 978
+//     3840x2160 (44) 695, 737, 1280x720 (75) 253, 207; 6M 1920x1080 (133) 577, 395, 3840x2160 (87) 1187, 976
 //   one sample of point splatting: 4M 1920x1080 (88) 239, 258, 1280x720 (100) 185, 183; 6M 3840x2160 (87) 615, 638,
 //     1920x1080 (133) 323, 293, 1280x720 (150) 255, 209
 //   faint ones, logits -2 and -3 on average, 6M 1920x1080 (48) 471, 533, (18) 416, 506; 8 samples 1862, 1931, 1540, 1632

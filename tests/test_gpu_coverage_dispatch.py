@@ -9,7 +9,7 @@ import torch
 
 import sgs_scenes
 from oracle import cpu
-from test_gpu_front_dispatch import HEIGHT, WIDTH, covered_all, render
+from test_gpu_front_dispatch import HEIGHT, WIDTH, binned, covered_all, render
 from test_gpu_front_to_back import deep_scene
 from test_gpu_schedule import KEYS, cam_dict
 from test_gpu_st_queue import dense_scene
@@ -49,3 +49,21 @@ def test_footprints_too_large_for_the_tests_do_not_count(cuda_device):
     header = render(deep_scene((1 << 21) + 45, -1.0).to(cuda_device).tensors(), cuda_device, samples=2, mode=1, gps=False)[2]
     larger = float(header[48:64].view(torch.float32).sum())
     assert larger > 10_000 * n_fb and covered_all(header) < 0.1 * larger
+
+
+def test_queues_that_may_fill_hinder_the_order(cuda_device):
+    """What finds a dense scene's queue full comes last in depth order, and together: such scenes are drawn as they lie."""
+    from StochasticGSCudaBackend import _C
+
+    scene = deep_scene((1 << 21) + 45, -3.8).to(cuda_device).tensors()
+    _, ordered, header = render(scene, cuda_device, samples=2, mode=1, gps=False, hybrid=True)
+    larger = header[80:128].view(torch.float32).view(3, 4).sum(dim=1).tolist()
+    listed = int(header[32:36].view(torch.int32))
+    assert covered_all(header) > 58 * WIDTH * HEIGHT and listed > 0
+    try:
+        _C.set_queue_limit(max(int(larger[2] * 0.8), 1))
+        _, as_they_lie, full = render(scene, cuda_device, samples=2, mode=1, gps=False, hybrid=True)
+    finally:
+        _C.set_queue_limit(0)
+    assert binned(header) < binned(full)  # groups that are left out are not counted
+    np.testing.assert_array_equal(as_they_lie, ordered)
