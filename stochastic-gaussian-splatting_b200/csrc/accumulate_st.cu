@@ -522,7 +522,7 @@ st_scatter_kernel(const AccumulateParams a) {
     if (kMode != kFrontToBack) {
         dense = dense_scene(a);
         queue_above = queued_above(a, dense);
-        scale = part_scale(a, dense);
+        if (dense) scale = part_scale(a, true);
     }
     Projected p;
     if (!project_gaussian(active, g, a.means, a.scales, a.rotations, a.opacities, a.w2c, a.cam, p, a.pre, a.quant)) return;
@@ -584,7 +584,7 @@ st_scatter_kernel(const AccumulateParams a) {
         if (lane == leader) e = atomicAdd(&a.queue->st_entries, static_cast<uint32_t>(__popc(big)));
         e = __shfl_sync(kFullMask, e, leader) + __popc(big & lt_mask);
         const bool fits = want && e < a.stq.capacity;
-        if (kMode == kFrontToBack) scale = part_scale(a, dense);
+        if (kMode == kFrontToBack || !dense) scale = part_scale(a, dense);
         const uint32_t parts =
             !fits   ? 0u
             : dense ? part_count(quad_rect(rect.x_min, rect.width, rect.y_min, rect.height), scale)
